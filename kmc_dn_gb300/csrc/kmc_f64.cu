@@ -1,28 +1,52 @@
-// kmc_f64.cu -- plain single-chain FP64 hop loop for sm_103a.
+// kmc_f64.cu -- plain FP64 hop loop for sm_103a, one thread block per chain.
 //
-// One thread block runs one chain with the semantics of the reference's
-// numba loop _simulate_discrete_record (kmc_dopant_networks.py:33-135), in
-// FP64 and with the reference's operand order, so that fed the same uniform
+// The semantics of the reference's numba loop _simulate_discrete_record
+// (kmc_dopant_networks.py:33-135) in FP64, so that fed the same uniform
 // stream it makes the same hop sequence:
 //
-//   energies   E_i = Ec_i + (-I_0 R) * sum_{j != i} (1 - occ_j)/d_ij, summed in
+//   energies   E_i = Ec_i + (-I_0 R) * sum_{j empty} 1/d_ij, summed in
 //              ascending j (:59-66); 1/d_ij is tabulated once (the same
 //              correctly rounded quotient the loop divides out each hop)
-//   rates      dense S x S, row-major: tc_ij * (dE > 0 ? nu*exp(-dE/kT) : nu),
+//   rates      tc_ij * (dE > 0 ? nu*exp(-dE/kT) : nu),
 //              dE = E_j - E_i - (I_0 R)/d_ij for acceptor pairs (:69-87)
-//   cumulative row-major running sum; each thread owns a contiguous chunk
-//              and continues the running sum from the FP64 prefix of the
-//              chunks before it (:91-97).  That prefix is a tree sum of the
-//              chunk totals, not the reference's strictly left-to-right sum,
-//              so cum_k and the total may differ in the last bit: the hop
-//              sequence is the reference's except where u2 lies within a
-//              few ulp of a boundary cum_k/total
+//   cumulative row-major running sum (:91-97)
 //   clock      dt = -log(1 - u1) * (1/total) (:100)
 //   event      first k with cum_k/total >= u2 (:103-110)
 //   record     traffic[from,to] += 1, post-hop occupancy credit (:126-130)
 //
-// This is the baseline kernel the batched FP32 engine is measured against,
-// and the kernel of the bit-exact replay check.
+// Only the allowed transitions are visited, A(h) = h(N-h) + hP + P(N-h) of
+// the S^2 pairs, in the dense loop's row-major order (a forbidden pair has
+// rate 0 and leaves every running sum as it is).  Thread g owns M
+// consecutive allowed pairs and continues the running sum from the FP64
+// prefix of the threads before it.  That prefix is a tree sum, not the
+// reference's strictly left-to-right sum, and the exponential is taken as a
+// product (below), so cum_k and the total may differ in the last bits: the
+// hop sequence is the reference's except where u2 lies within a few ulp of a
+// boundary cum_k/total.
+//
+// What bounds it is the FP64 pipe: a warp instruction holds its SM quarter's
+// unit for 64 cycles whatever its neighbours do (64.3 measured for dependent
+// and for independent chains; 128 with two warps on a quarter), so the count
+// of FP64 instructions is the time.  So:
+//   * exp(-dE/kT) is the product exp(E_i/kT) exp(-E_j/kT) exp(I_0R/d_ij/kT):
+//     one exponential a site and hop, the third factor tabulated together
+//     with tc, and a pair costs two multiplications and an integer minimum
+//     against tc*nu instead of two subtractions, a comparison and an
+//     exponential.  Mantissa and exponent are kept apart, so no factor can
+//     overflow, and no difference of large energies is rounded;
+//   * comparisons are integer compares of the bit patterns;
+//   * after the warps' scans one warp picks the event while another divides
+//     for the clock, and the uniforms' logarithms are taken for 32 hops at
+//     once: three block barriers a hop;
+//   * four warps, one a quarter of the SM: more would wait for the same pipe.
+// One N = 30, P = 8 chain: 4.0 us a hop (18.8 us with S^2 dense rates and
+// running sums in global memory, 6.1 us with the pairs' exponentials queued
+// 32 at a time); 256 chains of N = 60, P = 8, 300 hops with occupancy and
+// flux: 4.2 ms (28.9 ms, 6.6 ms).  Time against the same hop sequences in
+// 113-bit arithmetic, rms relative error over 40 networks: N = 30 1.3e-14
+// (dense rates 1.4e-14), N = 60 1.96e-13 (1.89e-13): the energies' rounding.
+#include <algorithm>
+#include <climits>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -32,205 +56,533 @@
 namespace kmc {
 namespace {
 
-constexpr int kThreads = 256;
-
-__device__ __forceinline__ bool possible(int i, int j, int N, const uint8_t *occ)
+constexpr int kThreads = 128;
+constexpr int kWarps = kThreads / 32;
+// x > 0 for finite and infinite x, false for NaN (as the comparison is), on
+// the integer pipe.
+__device__ __forceinline__ bool positive(double x)
 {
-    if (i >= N && j >= N) return false;
-    if (i >= N) return !occ[j];
-    if (j >= N) return occ[i] != 0;
-    if (i == j) return false;
-    return occ[i] && !occ[j];
+    return static_cast<unsigned long long>(__double_as_longlong(x)) - 1ull < 0x7ff0000000000000ull;
 }
 
-__device__ double block_exclusive_scan(double v, double *sh, double &total)
+// x >= y of positive finite values, on the integer pipe.
+__device__ __forceinline__ bool not_less(double x, long long y_bits)
 {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    double x = v;
+    return __double_as_longlong(x) >= y_bits;
+}
+
+// exp(x + y) = m * 2^k, 1 <= m <= 2, y a small correction of x, by table and
+// short polynomial (Tang, "Table-driven implementation of the exponential
+// function in IEEE floating-point arithmetic", ACM TOMS 15, 1989):
+// x = (128 k + j) ln2/128 + r, |r| <= ln2/256, m = 2^(j/128) (1 + p(r)), the
+// table entries with their low parts.  |x| < 2^17.  Within 0.51 ulp (largest
+// of 4e6 arguments in (-708, 0]; exp() there 0.87) while |x| < 5000; beyond,
+// the reduction rounds by 2^-53 |x|, as the energies themselves do.
+constexpr int kExpTable = 128;
+__device__ __forceinline__ double exp_split(double x, double y, const double2 *table, int &k)
+{
+    const double shift = 0x1.8p52;
+    const double t = fma(x, 0x1.71547652b82fep+7, shift);        // 128/ln2
+    const int n = __double2loint(t);
+    const double nf = t - shift;
+    // ln2/128 in a 33-bit part, whose products with small n are exact, and the rest
+    double r = fma(nf, -0x1.473de6af278edp-41, fma(nf, -0x1.62e42fefp-8, x));
+    if (__double_as_longlong(y) << 1) r += y;      // not for a zero: an add saved
+    double q = fma(r, 1.0 / 120.0, 1.0 / 24.0);
+    q = fma(fma(q, r, 1.0 / 6.0), r, 0.5);
+    const double p = fma(q, r * r, r);
+    const double2 T = table[n & (kExpTable - 1)];
+    k = n >> 7;
+    return T.x + fma(T.x, p, T.y);
+}
+
+// Entry j of that table, 2^(j/128) as hi + lo: the product of 2^(2^b/128)
+// over the bits of j in double-double arithmetic.
+__device__ double2 exp_table_entry(int j)
+{
+    const double hi[7] = {0x1.0163da9fb3335p+0, 0x1.02c9a3e778061p+0, 0x1.059b0d3158574p+0, 0x1.0b5586cf9890fp+0,
+                          0x1.172b83c7d517bp+0, 0x1.306fe0a31b715p+0, 0x1.6a09e667f3bcdp+0};
+    const double lo[7] = {0x1.b61299ab8cdb7p-54,  -0x1.19083535b085dp-56, 0x1.d73e2a475b465p-55,
+                          0x1.8a62e4adc610bp-54,  -0x1.19041b9d78a76p-55, 0x1.6f46ad23182e4p-55,
+                          -0x1.bdd3413b26456p-54};
+    double x = 1.0, y = 0.0;
 #pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const double o = __shfl_up_sync(0xffffffffu, x, d);
-        if (lane >= d) x += o;
-    }
-    if (lane == 31) sh[warp] = x;
-    __syncthreads();
-    if (warp == 0) {
-        double w = lane < kThreads / 32 ? sh[lane] : 0.0;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const double o = __shfl_up_sync(0xffffffffu, w, d);
-            if (lane >= d) w += o;
+    for (int b = 0; b < 7; ++b) {
+        if ((j >> b) & 1) {
+            const double m = x * hi[b];
+            const double e = fma(x, hi[b], -m) + (x * lo[b] + y * hi[b]);
+            x = m + e;
+            y = e - (x - m);
         }
-        if (lane < kThreads / 32) sh[lane] = w;
     }
-    __syncthreads();
-    const double warp_base = warp > 0 ? sh[warp - 1] : 0.0;
-    total = sh[kThreads / 32 - 1];
-    __syncthreads();
-    return warp_base + x - v;
+    return make_double2(x, y);
+}
+
+// A site in a list: exp(+-E/kT) = m 2^k (a source's +, a target's -).
+struct __align__(16) Site {
+    double m;
+    int id;
+    int k;
+};
+
+// |x| at and beyond which the split exponential is not used.
+__device__ __forceinline__ bool splittable(double x)
+{
+    return (__double2hiint(x) & 0x7fffffff) < 0x41000000;
+}
+
+// x / kT as the correctly rounded quotient (reciprocal product and one
+// residual, Markstein) and what it misses; `unit`: kT = 1.
+__device__ __forceinline__ double over_kT(double x, bool unit, double kT, double inv_kT, double &rest)
+{
+    rest = 0.0;
+    if (unit) return x;
+    const double y0 = x * inv_kT;
+    const double y = fma(fma(-y0, kT, x), inv_kT, y0);
+    rest = fma(-y, kT, x) * inv_kT;
+    return y;
+}
+
+// Exact n / T for 0 <= n < 2^22 from inv ~ 1/T: float quotient, one
+// correction step.
+__device__ __forceinline__ int div_small(int n, int T, float inv, int &rem)
+{
+    int q = __float2int_rz(__int2float_rn(n) * inv);
+    int r = n - q * T;
+    if (r < 0) { --q; r += T; } else if (r >= T) { ++q; r -= T; }
+    rem = r;
+    return q;
+}
+
+// Shared memory of one chain.  The three optional parts go to shared memory
+// when the launch gives them room (f64_layout), else they stay in the
+// caller's arrays and the workspace.
+struct Layout {
+    int S;                  // sites the lists are sized for
+    int tab, rates, invd;   // entries reserved, 0: not in shared memory
+};
+
+__host__ __device__ inline size_t layout_bytes(const Layout &l)
+{
+    return 20 * static_cast<size_t>(l.tab) + 8 * static_cast<size_t>(l.rates + l.invd) + 16 * kExpTable +
+           (2 * sizeof(Site) + 2 * 8 + 4) * static_cast<size_t>(l.S) + 8 * (kThreads + 64 + 128) + 4 * 64 + 32;
 }
 
 // One chain run by the whole block (the body of both kernels below).
+// kTab: tc and (I_0 R)/d are read from shared memory; kRate: the rates of a
+// hop sit there.
+template <bool kTab, bool kRate>
 __device__ __forceinline__ void f64_chain(
-    int N, int P, double nu, double kT, double I0, double R, uint8_t *occ_g, const double *d,
+    const Layout &lay, int N, int P, double nu, double kT, double I0, double R, uint8_t *occ_g, const double *d,
     const double *Ec, const double *se_in, const double *tc, int64_t *eo, int64_t hops,
     int record, double *traffic, double *oit, const double *uniforms, uint64_t seed,
     int32_t *hop_log, double *time_out, int32_t *status_out, double *ws, double *flux_time)
 {
     extern __shared__ __align__(16) unsigned char sraw[];
     const int S = N + P;
-    const int SS = S * S;
-    double *se = reinterpret_cast<double *>(sraw);            // [S]
-    double *red = se + S;                                     // [32] scan scratch
-    uint8_t *occ = reinterpret_cast<uint8_t *>(red + 32);     // [S]
-    __shared__ int ev_min;
-    __shared__ double sh_total, sh_hop_time;
-    __shared__ double sh_flux[64];   // expected net inflow of each electrode (flux_time only)
+    double2 *tab = reinterpret_cast<double2 *>(sraw);              // [S*S] tc*nu, mantissa of tc*nu*exp(I_0R/d/kT)
+    double2 *exp_tab = tab + lay.tab;                              // [kExpTable]
+    Site *src = reinterpret_cast<Site *>(exp_tab + kExpTable);     // [S] holes at 0.., electrode e at N + e
+    Site *tgt = src + lay.S;                                       // [S] empty acceptors at 0.., electrodes as there
+    double *rate_s = reinterpret_cast<double *>(tgt + lay.S);      // [A] this hop's rates
+    double *invd_s = rate_s + lay.rates;                           // [N*N] 1/d_ij at j*N + i
+    double *src_e = invd_s + lay.invd;                             // [S] energies of the sources
+    double *tgt_e = src_e + lay.S;                                 // [S] energies of the targets
+    double *incl = tgt_e + lay.S;                                  // [kThreads] warp-inclusive sums
+    double *u_ev = incl + kThreads;                                // [32] event uniforms
+    double *u_cl = u_ev + 32;                                      // [32] -log(1 - u1)
+    double *sh_J = u_cl + 32;                                      // [64] expected net inflow
+    double *sh_fx = sh_J + 64;                                     // [64] its time integral
+    int *tab_k = reinterpret_cast<int *>(sh_fx + 64);              // [S*S] exponents beside tab
+    int *eo_s = tab_k + lay.tab;                                   // [P]
+    uint32_t *occw = reinterpret_cast<uint32_t *>(eo_s + lay.S);   // [64] occupancy bits
+    __shared__ int wide_always, wide_now[2];   // energies or couplings beyond the split exponential
+    __shared__ int ev_from, ev_to;
+    __shared__ double sh_dt;
 
-    double *invd = ws;                  // [N*N] 1/d_ij
-    double *ird = ws + (size_t)N * N;   // [N*N] (I_0 R)/d_ij
-    double *cum = ws + 2 * (size_t)N * N;   // [S*S] rates, then running sums
+    // workspace: mantissas and exponents of the table, 1/d, rates
+    const size_t SS = (size_t)S * S;
+    double *W_g = ws;
+    int *k_g = reinterpret_cast<int *>(ws + SS);
+    double *invd_g = ws + SS + (SS + 1) / 2;
+    double *rates = kRate ? rate_s : invd_g + (size_t)N * N;
 
-    const int tid = threadIdx.x;
-    const bool kT_is_one = (kT == 1.0);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const bool unit = (kT == 1.0), nu_is_one = (nu == 1.0);
+    const double inv_kT = 1.0 / kT;
     const double IR = I0 * R;
     const double mIR = -I0 * R;
+    double *invd = lay.invd > 0 ? invd_s : invd_g;
+    for (int j = tid; j < kExpTable; j += kThreads) exp_tab[j] = exp_table_entry(j);
+    if (tid == 0) wide_always = wide_now[0] = wide_now[1] = 0;
     for (int k = tid; k < N * N; k += kThreads) {
         const int i = k / N, j = k - (k / N) * N;
         const double dij = d[(size_t)i * S + j];
-        invd[k] = (i != j) ? 1.0 / dij : 0.0;
-        ird[k] = (i != j) ? IR / dij : 0.0;
-    }
-    for (int i = tid; i < S; i += kThreads) {
-        se[i] = se_in[i];
-        occ[i] = (i < N) ? occ_g[i] : 0;
+        invd[(size_t)j * N + i] = (i != j) ? 1.0 / dij : 0.0;
     }
     __syncthreads();
+    for (int k = tid; k < S * S; k += kThreads) {
+        const int i = k / S, j = k - (k / S) * S;
+        const double cap = tc[k] * nu;
+        double rest, m = 1.0;
+        int e = 0;
+        if (i < N && j < N && i != j) {
+            const double x = over_kT(IR / d[k], unit, kT, inv_kT, rest);
+            if (splittable(x)) m = exp_split(x, rest, exp_tab, e);
+            else wide_always = 1;
+        }
+        // tc*nu in range: keep the factor's exponent apart from it
+        if (kTab) {
+            tab[k] = make_double2(cap, cap * m);
+            tab_k[k] = e;
+        } else {
+            W_g[k] = cap * m;
+            k_g[k] = e;
+        }
+    }
+    const int W = (N + 31) >> 5;
+    for (int w = tid; w < W; w += kThreads) {
+        uint32_t bits = 0;
+        for (int b = 0; b < 32 && w * 32 + b < N; ++b)
+            if (occ_g[w * 32 + b]) bits |= 1u << b;
+        occw[w] = bits;
+    }
+    for (int e = tid; e < P; e += kThreads) {
+        eo_s[e] = 0;
+        if (flux_time) sh_fx[e] = flux_time[e];
+    }
+    // the electrodes' list entries, the same every hop
+    for (int i = N + tid; i < S; i += kThreads) {
+        const double e = se_in[i];
+        double rest;
+        const double x = over_kT(e, unit, kT, inv_kT, rest);
+        src_e[i] = tgt_e[i] = e;
+        Site a{1.0, i, 0}, b{1.0, i, 0};
+        if (splittable(x)) {
+            a.m = exp_split(x, rest, exp_tab, a.k);
+            b.m = exp_split(-x, -rest, exp_tab, b.k);
+        } else {
+            wide_always = 1;
+        }
+        src[i] = a;
+        tgt[i] = b;
+    }
+    __syncthreads();
+    int h = 0;
+    for (int w = 0; w < W; ++w) h += __popc(occw[w]);
 
-    const int chunk = (SS + kThreads - 1) / kThreads;
-    const int kb = tid * chunk;
-    const int ke = min(kb + chunk, SS);
-    double time = 0.0;
+    double time = 0.0, dt = 0.0;     // (the clock: warp 1)
+    // this thread's first site: occupied time and constant energy
+    double oit0 = (record && tid < N) ? oit[tid] : 0.0;
+    const double Ec0 = tid < N ? Ec[tid] : 0.0;
     int status = KMC_OK;
+    int from = S, to = S;      // the last hop, not yet in occw (none before the first)
 
-    for (int64_t hop = 0; hop < hops; ++hop) {
-        // site energies
+    for (int64_t hop = 0;; ++hop) {
+        // ---- lists of the current state: the last hop applied to the bits ----
+        const int wf = from < N ? from >> 5 : -1, wt = to < N ? to >> 5 : -1;
+        const uint32_t bf = from < N ? 1u << (from & 31) : 0u, bt = to < N ? 1u << (to & 31) : 0u;
+        const int z = N - h;
         for (int i = tid; i < N; i += kThreads) {
-            double acc = 0.0;
-            const double *row = invd + (size_t)i * N;
-            for (int j = 0; j < N; ++j)
-                if (j != i && !occ[j]) acc += row[j];
-            double e = Ec[i];
+            double acc = 0.0, next = 0.0;
+            int below = 0, n_empty = 0;
+            bool occ_i = false;
+            for (int w = 0; w < W; ++w) {
+                uint32_t word = occw[w];
+                if (w == wf) word &= ~bf;
+                if (w == wt) word |= bt;
+                const int left = N - w * 32;
+                uint32_t empty = ~word & (left >= 32 ? 0xffffffffu : (1u << left) - 1u);
+                if ((i >> 5) == w) {
+                    below += __popc(word & ((1u << (i & 31)) - 1u));
+                    occ_i = (word >> (i & 31)) & 1u;
+                } else if ((i >> 5) > w) {
+                    below += __popc(word);
+                }
+                // ascending j, each entry loaded ahead of the add before it
+                // (the diagonal entry is 0)
+                const double *col = invd + (size_t)w * 32 * N + i;
+                while (empty) {
+                    const double v = col[(size_t)(__ffs(empty) - 1) * N];
+                    empty &= empty - 1;
+                    if (n_empty > 1) acc += next;
+                    else acc = next;
+                    ++n_empty;
+                    next = v;
+                }
+            }
+            if (n_empty > 1) acc += next;
+            else acc = next;
+            double e = i == tid ? Ec0 : Ec[i];
             e += mIR * acc;
-            se[i] = e;
+            double rest;
+            const double y = over_kT(e, unit, kT, inv_kT, rest);
+            Site a{1.0, i, 0};
+            if (splittable(y)) a.m = exp_split(occ_i ? y : -y, occ_i ? rest : -rest, exp_tab, a.k);
+            else wide_now[hop & 1] = 1;
+            if (occ_i) {
+                src[below] = a;
+                src_e[below] = e;
+                if (record && hop > 0) {
+                    if (i == tid) oit0 += dt;
+                    else oit[i] += dt;
+                }
+            } else {
+                tgt[i - below] = a;
+                tgt_e[i - below] = e;
+            }
+        }
+        if (hop >= hops) break;
+        if ((hop & 31) == 0 && warp == kWarps - 1) {
+            // the uniforms of the next 32 hops, mapped
+            const int64_t hh = hop + lane;
+            double u1 = 0.5, u2 = 0.5;
+            if (uniforms) {
+                if (hh < hops) {
+                    u1 = uniforms[2 * hh];
+                    u2 = uniforms[2 * hh + 1];
+                }
+            } else {
+                const u32x4 r = philox4x32_10(u32x4{static_cast<uint32_t>(hh), static_cast<uint32_t>(hh >> 32), 0u, 0u},
+                                              static_cast<uint32_t>(seed), static_cast<uint32_t>(seed >> 32));
+                u1 = u01_from64(r.x, r.y);
+                u2 = u01_from64(r.z, r.w);
+            }
+            u_ev[lane] = u2;
+            u_cl[lane] = -log(1.0 - u1);
         }
         __syncthreads();
-        // rates over this thread's chunk
-        double lsum = 0.0;
-        for (int k = kb; k < ke; ++k) {
-            const int i = k / S, j = k - (k / S) * S;
-            double t = 0.0;
-            if (possible(i, j, N, occ)) {
-                double dE;
-                if (i < N && j < N) dE = se[j] - se[i] - ird[(size_t)i * N + j];
-                else dE = se[j] - se[i];
-                // x / 1.0 == x exactly, so kT = 1 skips the division bit-exactly
-                t = (dE > 0) ? nu * exp(kT_is_one ? -dE : -dE / kT) : nu;
-            }
-            t = tc[k] * t;
-            cum[k] = t;
-            lsum += t;
+        const bool wide = wide_always | wide_now[hop & 1];
+        if (tid == 0) {      // every thread has read the bits: take the last hop in
+            wide_now[(hop + 1) & 1] = 0;
+            if (wf >= 0) occw[wf] &= ~bf;
+            if (wt >= 0) occw[wt] |= bt;
         }
-        double blocktot;
-        const double base = block_exclusive_scan(lsum, red, blocktot);
+
+        // ---- rates of the allowed pairs ----
+        const int T1 = z + P, T2 = z;
+        const int A1 = h * T1, A = A1 + P * T2;
+        const float inv1 = T1 > 0 ? __fdividef(1.0f, static_cast<float>(T1)) : 0.0f;
+        const float inv2 = T2 > 0 ? __fdividef(1.0f, static_cast<float>(T2)) : 0.0f;
+        const int M = (A + kThreads - 1) / kThreads;      // pairs per thread
+        const int kw = warp * 32 * M, kwe = min(kw + 32 * M, A);
+        // kAhead rounds of 32 pairs load together
+        constexpr int kAhead = 4;
+        for (int k0 = kw; k0 < kwe; k0 += 32 * kAhead) {
+            double cap[kAhead], g[kAhead];
+            int ex[kAhead];
+#pragma unroll
+            for (int a = 0; a < kAhead; ++a) {
+                const int k = k0 + 32 * a + lane;
+                cap[a] = g[a] = 0.0;
+                ex[a] = 0;
+                if (k < kwe) {
+                    int row, col;
+                    if (k < A1) row = div_small(k, T1, inv1, col);
+                    else row = N + div_small(k - A1, T2, inv2, col);
+                    if (col >= z) col += N - z;
+                    const Site f = src[row], t = tgt[col];
+                    const size_t at = (size_t)f.id * S + t.id;
+                    double w;
+                    if (kTab) {
+                        const double2 T = tab[at];
+                        cap[a] = T.x;
+                        w = T.y;
+                        ex[a] = tab_k[at];
+                    } else {
+                        cap[a] = nu_is_one ? tc[at] : tc[at] * nu;
+                        w = W_g[at];
+                        ex[a] = k_g[at];
+                    }
+                    ex[a] += f.k + t.k;
+                    g[a] = w * (f.m * t.m);
+                    if (wide) {
+                        // the reference's expression
+                        double dE = tgt_e[col] - src_e[row];
+                        if (row < N && col < N) dE -= IR / d[at];
+                        g[a] = tc[at] * (dE > 0 ? nu * exp(-dE / kT) : nu);
+                        ex[a] = INT_MIN;
+                    }
+                }
+            }
+#pragma unroll
+            for (int a = 0; a < kAhead; ++a) {
+                const int k = k0 + 32 * a + lane;
+                if (k < kwe) {
+                    // min(cap, g 2^ex): a NaN energy difference counts as
+                    // downhill, as the comparison dE > 0 has it
+                    double r = g[a];
+                    if (ex[a] != INT_MIN) {
+                        const int er = __double2hiint(r) >> 20, e = er + ex[a];
+                        if (er == 0 || (er < 2047 && e <= 0))
+                            r = scalbn(r, ex[a]);      // zero, subnormal or about to be
+                        else if (e < 2047 && er < 2047)
+                            r = __hiloint2double(__double2hiint(r) + (ex[a] << 20), __double2loint(r));
+                        else
+                            r = cap[a];
+                        if (static_cast<unsigned long long>(__double_as_longlong(r)) >
+                            static_cast<unsigned long long>(__double_as_longlong(cap[a])))
+                            r = cap[a];
+                    }
+                    rates[k] = r;
+                }
+            }
+        }
+        __syncwarp();
+        const int kb = min(kw + lane * M, kwe), ke = min(kb + M, kwe);
+        double lsum = kb < ke ? rates[kb] : 0.0;
+        for (int k = kb + 1; k < ke; ++k) lsum += rates[k];
+        double x = lsum;
+        if (kw < kwe) {
+#pragma unroll
+            for (int s = 1; s < 32; s <<= 1) {
+                const double o = __shfl_up_sync(0xffffffffu, x, s);
+                if (lane >= s) x += o;
+            }
+        }
+        incl[tid] = x;
+        __syncthreads();
+
+        // ---- warp 0: the event; warp 1: the clock; then the flux ----
+        if (warp < 2) {
+            double upto[kWarps];      // sums up to the end of each warp
+            upto[0] = incl[31];
+#pragma unroll
+            for (int w = 1; w < kWarps; ++w) upto[w] = upto[w - 1] + incl[w * 32 + 31];
+            const double total = upto[kWarps - 1];
+            if (warp == 1) {
+                const double scale = 1.0 / total;
+                const double step = u_cl[hop & 31] * scale;
+                if (lane == 0) sh_dt = step;
+                if (positive(total) && !not_less(total, __double_as_longlong(1.0e300))) time += step;
+            } else if (!positive(total) || not_less(total, __double_as_longlong(1.0e300))) {
+                if (lane == 0) ev_from = -1;      // zero, negative, infinite or NaN
+            } else {
+                const double u2 = u_ev[hop & 31];
+                // First k with cum_k/total >= u2 (the reference's test).
+                // Where cum_k is 2^13 units in the last place or more away
+                // from u2*total (over 1e-12 relative, far more than the
+                // rounding of either side), the product decides it, else a
+                // division.
+                const long long ut = __double_as_longlong(u2 * total), lo = ut - 8192, hi = ut + 8192;
+                // the first warp, then the first thread, whose last sum may pass
+                int w = 0;
+                double before = 0.0;
+#pragma unroll
+                for (int v = 0; v < kWarps - 1; ++v)
+                    if (!not_less(upto[v], lo)) { w = v + 1; before = upto[v]; }
+                double sums = before + incl[w * 32 + lane];     // up to each thread's end
+                const unsigned b = __ballot_sync(0xffffffffu, not_less(sums, lo));
+                int g = w * 32 + (b ? __ffs(b) - 1 : 31);
+                int ev = -1, last = 0;
+                double run = __shfl_sync(0xffffffffu, sums, (g - 1) & 31);
+                if (!(g & 31)) run = before;
+                for (;;) {
+                    // 32 pairs of thread g's run at a time, a lane each
+                    const int gb = g * M, ge = min(gb + M, A);
+                    for (int k0 = gb; k0 < ge && ev < 0; k0 += 32) {
+                        const int k = k0 + lane;
+                        const double r = k < ge ? rates[k] : 0.0;
+                        double x = r;
+                        const int n = min(32, ge - k0);
+                        for (int s = 1; s < n; s <<= 1) {
+                            const double o = __shfl_up_sync(0xffffffffu, x, s);
+                            if (lane >= s) x += o;
+                        }
+                        const double cum = run + x;
+                        const bool hit = k < ge && (not_less(cum, hi) || (not_less(cum, lo) && cum / total >= u2));
+                        const unsigned hits = __ballot_sync(0xffffffffu, hit);
+                        if (hits) {
+                            ev = k0 + __ffs(hits) - 1;
+                        } else {
+                            const unsigned some = __ballot_sync(0xffffffffu, positive(r));
+                            if (some) last = k0 + 31 - __clz(some);
+                            run = __shfl_sync(0xffffffffu, cum, 31);
+                        }
+                    }
+                    if (ev >= 0 || ++g >= kThreads || g * M >= A) break;
+                    // not in that run after all: the next thread's, from the
+                    // prefix it has
+                    if ((g >> 5) != w) before += incl[w++ * 32 + 31];
+                    run = (g & 31) ? before + incl[g - 1] : before;
+                }
+                // u2 within the rounding of 1: the last pair that can hop
+                if (ev < 0) ev = last;
+                int row, col;
+                if (ev < A1) row = div_small(ev, T1, inv1, col);
+                else row = N + div_small(ev - A1, T2, inv2, col);
+                if (col >= z) col += N - z;
+                if (lane == 0) {
+                    const int f = src[row].id, t = tgt[col].id;
+                    ev_from = f;
+                    ev_to = t;
+                    if (f >= N) eo_s[f - N] -= 1;
+                    if (t >= N) eo_s[t - N] += 1;
+                    // fire and forget: nothing of this launch reads it
+                    if (record) atomicAdd(&traffic[(size_t)f * S + t], 1.0);
+                    if (hop_log) { hop_log[2 * hop] = f; hop_log[2 * hop + 1] = t; }
+                }
+            }
+        }
         if (flux_time) {
-            // every rate of this state is in cum (the scan synchronised): the
-            // expected net hole flow into each electrode, column N+e minus
-            // row N+e, summed in ascending site order
-            for (int e = tid; e < P; e += kThreads) {
+            // expected net hole flow into each electrode: its column of the
+            // rate matrix minus its row
+            for (int e = kWarps - 1 - warp; e < P; e += kWarps) {
                 double in = 0.0, out = 0.0;
-                for (int i = 0; i < N; ++i) in += cum[(size_t)i * S + N + e];
-                for (int j = 0; j < N; ++j) out += cum[(size_t)(N + e) * S + j];
-                sh_flux[e] = in - out;
+                for (int r = lane; r < h; r += 32) in += rates[r * T1 + z + e];
+                for (int c = lane; c < z; c += 32) out += rates[A1 + e * T2 + c];
+                double J = in - out;
+#pragma unroll
+                for (int s = 16; s > 0; s >>= 1) J += __shfl_xor_sync(0xffffffffu, J, s);
+                if (lane == 0) sh_J[e] = J;
             }
-            __syncthreads();
         }
-        // running sums continued from the chunk's base
-        double run = base;
-        for (int k = kb; k < ke; ++k) {
-            run = (k == 0) ? cum[k] : cum[k] + run;
-            cum[k] = run;
-        }
-        if (ke == SS && kb < ke) sh_total = run;
-        if (tid == 0) ev_min = 0x7fffffff;
         __syncthreads();
-        const double total = sh_total;
-        if (!(total > 0.0) || !(total < 1.0e300)) {
+        from = ev_from;
+        if (from < 0) {
             status = KMC_ERR_NONFINITE;
             break;
         }
-        double u1, u2;
-        if (uniforms) {
-            u1 = uniforms[2 * hop];
-            u2 = uniforms[2 * hop + 1];
-        } else {
-            const u32x4 r = philox4x32_10(u32x4{static_cast<uint32_t>(hop), static_cast<uint32_t>(hop >> 32), 0u, 0u},
-                                          static_cast<uint32_t>(seed), static_cast<uint32_t>(seed >> 32));
-            u1 = u01_from64(r.x, r.y);
-            u2 = u01_from64(r.z, r.w);
-        }
-        // First k with cum_k/total >= u2 (the reference's test, one FP64
-        // division per candidate).  cum is non-decreasing, so only the chunk
-        // whose last entry passes can hold it; a chunk whose last entry is
-        // below u2*total by far more than the rounding of either side (a
-        // relative 1e-12) cannot pass and is skipped without dividing.
-        if (kb < ke && !(cum[ke - 1] < u2 * total * (1.0 - 1.0e-12))) {
-            for (int k = kb; k < ke; ++k) {
-                if (cum[k] / total >= u2) { atomicMin(&ev_min, k); break; }
-            }
-        }
-        __syncthreads();
-        if (tid == 0) {
-            int ev = ev_min;
-            if (ev == 0x7fffffff) ev = 0;   // cannot happen: cum[SS-1]/total == 1 > u2
-            const int from = ev / S, to = ev - (ev / S) * S;
-            const double scale = 1.0 / total;
-            const double hop_time = -log(1.0 - u1) * scale;
-            if (from < N) occ[from] = 0; else eo[from - N] -= 1;
-            if (to < N) occ[to] = 1; else eo[to - N] += 1;
-            if (record) traffic[(size_t)from * S + to] += 1.0;
-            if (hop_log) { hop_log[2 * hop] = from; hop_log[2 * hop + 1] = to; }
-            if (flux_time)
-                for (int e = 0; e < P; ++e) flux_time[e] += sh_flux[e] * hop_time;
-            sh_hop_time = hop_time;
-        }
-        __syncthreads();
-        const double hop_time = sh_hop_time;
-        if (record)
-            for (int i = tid; i < N; i += kThreads)
-                if (occ[i]) oit[i] += hop_time;
-        time += hop_time;
+        to = ev_to;
+        dt = sh_dt;
+        h += (to < N ? 1 : 0) - (from < N ? 1 : 0);
+        if (flux_time)
+            for (int e = tid; e < P; e += kThreads) sh_fx[e] += sh_J[e] * dt;
     }
-    for (int i = tid; i < N; i += kThreads) occ_g[i] = occ[i];
-    if (tid == 0) {
-        *time_out = time;
-        *status_out = status;
+    __syncthreads();
+    // the loop ends with the last hop not yet in the bits (an error: with
+    // the bits up to date)
+    if (status == KMC_OK && tid == 0) {
+        if (from < N) occw[from >> 5] &= ~(1u << (from & 31));
+        if (to < N) occw[to >> 5] |= 1u << (to & 31);
     }
+    __syncthreads();
+    for (int i = tid; i < N; i += kThreads) occ_g[i] = (occw[i >> 5] >> (i & 31)) & 1u;
+    if (record && tid < N) oit[tid] = oit0;
+    for (int e = tid; e < P; e += kThreads) {
+        eo[e] += eo_s[e];
+        if (flux_time) flux_time[e] = sh_fx[e];
+    }
+    if (tid == 32) *time_out = time;
+    if (tid == 0) *status_out = status;
 }
 
-__global__ void __launch_bounds__(kThreads) f64_chain_kernel(
-    int N, int P, double nu, double kT, double I0, double R, uint8_t *occ_g, const double *d,
+template <bool kTab, bool kRate>
+__global__ void __launch_bounds__(kThreads, 1) f64_chain_kernel(
+    const Layout lay, int N, int P, double nu, double kT, double I0, double R, uint8_t *occ_g, const double *d,
     const double *Ec, const double *se_in, const double *tc, int64_t *eo, int64_t hops,
     int record, double *traffic, double *oit, const double *uniforms, uint64_t seed,
     int32_t *hop_log, double *time_out, int32_t *status_out, double *ws, double *flux_time)
 {
-    f64_chain(N, P, nu, kT, I0, R, occ_g, d, Ec, se_in, tc, eo, hops, record, traffic, oit, uniforms,
-              seed, hop_log, time_out, status_out, ws, flux_time);
+    f64_chain<kTab, kRate>(lay, N, P, nu, kT, I0, R, occ_g, d, Ec, se_in, tc, eo, hops, record, traffic, oit,
+                           uniforms, seed, hop_log, time_out, status_out, ws, flux_time);
 }
 
 // Many independent chains in one launch, one block each (Philox streams
 // keyed by each chain's own seed).
-__global__ void __launch_bounds__(kThreads) f64_batch_kernel(const kmc_f64_batch B, size_t ws_doubles)
+template <bool kTab, bool kRate>
+__global__ void __launch_bounds__(kThreads, 1) f64_batch_kernel(const Layout lay, const kmc_f64_batch B,
+                                                             size_t ws_doubles)
 {
     const int c = blockIdx.x;
     const int N = B.N[c], P = B.P[c];
@@ -248,10 +600,40 @@ __global__ void __launch_bounds__(kThreads) f64_batch_kernel(const kmc_f64_batch
     double *fx = B.flux_time ? B.flux_time + eo : nullptr;
     double *tr = B.record ? B.traffic + B.traffic_off[c] : nullptr;
     double *oit = B.record ? B.occupations_in_time + so : nullptr;
-    f64_chain(N, P, B.nu[c], B.kT[c], B.I_0[c], B.R[c], B.occupation + so, B.distances + po, B.E_constant + so,
-              B.site_energies + vo, B.transitions_constant + po, B.electrode_occupation + eo, B.hops[c],
-              B.record, tr, oit, nullptr, B.seeds[c], nullptr, B.time_out + c, B.status_out + c,
-              B.workspace + (size_t)c * ws_doubles, fx);
+    f64_chain<kTab, kRate>(lay, N, P, B.nu[c], B.kT[c], B.I_0[c], B.R[c], B.occupation + so, B.distances + po,
+                           B.E_constant + so, B.site_energies + vo, B.transitions_constant + po,
+                           B.electrode_occupation + eo, B.hops[c], B.record, tr, oit, nullptr, B.seeds[c], nullptr,
+                           B.time_out + c, B.status_out + c, B.workspace + (size_t)c * ws_doubles, fx);
+}
+
+// Where a launch's arrays go: `budget` bytes of shared memory a block, for at
+// most A_max allowed pairs.  The rates first (written and read twice a hop),
+// then the pair table (two reads a pair), then 1/d (z reads a site).
+Layout f64_layout(int S, int N, int64_t A_max, size_t budget)
+{
+    Layout l{S, 0, 0, 0};
+    auto take = [&](int Layout::*part, int64_t entries) {
+        Layout t = l;
+        if (entries > (1 << 20)) return;
+        t.*part = static_cast<int>((entries + 1) & ~static_cast<int64_t>(1));
+        if (layout_bytes(t) <= budget) l = t;
+    };
+    take(&Layout::rates, A_max);
+    if (l.rates > 0) take(&Layout::tab, static_cast<int64_t>(S) * S);
+    take(&Layout::invd, static_cast<int64_t>(N) * N);
+    return l;
+}
+
+constexpr size_t kBlockSmem = 220 * 1024;    // dynamic shared memory of one block
+constexpr size_t kSmSmem = 227 * 1024;       // shared by the blocks of an SM (1 KB of each is the system's)
+
+template <typename K>
+int allow_smem(K *kernel, size_t smem)
+{
+    if (smem <= 48 * 1024) return KMC_OK;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               static_cast<int>(kBlockSmem));
+    return e == cudaSuccess ? KMC_OK : fail_cuda(e, "cudaFuncSetAttribute(f64)");
 }
 
 }  // namespace
@@ -279,15 +661,20 @@ int simulate_f64(int N, int P, double nu, double kT, double I0, double R, uint8_
         return fail(KMC_ERR_INVALID, "simulate_f64: workspace %zu bytes < %zu", ws_bytes, f64_workspace_size(S));
     if (!(kT > 0)) return fail(KMC_ERR_INVALID, "simulate_f64: kT must be positive");
     if (flux_time && P > 64) return fail(KMC_ERR_INVALID, "simulate_f64: flux_time supports at most 64 electrodes");
-    const size_t smem = sizeof(double) * (S + 32) + S + 16;
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(f64_chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             static_cast<int>(smem));
-        if (e != cudaSuccess) return fail_cuda(e, "cudaFuncSetAttribute(f64)");
-    }
-    f64_chain_kernel<<<1, kThreads, smem, st>>>(N, P, nu, kT, I0, R, occ, d, Ec, se, tc, eo, hops,
-                                                record, traffic, oit, uniforms, seed, hop_log,
-                                                time_out, status_out, static_cast<double *>(ws), flux_time);
+    // A(h) = h(N - h) + N P is largest at h = N/2
+    const Layout lay = f64_layout(S, N, static_cast<int64_t>(N) * N / 4 + static_cast<int64_t>(N) * P, kBlockSmem);
+    const size_t smem = layout_bytes(lay);
+    auto launch = [&](auto *kernel) -> int {
+        const int rc = allow_smem(kernel, smem);
+        if (rc != KMC_OK) return rc;
+        kernel<<<1, kThreads, smem, st>>>(lay, N, P, nu, kT, I0, R, occ, d, Ec, se, tc, eo, hops, record, traffic,
+                                          oit, uniforms, seed, hop_log, time_out, status_out,
+                                          static_cast<double *>(ws), flux_time);
+        return KMC_OK;
+    };
+    const int rc = lay.tab > 0 ? launch(f64_chain_kernel<true, true>)
+                   : lay.rates > 0 ? launch(f64_chain_kernel<false, true>) : launch(f64_chain_kernel<false, false>);
+    if (rc != KMC_OK) return rc;
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail_cuda(e, "f64 launch");
     return KMC_OK;
@@ -317,14 +704,27 @@ int simulate_f64_batch(const kmc_f64_batch &B, cudaStream_t st)
                     f64_batch_workspace_size(B.n_chains, B.max_sites));
     // per-chain sizes are checked by each block (KMC_ERR_INVALID in status_out)
     const int S = B.max_sites;
-    const size_t smem = sizeof(double) * (S + 32) + S + 16;
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(f64_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             static_cast<int>(smem));
-        if (e != cudaSuccess) return fail_cuda(e, "cudaFuncSetAttribute(f64 batch)");
-    }
-    f64_batch_kernel<<<B.n_chains, kThreads, smem, st>>>(B, f64_workspace_size(S) / sizeof(double));
-    cudaError_t e = cudaGetLastError();
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return fail_cuda(e, "simulate_f64_batch: device query");
+    // Blocks that share an SM overlap their serial phases, so a launch of
+    // more chains than SMs divides an SM's shared memory among up to four.
+    const int per_sm = std::max(1, std::min(4, (B.n_chains + sms - 1) / std::max(sms, 1)));
+    // A(h) <= S^2/3 for any split of S sites into acceptors and electrodes
+    const Layout lay = f64_layout(S, S, static_cast<int64_t>(S) * S / 3 + 1,
+                                  std::min(kBlockSmem, kSmSmem / per_sm - 1280));
+    const size_t smem = layout_bytes(lay);
+    auto launch = [&](auto *kernel) -> int {
+        const int rc = allow_smem(kernel, smem);
+        if (rc != KMC_OK) return rc;
+        kernel<<<B.n_chains, kThreads, smem, st>>>(lay, B, f64_workspace_size(S) / sizeof(double));
+        return KMC_OK;
+    };
+    const int rc = lay.tab > 0 ? launch(f64_batch_kernel<true, true>)
+                   : lay.rates > 0 ? launch(f64_batch_kernel<false, true>) : launch(f64_batch_kernel<false, false>);
+    if (rc != KMC_OK) return rc;
+    e = cudaGetLastError();
     return e == cudaSuccess ? KMC_OK : fail_cuda(e, "f64 batch launch");
 }
 
@@ -396,8 +796,12 @@ namespace kmc {
 int preload_f64()
 {
     int rc;
-    if ((rc = touch_kernel(f64_chain_kernel)) != KMC_OK) return rc;
-    return touch_kernel(f64_batch_kernel);
+    if ((rc = touch_kernel(f64_chain_kernel<true, true>)) != KMC_OK) return rc;
+    if ((rc = touch_kernel(f64_chain_kernel<false, true>)) != KMC_OK) return rc;
+    if ((rc = touch_kernel(f64_chain_kernel<false, false>)) != KMC_OK) return rc;
+    if ((rc = touch_kernel(f64_batch_kernel<true, true>)) != KMC_OK) return rc;
+    if ((rc = touch_kernel(f64_batch_kernel<false, true>)) != KMC_OK) return rc;
+    return touch_kernel(f64_batch_kernel<false, false>);
 }
 
 }  // namespace kmc

@@ -144,6 +144,18 @@ __device__ __forceinline__ uint64_t globaltimer_ns()
     return t;
 }
 
+// x as a double.  The conversion instruction runs on the FP64 unit (93 cycles
+// measured, and the add that uses it waits); the bits of a normal number
+// move with integer instructions.
+__device__ __forceinline__ double widen(float x)
+{
+    const uint32_t b = __float_as_uint(x), a = b & 0x7fffffffu;
+    if (a - 0x00800000u < 0x7f000000u)
+        return __hiloint2double(static_cast<int>((b & 0x80000000u) | ((a >> 3) + 0x38000000u)),
+                                static_cast<int>(b << 29));
+    return static_cast<double>(x);
+}
+
 __device__ __forceinline__ float rsqrt_approx(float x)
 {
     float y;
@@ -242,6 +254,27 @@ __device__ __forceinline__ uint64_t u01_fixed_from_double(double u)
 {
     return __double2ull_rz(u * 0x1.0p64);
 }
+
+// Which thread's run holds the event, and what remains of u*total there.
+struct Selection {
+    int L = -1;
+    float rem = 0.0f;
+    float totf = 0.0f;
+    int emax = 0;
+    bool ok = false;
+    // the scale from the bit pattern of the largest sum (positive FP32 values
+    // order as their bit patterns; NaN and infinity sit above every finite one)
+    __device__ __forceinline__ bool scale(uint32_t mx)
+    {
+        emax = static_cast<int>(mx >> 23);
+        return mx != 0u && mx < 0x7f800000u;
+    }
+    __device__ __forceinline__ bool total(uint64_t tot, int shift)
+    {
+        totf = from_fixed(tot, emax, shift);
+        return ok = totf <= 3.0e38f;
+    }
+};
 
 // Exact n / T for 0 <= n < 2^22 from inv ~ 1/T (float reciprocal, one
 // correction step), as in decode_pair below.
@@ -538,9 +571,73 @@ struct WarpGroup {
         tot = __shfl_sync(mask, x, G - 1, G);
         return x;
     }
+    // The event's thread: exact fixed-point scan of the group's sums (see
+    // Selection).
+    __device__ __forceinline__ Selection select(float lsum, uint64_t u_ev, bool has_run) const
+    {
+        constexpr int kShift = FixShift<G>::kShift;
+        Selection r;
+        if (!r.scale(max_u32(__float_as_uint(lsum)))) return r;
+        uint64_t excl, tot;
+        const uint64_t incl = scan_u64(to_fixed(lsum, r.emax, kShift), excl, tot);
+        if (!r.total(tot, kShift)) return r;
+        // thread L's run holds the first pair whose cumulative rate reaches
+        // u*total (tot >= target, so some thread qualifies)
+        const uint64_t target = fixed_target(u_ev, tot);
+        r.L = first(incl >= target);
+        if (r.L < 0) r.L = last(has_run);
+        // what remains of u*total beyond the runs before L, back in FP32
+        r.rem = bcast(from_fixed(target - excl, r.emax, kShift), r.L);
+        return r;
+    }
+    __device__ __forceinline__ int scan_hit(float r, bool pos, float rem, int &last_pos, float &tot) const
+    {
+        const float q = scanf(r, tot);
+        const int hit = first(pos && q >= rem);
+        last_pos = hit >= 0 ? -1 : last(pos);
+        return hit;
+    }
+    // the first of the n stored sums at p, stride RS, that reaches rem, or -1:
+    // thread g tests elements g, g + G, ..., a chunk of G elements per round
+    // with both rounds' loads issued first (the sums do not decrease, so the
+    // lowest element of the first chunk with a hit is the one)
+    template <int RS>
+    __device__ __forceinline__ int search(const float *p, int n, float rem) const
+    {
+        for (int i0 = 0; i0 < n; i0 += 2 * G) {
+            const int ia = i0 + g, ib = i0 + G + g;
+            const float va = ia < n ? p[ia * RS] : -1.0f;
+            const float vb = ib < n ? p[ib * RS] : -1.0f;
+            const int ha = first(va >= rem);
+            const int hb = first(vb >= rem);
+            if (ha >= 0) return i0 + ha;
+            if (hb >= 0) return i0 + G + hb;
+        }
+        return -1;
+    }
+    template <typename V>
+    __device__ __forceinline__ V lane_value(V v, int src) const { return bcast(v, src); }
+    __device__ __forceinline__ bool keeps_clock() const { return true; }
 };
 
-// Block-wide group; its scratch lives in static shared memory.
+// Static shared memory of a block-wide group.
+template <int T>
+struct BlockScratch {
+    static constexpr int kWarps = T / 32;
+    alignas(16) uint64_t sums[T];   // per-thread sums (BlockGroup::select)
+    float chunk[kWarps];            // warp sums of a chunk (scan_hit)
+    int2 hits[kWarps];              // first hit, last positive rate of a warp's part of a chunk
+    uint32_t wmax[kWarps];
+    double sd[kWarps + 2];
+    int si[2];
+};
+
+// Block-wide group.  Each call of a collective below costs its barriers, 24
+// to 54 cycles for 1 to 16 warps plus the skew of the warps that wait, and a
+// hop that ran them one after another spent more time there than on its
+// pairs (N = 30 alone: 23 barriers).  The hop loop therefore publishes the
+// per-thread sums once and lets every warp repeat the rest of the selection
+// by itself (select, and the search of one run's stored sums).
 template <int T>
 struct BlockGroup {
     static constexpr int kSize = T;
@@ -548,6 +645,164 @@ struct BlockGroup {
     int g;
     double *sd;   // [kWarps + 2]
     int *si;      // [2]
+    BlockScratch<T> *sc;
+
+    // The event's thread: exact fixed-point scan of the group's sums (see
+    // Selection).  Synchronises the block once (up to 128 threads: every warp
+    // reads all sums, T/32 a lane) or twice (each thread converts its own
+    // sum, which needs the largest one first).
+    __device__ __forceinline__ Selection select(float lsum, uint64_t u_ev, bool /*has_run*/) const
+    {
+        constexpr int kShift = FixShift<T>::kShift;
+        const int lane = g & 31;
+        Selection r;
+        if constexpr (T <= 128) {
+            constexpr int K = T / 32;
+            float *s = reinterpret_cast<float *>(sc->sums);
+            s[g] = lsum;
+            __syncthreads();
+            float v[K];
+            if constexpr (K == 2) {
+                const float2 q = reinterpret_cast<const float2 *>(s)[lane];
+                v[0] = q.x;
+                v[1] = q.y;
+            } else {
+                const float4 q = reinterpret_cast<const float4 *>(s)[lane];
+                v[0] = q.x;
+                v[1] = q.y;
+                v[2] = q.z;
+                v[3] = q.w;
+            }
+            uint32_t m = __float_as_uint(v[0]);
+#pragma unroll
+            for (int i = 1; i < K; ++i) m = max(m, __float_as_uint(v[i]));
+            const uint32_t mx = __reduce_max_sync(0xffffffffu, m);
+            if (!r.scale(mx)) return r;
+            uint64_t f[K], x = 0;
+#pragma unroll
+            for (int i = 0; i < K; ++i) {
+                f[i] = to_fixed(v[i], r.emax, kShift);
+                x += f[i];
+            }
+            const uint64_t own = x;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const uint64_t o = __shfl_up_sync(0xffffffffu, x, d);
+                if (lane >= d) x += o;
+            }
+            const uint64_t tot = __shfl_sync(0xffffffffu, x, 31);
+            if (!r.total(tot, kShift)) return r;
+            const uint64_t target = fixed_target(u_ev, tot);
+            // the first lane that reaches the target, and its first sum that
+            // does (the total reaches it, so there is one)
+            const int at = __ffs(__ballot_sync(0xffffffffu, x >= target)) - 1;
+            uint64_t base = x - own;
+            int k = 0;
+#pragma unroll
+            for (int i = 0; i < K - 1; ++i)
+                if (k == i && base + f[i] < target) {
+                    base += f[i];
+                    k = i + 1;
+                }
+            r.L = __shfl_sync(0xffffffffu, lane * K + k, at);
+            r.rem = __shfl_sync(0xffffffffu, from_fixed(target - base, r.emax, kShift), at);
+        } else {
+            const uint32_t wm = __reduce_max_sync(0xffffffffu, __float_as_uint(lsum));
+            if (lane == 0) sc->wmax[g >> 5] = wm;
+            __syncthreads();
+            const uint32_t mx = __reduce_max_sync(0xffffffffu, lane < kWarps ? sc->wmax[lane] : 0u);
+            if (!r.scale(mx)) return r;
+            uint64_t x = to_fixed(lsum, r.emax, kShift);
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const uint64_t o = __shfl_up_sync(0xffffffffu, x, d);
+                if (lane >= d) x += o;
+            }
+            sc->sums[g] = x;
+            __syncthreads();
+            uint64_t y = lane < kWarps ? sc->sums[lane * 32 + 31] : 0ull;
+#pragma unroll
+            for (int d = 1; d < kWarps; d <<= 1) {
+                const uint64_t o = __shfl_up_sync(0xffffffffu, y, d);
+                if (lane >= d) y += o;
+            }
+            const uint64_t tot = __shfl_sync(0xffffffffu, y, kWarps - 1);
+            if (!r.total(tot, kShift)) return r;
+            const uint64_t target = fixed_target(u_ev, tot);
+            const int w = __ffs(__ballot_sync(0xffffffffu, lane < kWarps && y >= target)) - 1;
+            uint64_t base = __shfl_sync(0xffffffffu, y, (w - 1) & 31);
+            if (w == 0) base = 0;
+            x = base + sc->sums[w * 32 + lane];
+            const int at = __ffs(__ballot_sync(0xffffffffu, x >= target)) - 1;
+            const uint64_t prev = __shfl_sync(0xffffffffu, x, (at - 1) & 31);
+            if (at > 0) base = prev;
+            r.L = w * 32 + at;
+            r.rem = from_fixed(target - base, r.emax, kShift);
+        }
+        return r;
+    }
+
+    // One chunk of a re-evaluated run, thread g holding element g's rate r
+    // (positive: pos): the first element whose running sum reaches rem, the
+    // last positive one (-1: none) and the chunk's sum.  The running sums
+    // associate as scanf's do.
+    __device__ __forceinline__ int scan_hit(float r, bool pos, float rem, int &last_pos, float &tot) const
+    {
+        const int lane = g & 31, w = g >> 5;
+        float x = r;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const float o = __shfl_up_sync(0xffffffffu, x, d);
+            if (lane >= d) x += o;
+        }
+        if (lane == 31) sc->chunk[w] = x;
+        __syncthreads();
+        float y = lane < kWarps ? sc->chunk[lane] : 0.0f;
+#pragma unroll
+        for (int d = 1; d < kWarps; d <<= 1) {
+            const float o = __shfl_up_sync(0xffffffffu, y, d);
+            if (lane >= d) y += o;
+        }
+        tot = __shfl_sync(0xffffffffu, y, kWarps - 1);
+        const float before = __shfl_sync(0xffffffffu, y, (w - 1) & 31);
+        const float q = x + (w > 0 ? before : 0.0f);
+        const unsigned hb = __ballot_sync(0xffffffffu, pos && q >= rem);
+        const unsigned pb = __ballot_sync(0xffffffffu, pos);
+        if (lane == 0)
+            sc->hits[w] = make_int2(hb ? w * 32 + __ffs(hb) - 1 : -1, pb ? w * 32 + 31 - __clz(pb) : -1);
+        __syncthreads();
+        const int2 h = lane < kWarps ? sc->hits[lane] : make_int2(-1, -1);
+        const unsigned hw = __ballot_sync(0xffffffffu, h.x >= 0);
+        last_pos = static_cast<int>(__reduce_max_sync(0xffffffffu, static_cast<unsigned>(h.y + 1))) - 1;
+        return hw ? __shfl_sync(0xffffffffu, h.x, __ffs(hw) - 1) : -1;
+    }
+
+    // the first of the n stored sums at p, stride RS, that reaches rem, or -1
+    // (they do not decrease): every warp narrows the range 32-fold a round
+    template <int RS>
+    __device__ __forceinline__ int search(const float *p, int n, float rem) const
+    {
+        const int lane = g & 31;
+        int lo = 0;
+        while (n > 32) {
+            const int q = (n + 31) >> 5;
+            const float v = p[(lo + min((lane + 1) * q, n) - 1) * RS];
+            const unsigned b = __ballot_sync(0xffffffffu, v >= rem);
+            if (!b) return -1;
+            const int skip = (__ffs(b) - 1) * q;
+            lo += skip;
+            n = min(q, n - skip);
+        }
+        const float v = lane < n ? p[(lo + lane) * RS] : -1.0f;
+        const unsigned b = __ballot_sync(0xffffffffu, v >= rem);
+        return b ? lo + __ffs(b) - 1 : -1;
+    }
+
+    // a per-lane value that every warp holds alike
+    template <typename V>
+    __device__ __forceinline__ V lane_value(V v, int src) const { return __shfl_sync(0xffffffffu, v, src); }
+    // whether this thread keeps the chain's clock
+    __device__ __forceinline__ bool keeps_clock() const { return g < 32; }
     __device__ __forceinline__ void init() { g = threadIdx.x; }
     __device__ __forceinline__ void sync() const { __syncthreads(); }
     __device__ float scanf(float v, float &tot) const
@@ -643,35 +898,6 @@ struct BlockGroup {
         for (int k = 1; k < kWarps; ++k) m = max(m, s[k]);
         __syncthreads();
         return m;
-    }
-    __device__ uint64_t scan_u64(uint64_t v, uint64_t &excl, uint64_t &tot) const
-    {
-        const int lane = g & 31, w = g >> 5;
-        uint64_t x = v;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const uint64_t o = __shfl_up_sync(0xffffffffu, x, d);
-            if (lane >= d) x += o;
-        }
-        uint64_t *s = reinterpret_cast<uint64_t *>(sd);   // kWarps slots
-        if (lane == 31) s[w] = x;
-        __syncthreads();
-        if (w == 0) {
-            uint64_t y = lane < kWarps ? s[lane] : 0ull;
-#pragma unroll
-            for (int d = 1; d < kWarps; d <<= 1) {
-                const uint64_t o = __shfl_up_sync(0xffffffffu, y, d);
-                if (lane >= d) y += o;
-            }
-            if (lane < kWarps) s[lane] = y;
-        }
-        __syncthreads();
-        const uint64_t base = w > 0 ? s[w - 1] : 0ull;
-        tot = s[kWarps - 1];
-        __syncthreads();
-        x += base;
-        excl = x - v;
-        return x;
     }
     template <typename V>
     __device__ V bcast(V v, int src) const
@@ -1113,29 +1339,21 @@ __device__ void run_chain(const kmc_batch &B, const Grp &grp, ChainSmem<typename
                 rnd_u = u01_fixed(w.y, w.z);
             }
             const int ri = static_cast<int>(hop - rbase);
-            e1 = grp.bcast(rnd_e1, ri);
-            u_ev = grp.bcast(rnd_u, ri);
+            // (in a block group every warp holds the same 32 hops' draws)
+            e1 = grp.lane_value(rnd_e1, ri);
+            u_ev = grp.lane_value(rnd_u, ri);
         }
-        if (stored) grp.sync();   // stored rates visible to the whole group
+        // the stored sums become visible to the whole group (a block group's
+        // select synchronises it)
+        if (G <= 32 && stored) grp.sync();
         KMC_SECTION(2);
-        // ---- exact fixed-point scan of the per-thread sums ----
-        // scale: the largest per-thread sum (positive FP32 values order as
-        // their bit patterns; NaN and infinity sit above every finite value)
-        const uint32_t mx = grp.max_u32(__float_as_uint(lsum));
-        if (mx == 0u || mx >= 0x7f800000u) { status = KMC_ERR_NONFINITE; break; }
-        constexpr int kShift = FixShift<G>::kShift;
-        const int emax = static_cast<int>(mx >> 23);
-        uint64_t excl, tot;
-        const uint64_t incl = grp.scan_u64(to_fixed(lsum, emax, kShift), excl, tot);
-        const float totf = from_fixed(tot, emax, kShift);
-        if (!(totf <= 3.0e38f)) { status = KMC_ERR_NONFINITE; break; }
-        // the event is the first pair whose cumulative rate reaches u*total:
-        // thread L's run holds it (tot >= target, so some thread qualifies)
-        const uint64_t target = fixed_target(u_ev, tot);
-        int L = grp.first(incl >= target);
-        if (L < 0) L = grp.last(run_e > run_b);
-        // what remains of u*total beyond the runs before L, back in FP32
-        float rem = grp.bcast(from_fixed(target - excl, emax, kShift), L);
+        // ---- exact fixed-point scan of the per-thread sums: the event is
+        // the first pair whose cumulative rate reaches u*total ----
+        const Selection sel = grp.select(lsum, u_ev, run_e > run_b);
+        if (!sel.ok) { status = KMC_ERR_NONFINITE; break; }
+        const float totf = sel.totf;
+        const int L = sel.L;
+        float rem = sel.rem;
         KMC_SECTION(3);
         // ---- find the event inside thread L's run ----
         int chosen = -1, last_pos = -1;
@@ -1143,24 +1361,10 @@ __device__ void run_chain(const kmc_batch &B, const Grp &grp, ChainSmem<typename
         int kbL, keL;
         run_of(L, kbL, keL);
         if (stored) {
-            // Thread L kept its running sums: the event is the first pair whose
-            // sum reaches rem.  Each thread of the group searches one block of
-            // them; the lowest block with a hit wins.
+            // Thread L kept its running sums: the event is the first pair
+            // whose sum reaches rem.
             const int len = keL - kbL;
-            // Thread g tests elements g, g + G, ... of thread L's run, a chunk
-            // of G elements per round with both rounds' loads issued first;
-            // the running sums do not decrease, so the lowest element of the
-            // first chunk with a hit is the event.
-            int idx = -1;
-            for (int i0 = 0; i0 < len && idx < 0; i0 += 2 * G) {
-                const int ia = i0 + g, ib = i0 + G + g;
-                const float va = ia < len ? sm.rates[ia * RS + L] : -1.0f;
-                const float vb = ib < len ? sm.rates[ib * RS + L] : -1.0f;
-                const int ha = grp.first(va >= rem);
-                const int hb = grp.first(vb >= rem);
-                if (ha >= 0) idx = i0 + ha;
-                else if (hb >= 0) idx = i0 + G + hb;
-            }
+            const int idx = grp.template search<RS>(sm.rates + L, len, rem);
             if (idx >= 0) {
                 chosen = kbL + idx;
             } else if (len > 0) {
@@ -1184,11 +1388,9 @@ __device__ void run_chain(const kmc_batch &B, const Grp &grp, ChainSmem<typename
                     r = pairs.rate(sm.src[row], tgt_load<Pairs>(sm.tgt, col), row < h && col < z, cs);
                 }
                 float ctot;
-                const float q = grp.scanf(r, ctot);
-                const bool pos = (i < len) && (r > 0.0f);
-                const int hit = grp.first(pos && q >= rem);
+                int lp;
+                const int hit = grp.scan_hit(r, (i < len) && (r > 0.0f), rem, lp, ctot);
                 if (hit >= 0) { chosen = kb + i0 + hit; break; }
-                const int lp = grp.last(pos);
                 if (lp >= 0) last_pos = kb + i0 + lp;
                 rem -= ctot;
             }
@@ -1246,7 +1448,7 @@ __device__ void run_chain(const kmc_batch &B, const Grp &grp, ChainSmem<typename
         // ---- clock ----
         const float dt = e1 * rcp_approx(totf);
         const double t_before = t;
-        t += static_cast<double>(dt);
+        if (grp.keeps_clock()) t += widen(dt);
         if (B.flux_time) {
             // Expected net hole flow into each electrode in this state,
             // J_e = sum_holes rate(i -> e) - sum_empty rate(e -> j), times
@@ -1342,7 +1544,7 @@ __device__ void run_chain(const kmc_batch &B, const Grp &grp, ChainSmem<typename
 #endif
     // ---- write back ----
     if (record) {
-        const double td = t;
+        const double td = G > 32 ? grp.bcast(t, 0) : t;
         for (int j = g; j < N; j += G)
             if ((sm.occw[j >> 5] >> (j & 31)) & 1u) {
                 occ_time[j] += td - occ_since[j];
@@ -1448,19 +1650,22 @@ __global__ void __launch_bounds__(256, MinBlocks) warp_engine_kernel(const kmc_b
     run_chain<WarpGroup<G>, Pairs>(B, grp, sm, c, stab);
 }
 
-// Block kernel: one chain per block of T threads.
+// Block kernel: one chain per block of T threads.  512 / T blocks an SM leave
+// 128 registers a thread; without the bound the compiler took 64 or 72 for
+// the positions kernels and spilled 150 to 390 bytes inside the hop loop.
 template <int T, typename Pairs>
-__global__ void __launch_bounds__(T) block_engine_kernel(const kmc_batch B, int rate_words,
+__global__ void __launch_bounds__(T, 512 / T) block_engine_kernel(const kmc_batch B, int rate_words,
                                                          int table_words)
 {
     extern __shared__ __align__(16) uint32_t smem[];
-    __shared__ double scratch[T / 32 + 2];
-    __shared__ int iscratch[2];
+    __shared__ BlockScratch<T> scratch;
+    int *iscratch = scratch.si;
     const float2 *stab = stage_table(B, smem, table_words);
     BlockGroup<T> grp;
     grp.init();
-    grp.sd = scratch;
-    grp.si = iscratch;
+    grp.sd = scratch.sd;
+    grp.si = scratch.si;
+    grp.sc = &scratch;
     using Rec = typename Pairs::Rec;
     ChainSmem<Rec> sm = carve<Rec>(smem + table_words, B.max_sites, rate_words);
     if (B.work_counter) {

@@ -1,6 +1,7 @@
-// kmc_f32_engine.cuh -- batched FP32 hop-loop engine for sm_103a (the
-// kernels; kmc_f32_*.cu instantiate them, kmc_f32.cu validates and
-// dispatches a launch).
+// kmc_f32_engine.cuh -- batched FP32 hop-loop engine for sm_103a: what its
+// kernels share, and the block-group kernel (kmc_f32_warp.cuh: the warp-slice
+// kernel; kmc_f32_*.cu instantiate them, kmc_f32.cu validates and dispatches
+// a launch).
 //
 // A chain is run by a group of threads: a G-lane slice of a warp (G = 4, 8,
 // 16, 32; 32/G chains per warp) for small networks, or a whole thread block
@@ -105,6 +106,11 @@ inline int section_clocks_read(uint64_t *out, int reset)
 #else
 #define KMC_SECTION(k) do { } while (0)
 #endif
+
+#ifndef KMC_PAIR_STEP
+#define KMC_PAIR_STEP 4
+#endif
+constexpr int kPairStep = KMC_PAIR_STEP;
 
 #ifndef KMC_PAIR_UNROLL
 #define KMC_PAIR_UNROLL 4
@@ -367,7 +373,7 @@ struct TablePairs {
     __device__ __forceinline__ Rec rec(int site, float e) const { return make_int2(site, __float_as_int(e)); }
     __device__ __forceinline__ float rate(Rec s, Rec t, bool /*acc*/, float cs) const
     {
-        const float2 lb = tab[s.x * S + t.x];
+        const float2 lb = kStaged ? tab[s.x * S + t.x] : __ldg(&tab[s.x * S + t.x]);
         const float d = __int_as_float(t.y) - __int_as_float(s.y);
         const float lcb = kUniform ? lb.y : fmaf(cs, lb.y, lb.x);
         return ex2_approx(fminf(lb.x, lcb - d));
@@ -378,7 +384,7 @@ struct TablePairs {
     // Coulomb term I_0 R / d_jk between acceptors j, k (0 on the diagonal).
     __device__ __forceinline__ float coulomb(int j, int k) const
     {
-        return kUniform ? coul[j * S + k] : tab[j * S + k].y;
+        return kUniform ? coul[j * S + k] : kStaged ? tab[j * S + k].y : __ldg(&tab[j * S + k].y);
     }
 };
 
@@ -492,133 +498,83 @@ __device__ __forceinline__ void tgt_store(typename Pairs::Rec *t, int col, const
     }
 }
 
-// ---------------------------------------------------------------------------
-// Thread groups: a G-lane slice of a warp, or a whole block
-// ---------------------------------------------------------------------------
-
-template <int G>
-struct WarpGroup {
-    static constexpr int kSize = G;
-    int g;            // rank in the group
-    int sub;          // group index within the warp
-    unsigned mask;
-    __device__ __forceinline__ void init()
+// The pair enumeration of one state.
+struct PairRange {
+    int h, z, P;         // holes, empty acceptors, electrodes
+    int T1, T2, A1, A;   // targets of a hole row / an electrode row, pairs of the hole rows, all pairs
+    float inv1, inv2;    // 1/T1, 1/T2
+    __device__ __forceinline__ void init(int h_, int N, int P_)
     {
-        const int lane = threadIdx.x & 31;
-        sub = lane / G;
-        g = lane % G;
-        mask = (G == 32 ? 0xffffffffu : ((1u << G) - 1u)) << (sub * G);
+        h = h_;
+        P = P_;
+        z = N - h_;
+        T1 = z + P;
+        T2 = z;
+        A1 = h * T1;
+        A = A1 + P * T2;
+        inv1 = T1 > 0 ? rcp_approx(static_cast<float>(T1)) : 0.0f;
+        inv2 = T2 > 0 ? rcp_approx(static_cast<float>(T2)) : 0.0f;
     }
-    __device__ __forceinline__ void sync() const { __syncwarp(mask); }
-    __device__ __forceinline__ float scanf(float v, float &tot) const
-    {
-        float x = v;
-#pragma unroll
-        for (int d = 1; d < G; d <<= 1) {
-            const float o = __shfl_up_sync(mask, x, d, G);
-            if (g >= d) x += o;
-        }
-        tot = __shfl_sync(mask, x, G - 1, G);
-        return x;
-    }
-    // lowest / highest rank with p true, or -1
-    __device__ __forceinline__ int first(bool p) const
-    {
-        const unsigned low = (G == 32) ? 0xffffffffu : ((1u << G) - 1u);
-        const unsigned b = (__ballot_sync(mask, p) >> (sub * G)) & low;
-        return b ? __ffs(b) - 1 : -1;
-    }
-    __device__ __forceinline__ int last(bool p) const
-    {
-        const unsigned low = (G == 32) ? 0xffffffffu : ((1u << G) - 1u);
-        const unsigned b = (__ballot_sync(mask, p) >> (sub * G)) & low;
-        return b ? 31 - __clz(b) : -1;
-    }
-    template <typename V>
-    __device__ __forceinline__ V bcast(V v, int src) const { return __shfl_sync(mask, v, src, G); }
-    __device__ __forceinline__ uint32_t max_u32(uint32_t v) const { return __reduce_max_sync(mask, v); }
-    __device__ __forceinline__ float sumf(float v) const
-    {
-#pragma unroll
-        for (int d = G / 2; d >= 1; d >>= 1) v += __shfl_xor_sync(mask, v, d, G);
-        return v;
-    }
-#ifdef KMC_DEBUG_CHECKS
-    // FP64 inclusive scan (debug builds: the cross-check of the selection)
-    __device__ double scan_f64(double v, double &excl, double &tot) const
-    {
-        double x = v;
-        for (int d = 1; d < G; d <<= 1) {
-            const double o = __shfl_up_sync(mask, x, d, G);
-            if (g >= d) x += o;
-        }
-        const double e = __shfl_up_sync(mask, x, 1, G);
-        excl = g == 0 ? 0.0 : e;
-        tot = __shfl_sync(mask, x, G - 1, G);
-        return x;
-    }
-#endif
-    // inclusive integer scan; sets the exclusive value and the total
-    __device__ __forceinline__ uint64_t scan_u64(uint64_t v, uint64_t &excl, uint64_t &tot) const
-    {
-        uint64_t x = v;
-#pragma unroll
-        for (int d = 1; d < G; d <<= 1) {
-            const uint64_t o = __shfl_up_sync(mask, x, d, G);
-            if (g >= d) x += o;
-        }
-        excl = x - v;
-        tot = __shfl_sync(mask, x, G - 1, G);
-        return x;
-    }
-    // The event's thread: exact fixed-point scan of the group's sums (see
-    // Selection).
-    __device__ __forceinline__ Selection select(float lsum, uint64_t u_ev, bool has_run) const
-    {
-        constexpr int kShift = FixShift<G>::kShift;
-        Selection r;
-        if (!r.scale(max_u32(__float_as_uint(lsum)))) return r;
-        uint64_t excl, tot;
-        const uint64_t incl = scan_u64(to_fixed(lsum, r.emax, kShift), excl, tot);
-        if (!r.total(tot, kShift)) return r;
-        // thread L's run holds the first pair whose cumulative rate reaches
-        // u*total (tot >= target, so some thread qualifies)
-        const uint64_t target = fixed_target(u_ev, tot);
-        r.L = first(incl >= target);
-        if (r.L < 0) r.L = last(has_run);
-        // what remains of u*total beyond the runs before L, back in FP32
-        r.rem = bcast(from_fixed(target - excl, r.emax, kShift), r.L);
-        return r;
-    }
-    __device__ __forceinline__ int scan_hit(float r, bool pos, float rem, int &last_pos, float &tot) const
-    {
-        const float q = scanf(r, tot);
-        const int hit = first(pos && q >= rem);
-        last_pos = hit >= 0 ? -1 : last(pos);
-        return hit;
-    }
-    // the first of the n stored sums at p, stride RS, that reaches rem, or -1:
-    // thread g tests elements g, g + G, ..., a chunk of G elements per round
-    // with both rounds' loads issued first (the sums do not decrease, so the
-    // lowest element of the first chunk with a hit is the one)
-    template <int RS>
-    __device__ __forceinline__ int search(const float *p, int n, float rem) const
-    {
-        for (int i0 = 0; i0 < n; i0 += 2 * G) {
-            const int ia = i0 + g, ib = i0 + G + g;
-            const float va = ia < n ? p[ia * RS] : -1.0f;
-            const float vb = ib < n ? p[ib * RS] : -1.0f;
-            const int ha = first(va >= rem);
-            const int hb = first(vb >= rem);
-            if (ha >= 0) return i0 + ha;
-            if (hb >= 0) return i0 + G + hb;
-        }
-        return -1;
-    }
-    template <typename V>
-    __device__ __forceinline__ V lane_value(V v, int src) const { return bcast(v, src); }
-    __device__ __forceinline__ bool keeps_clock() const { return true; }
 };
+
+// Walks pairs [b, e) in row-major order, kPairStep pairs a step: all loads
+// and rates of a step come before its stores, because the compiler moves no
+// list or table load across a store of the running sums, and a step's latency
+// (two dependent shared loads and an ex2) is then paid once for kPairStep
+// pairs instead of for every two.  A row change is a select plus a predicated
+// reload of the source record, not a branch.  kSum: the rates add up in s, in
+// order; kKeep: the sum (without kSum the rate) of every pair goes to rp,
+// rp + kStride, ...  Measured with 2, 4 and 8 pairs a
+// step: 4096 N=30 chains (staged table) 32.0 / 31.9 / 33.1 ms, a search
+// population of 384 networks (tables in L2) 95.7 / 79.3 / 77.2 ms, one N=100
+// chain 24.1 / 23.1 / 24.8 ms.  (Two phases, all rates by the whole group in
+// coalesced order and then each thread's sums, measured 37 to 39 ms on the
+// N=30 chains: fewer bank conflicts, more instructions.)
+template <bool kSum, bool kKeep, int kStride, int kStep, typename Pairs>
+__device__ __forceinline__ void walk_pairs(const Pairs &pairs, const typename Pairs::Rec *src,
+                                           const typename Pairs::Rec *tgt, const PairRange &R, int b, int e, float cs,
+                                           float *rp, float &s)
+{
+    int row, col;
+    decode_pair(b, R.h, R.A1, R.T1, R.T2, R.inv1, R.inv2, row, col);
+    bool sa = row < R.h;
+    int Tc = sa ? R.T1 : R.T2;
+    typename Pairs::Rec sr = src[row];
+    auto step = [&](auto whole, int left) {
+        constexpr bool kWhole = decltype(whole)::value;
+        float r[kStep];
+#pragma unroll
+        for (int u = 0; u < kStep; ++u) {
+            if (kWhole || u < left) {
+                r[u] = pairs.rate(sr, tgt_load<Pairs>(tgt, col), sa && col < R.z, cs);
+                // (the row after a last pair is not read)
+                const bool w = (col + 1 == Tc);
+                col = w ? 0 : col + 1;
+                row += w ? 1 : 0;
+                if (w && (kWhole || u + 1 < left)) sr = src[row];
+                sa = row < R.h;
+                Tc = sa ? R.T1 : R.T2;
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kStep; ++u) {
+            if (kWhole || u < left) {
+                if constexpr (kSum) s += r[u];
+                if constexpr (kKeep) rp[u * kStride] = kSum ? s : r[u];
+            }
+        }
+    };
+    int k = b;
+    for (; k + kStep <= e; k += kStep) {
+        step(BoolC<true>{}, kStep);
+        if constexpr (kKeep) rp += kStep * kStride;
+    }
+    if (k < e) step(BoolC<false>{}, e - k);
+}
+
+// ---------------------------------------------------------------------------
+// Block-wide thread groups
+// ---------------------------------------------------------------------------
 
 // Static shared memory of a block-wide group.
 template <int T>
@@ -651,7 +607,7 @@ struct BlockGroup {
     // Selection).  Synchronises the block once (up to 128 threads: every warp
     // reads all sums, T/32 a lane) or twice (each thread converts its own
     // sum, which needs the largest one first).
-    __device__ __forceinline__ Selection select(float lsum, uint64_t u_ev, bool /*has_run*/) const
+    __device__ __forceinline__ Selection select(float lsum, uint64_t u_ev) const
     {
         constexpr int kShift = FixShift<T>::kShift;
         const int lane = g & 31;
@@ -798,11 +754,6 @@ struct BlockGroup {
         return b ? lo + __ffs(b) - 1 : -1;
     }
 
-    // a per-lane value that every warp holds alike
-    template <typename V>
-    __device__ __forceinline__ V lane_value(V v, int src) const { return __shfl_sync(0xffffffffu, v, src); }
-    // whether this thread keeps the chain's clock
-    __device__ __forceinline__ bool keeps_clock() const { return g < 32; }
     __device__ __forceinline__ void init() { g = threadIdx.x; }
     __device__ __forceinline__ void sync() const { __syncthreads(); }
     __device__ float scanf(float v, float &tot) const
@@ -987,7 +938,7 @@ __device__ __forceinline__ ChainSmem<Rec> carve(uint32_t *base, int S, int rate_
 }
 
 // ---------------------------------------------------------------------------
-// The hop loop of one chain, run by one group
+// The hop loop of one chain, run by one block
 // ---------------------------------------------------------------------------
 
 template <typename Grp, typename Pairs>
@@ -1066,17 +1017,11 @@ __device__ void run_chain(const kmc_batch &B, const Grp &grp, ChainSmem<typename
     // last anchor are compared with the recomputed ones first, and the
     // largest difference (in units of kT) is kept per chain.
     float drift_max = 0.0f;
-    // Compensated energies (TwoSum per increment) in block groups, where
-    // networks are large and hundreds of terms per hop would otherwise let
-    // the FP32 energies drift by up to 0.02 kT between re-anchors (measured
-    // on N=1000 networks); warp slices run small networks whose drift stays
-    // near 1e-3 kT and keep one add per increment (the compensation cost
-    // 2.5 % of the N=30 ensemble's throughput).
-    constexpr bool kComp = G >= 64;
-    auto eadd = [](float &hi, float &lo, float c) {
-        if (kComp) comp_add(hi, lo, c);
-        else hi += c;
-    };
+    // Energies are compensated (TwoSum per increment): networks are large
+    // here, and hundreds of terms per hop would otherwise let the FP32
+    // energies drift by up to 0.02 kT between re-anchors (measured on N=1000
+    // networks); warp slices run small networks whose drift stays near 1e-3
+    // kT and keep one add per increment.
     // The record of electrode g (thread g < P), the same every hop of the
     // launch: the rebuilds after a hop copy it instead of reading the
     // electrode's energy from global memory again.
@@ -1086,10 +1031,10 @@ __device__ void run_chain(const kmc_batch &B, const Grp &grp, ChainSmem<typename
             // E_j = Ec_j - sum_{k empty} B_jk, summed with compensation
             float hi = Ec[j], lo = 0.0f;
             for (int k = 0; k < N; ++k)
-                if (!((sm.occw[k >> 5] >> (k & 31)) & 1u)) eadd(hi, lo, -pairs.coulomb(j, k));
-            if (drift) drift_max = fmaxf(drift_max, fabsf((hi - sm.E[j]) + (lo - (kComp ? sm.Elo[j] : 0.0f))));
+                if (!((sm.occw[k >> 5] >> (k & 31)) & 1u)) comp_add(hi, lo, -pairs.coulomb(j, k));
+            if (drift) drift_max = fmaxf(drift_max, fabsf((hi - sm.E[j]) + (lo - sm.Elo[j])));
             sm.E[j] = hi;
-            if (kComp) sm.Elo[j] = lo;
+            sm.Elo[j] = lo;
         }
         const int z = N - h;
         int wcur = 0, cum = 0;
@@ -1098,7 +1043,7 @@ __device__ void run_chain(const kmc_batch &B, const Grp &grp, ChainSmem<typename
             while (wcur < w) { cum += __popc(sm.occw[wcur]); ++wcur; }
             const uint32_t word = sm.occw[w];
             const int below = cum + __popc(word & ((1u << (j & 31)) - 1u));
-            const Rec r = pairs.rec(j, cs * (kComp ? sm.E[j] + sm.Elo[j] : sm.E[j]));
+            const Rec r = pairs.rec(j, cs * (sm.E[j] + sm.Elo[j]));
             if ((word >> (j & 31)) & 1u) {
                 sm.src[below] = r;
                 if (!Pairs::kSiteInRec) sm.src_id[below] = j;
@@ -1127,7 +1072,7 @@ __device__ void run_chain(const kmc_batch &B, const Grp &grp, ChainSmem<typename
     float rnd_e1 = 0.0f;
     uint64_t rnd_u = 0;
     int64_t rbase = INT64_MIN / 2;
-    constexpr int RW = G < 32 ? G : 32;   // hops per refill
+    constexpr int RW = 32;   // hops per refill
 
 #ifdef KMC_SECTION_CLOCKS
     uint32_t sec_cycles[kSections] = {};
@@ -1176,15 +1121,14 @@ __device__ void run_chain(const kmc_batch &B, const Grp &grp, ChainSmem<typename
         // least 32 targets and runs of at least 1.5 rows; warp slices are
         // compiled with balanced runs only.
 #ifdef KMC_FORCE_BALANCED_RUNS
-        constexpr bool kAlignedRuns = false;   // measurement builds: the balanced split only
+        const bool aligned = false;   // measurement builds: the balanced split only
 #else
-        constexpr bool kAlignedRuns = G >= 64;
+        const bool aligned = T1 >= 32 && A >= ((3 * G * T1) >> 1);
 #endif
-        const bool aligned = kAlignedRuns && T1 >= 32 && A >= ((3 * G * T1) >> 1);
-        // Balanced run length.  Block groups round it up to an odd number:
-        // thread g's run starts M records after thread g-1's, and with long
-        // rows an odd stride puts the threads' record loads in distinct banks.
-        const int M = ((A + G - 1) / G) | (G >= 64 ? 1 : 0);
+        // Balanced run length, rounded up to an odd number: thread g's run
+        // starts M records after thread g-1's, and with long rows an odd
+        // stride puts the threads' record loads in distinct banks.
+        const int M = ((A + G - 1) / G) | 1;
         int run_b, run_e, r0 = 0, r1 = 0;
         if (aligned) {
             r0 = row_bound(g, G, A, A1, h, P, T1, T2, inv1, inv2);
@@ -1258,47 +1202,8 @@ __device__ void run_chain(const kmc_batch &B, const Grp &grp, ChainSmem<typename
             }
         };
         auto walk_balanced = [&](auto store) {
-            constexpr bool kStore = decltype(store)::value;
-            // The thread walks its run in row-major order, two pairs per step
-            // (two independent load -> rate chains; a row change is a select
-            // plus a predicated reload, not a branch).
-            const int kb = run_b, ke = run_e;
-            int row, col;
-            decode_pair(kb, h, A1, T1, T2, inv1, inv2, row, col);
-            KMC_DCHECK(ke <= A && row >= 0 && row < h + P && col >= 0 && col < (row < h ? T1 : T2));
-            bool sa = row < h;
-            int Tc = sa ? T1 : T2;
-            Rec sr = sm.src[row];
-            int k = kb;
-#pragma unroll kPairUnroll
-            for (; k + 1 < ke; k += 2) {
-                // second pair of the step
-                const bool wa = (col + 1 == Tc);
-                const int colb = wa ? 0 : col + 1;
-                const int rowb = row + (wa ? 1 : 0);
-                Rec srb = sr;
-                if (wa) srb = sm.src[rowb];        // reload only on a row change
-                const bool sab = rowb < h;
-                const int Tcb = sab ? T1 : T2;
-                const float ra = pairs.rate(sr, tgt_load<Pairs>(sm.tgt, col), sa && col < z, cs);
-                const float rb = pairs.rate(srb, tgt_load<Pairs>(sm.tgt, colb), sab && colb < z, cs);
-                lsum += ra;
-                if constexpr (kStore) rp[0] = lsum;
-                lsum += rb;
-                if constexpr (kStore) { rp[RS] = lsum; rp += 2 * RS; }
-                // advance past the second pair
-                const bool wb = (colb + 1 == Tcb);
-                col = wb ? 0 : colb + 1;
-                row = rowb + (wb ? 1 : 0);
-                sr = srb;
-                if (wb) sr = sm.src[row];
-                sa = row < h;
-                Tc = sa ? T1 : T2;
-            }
-            if (k < ke) {
-                lsum += pairs.rate(sr, tgt_load<Pairs>(sm.tgt, col), sa && col < z, cs);
-                if constexpr (kStore) rp[0] = lsum;
-            }
+            PairRange range{h, z, P, T1, T2, A1, A, inv1, inv2};
+            walk_pairs<true, decltype(store)::value, RS, kPairStep>(pairs, sm.src, sm.tgt, range, run_b, run_e, cs, rp, lsum);
         };
         if (aligned) {
             if (rp) walk_aligned(BoolC<true>{});
@@ -1339,17 +1244,15 @@ __device__ void run_chain(const kmc_batch &B, const Grp &grp, ChainSmem<typename
                 rnd_u = u01_fixed(w.y, w.z);
             }
             const int ri = static_cast<int>(hop - rbase);
-            // (in a block group every warp holds the same 32 hops' draws)
-            e1 = grp.lane_value(rnd_e1, ri);
-            u_ev = grp.lane_value(rnd_u, ri);
+            // (every warp holds the same 32 hops' draws)
+            e1 = __shfl_sync(0xffffffffu, rnd_e1, ri);
+            u_ev = __shfl_sync(0xffffffffu, rnd_u, ri);
         }
-        // the stored sums become visible to the whole group (a block group's
-        // select synchronises it)
-        if (G <= 32 && stored) grp.sync();
         KMC_SECTION(2);
         // ---- exact fixed-point scan of the per-thread sums: the event is
         // the first pair whose cumulative rate reaches u*total ----
-        const Selection sel = grp.select(lsum, u_ev, run_e > run_b);
+        // (select synchronises the block: the stored sums are visible then)
+        const Selection sel = grp.select(lsum, u_ev);
         if (!sel.ok) { status = KMC_ERR_NONFINITE; break; }
         const float totf = sel.totf;
         const int L = sel.L;
@@ -1448,7 +1351,7 @@ __device__ void run_chain(const kmc_batch &B, const Grp &grp, ChainSmem<typename
         // ---- clock ----
         const float dt = e1 * rcp_approx(totf);
         const double t_before = t;
-        if (grp.keeps_clock()) t += widen(dt);
+        if (g < 32) t += widen(dt);      // the first warp keeps the clock
         if (B.flux_time) {
             // Expected net hole flow into each electrode in this state,
             // J_e = sum_holes rate(i -> e) - sum_empty rate(e -> j), times
@@ -1475,11 +1378,11 @@ __device__ void run_chain(const kmc_batch &B, const Grp &grp, ChainSmem<typename
             int wcur = 0, cum = 0;
             for (int j = g; j < N; j += G) {
                 // O(N) update (makeJump, simulation.go:107-130), compensated
-                float Ej = sm.E[j], Elo = kComp ? sm.Elo[j] : 0.0f;
-                if (fa && j != from) eadd(Ej, Elo, -pairs.coulomb(j, from));
-                if (tb && j != to) eadd(Ej, Elo, pairs.coulomb(j, to));
+                float Ej = sm.E[j], Elo = sm.Elo[j];
+                if (fa && j != from) comp_add(Ej, Elo, -pairs.coulomb(j, from));
+                if (tb && j != to) comp_add(Ej, Elo, pairs.coulomb(j, to));
                 sm.E[j] = Ej;
-                if (kComp) sm.Elo[j] = Elo;
+                sm.Elo[j] = Elo;
                 const int w = j >> 5;
                 while (wcur < w) { cum += __popc(sm.occw[wcur]); ++wcur; }
                 const uint32_t word = sm.occw[w];
@@ -1493,7 +1396,7 @@ __device__ void run_chain(const kmc_batch &B, const Grp &grp, ChainSmem<typename
                     continue;
                 }
 #endif
-                const Rec r = pairs.rec(j, cs * (kComp ? Ej + Elo : Ej));
+                const Rec r = pairs.rec(j, cs * (Ej + Elo));
                 if (occ_j) {
                     sm.src[below] = r;
                     if (!Pairs::kSiteInRec) sm.src_id[below] = j;
@@ -1544,7 +1447,7 @@ __device__ void run_chain(const kmc_batch &B, const Grp &grp, ChainSmem<typename
 #endif
     // ---- write back ----
     if (record) {
-        const double td = G > 32 ? grp.bcast(t, 0) : t;
+        const double td = grp.bcast(t, 0);
         for (int j = g; j < N; j += G)
             if ((sm.occw[j >> 5] >> (j & 31)) & 1u) {
                 occ_time[j] += td - occ_since[j];
@@ -1580,74 +1483,6 @@ __device__ __forceinline__ const float2 *stage_table(const kmc_batch &B, uint32_
     for (int i = threadIdx.x; i < S * S; i += blockDim.x) dst[i] = __ldg(&src[i]);
     __syncthreads();
     return reinterpret_cast<const float2 *>(smem);
-}
-
-// Stage the one pair table of a launch whose chains all have kT = kT_u as
-// (L, fma(c, B, L)) pairs followed by the B values, c = log2(e)/kT_u.
-__device__ __forceinline__ const float2 *stage_table_uniform(const kmc_batch &B, uint32_t *smem, int table_words)
-{
-    if (table_words <= 0) return nullptr;
-    const int S = B.tab_N[0] + B.tab_P[0];
-    if (S > B.max_sites) return nullptr;   // invalid launch: chains report it
-    const float cu = kLog2e / B.uniform_kT;
-    const float2 *src = reinterpret_cast<const float2 *>(B.tab_LB + B.tab_off[0]);
-    float2 *dst = reinterpret_cast<float2 *>(smem);
-    float *bdst = reinterpret_cast<float *>(dst + S * S);
-    for (int i = threadIdx.x; i < S * S; i += blockDim.x) {
-        const float2 lb = __ldg(&src[i]);
-        dst[i] = make_float2(lb.x, fmaf(cu, lb.y, lb.x));
-        bdst[i] = lb.y;
-    }
-    __syncthreads();
-    return reinterpret_cast<const float2 *>(smem);
-}
-
-// Warp-sliced kernel: 32/G chains per warp, warps_per_block warps.  Two
-// register budgets: MinBlocks = 3 blocks of 256 threads keeps registers at
-// or below 85 so that 24 warps fit on an SM (launches with more blocks than
-// the SMs hold at 2 each); MinBlocks = 2 allows 128 registers (16 warps per
-// SM), which the pair walk uses without spills: 5.6 % faster on 4096 N=30
-// chains, whose 256 blocks all fit.  table_words > 0: every chain of the
-// launch uses table 0, staged in shared memory ahead of the per-chain areas.
-template <int G, typename Pairs, int MinBlocks>
-__global__ void __launch_bounds__(256, MinBlocks) warp_engine_kernel(const kmc_batch B, int rate_words,
-                                                                     int table_words)
-{
-    constexpr int CPW = 32 / G;
-    extern __shared__ __align__(16) uint32_t smem[];
-    const float2 *stab = Pairs::kUniformTable ? stage_table_uniform(B, smem, table_words)
-                                              : stage_table(B, smem, table_words);
-    WarpGroup<G> grp;
-    grp.init();
-    const int warp = threadIdx.x >> 5;
-    using Rec = typename Pairs::Rec;
-    const int words = chain_list_words<Rec>(B.max_sites) + rate_words;
-    ChainSmem<Rec> sm = carve<Rec>(smem + table_words + (warp * CPW + grp.sub) * words, B.max_sites,
-                                   rate_words);
-    if (B.work_counter) {
-        // Persistent launch: each warp claims the next unclaimed item when
-        // the chains of its last one are done, so a warp whose chains end
-        // early takes more work instead of idling until its block ends.
-        // Every lane of the warp takes part in each claim (an item with an
-        // empty slot leaves that group idle until the next claim), and the
-        // loop ends for the whole warp at once, when the list is used up.
-        const int lane = threadIdx.x & 31;
-        for (;;) {
-            int item = 0;
-            if (lane == 0) item = atomicAdd(B.work_counter, 1);
-            item = __shfl_sync(0xffffffffu, item, 0);
-            if (item >= B.n_work) break;
-            const int c = B.work[item * CPW + grp.sub];
-            if (c >= 0 && c < B.n_chains) run_chain<WarpGroup<G>, Pairs>(B, grp, sm, c, stab);
-            __syncwarp();
-        }
-        return;
-    }
-    const int item = blockIdx.x * B.warps_per_block + warp;
-    if (item >= B.n_work) return;
-    const int c = B.work[item * CPW + grp.sub];
-    if (c < 0 || c >= B.n_chains) return;   // the whole group leaves together
-    run_chain<WarpGroup<G>, Pairs>(B, grp, sm, c, stab);
 }
 
 // Block kernel: one chain per block of T threads.  512 / T blocks an SM leave
@@ -1730,82 +1565,6 @@ int table_stage_words(const kmc_batch &b, size_t rest)
     return (w * 4 + rest <= kSmemBudget && w * 4 <= 64 * 1024) ? static_cast<int>(w) : 0;
 }
 
-template <int G, typename Pairs>
-int launch_warp_kernel(const kmc_batch &b, cudaStream_t st, int grid, size_t smem, int rw, int tw)
-{
-    // The register-rich variant when every block of the launch is resident
-    // at once with 16 warps per SM, else the one that fits 24.
-    const int wpb = b.warps_per_block;
-    const int rich_blocks = (16 / wpb) * sm_count();
-    if (b.work_counter) {
-        // persistent: as many blocks as stay resident at once (85-register
-        // variant), no more than the work needs
-        static int configured_p = 0;
-        const int rc = set_smem(warp_engine_kernel<G, Pairs, 3>, smem, configured_p);
-        if (rc != KMC_OK) return rc;
-        int per_sm = 0;
-        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, warp_engine_kernel<G, Pairs, 3>,
-                                                                      wpb * 32, smem);
-        if (e != cudaSuccess) return fail_cuda(e, "engine occupancy");
-        int pgrid = min(grid, max(1, per_sm) * sm_count());
-        if (b.max_grid > 0) pgrid = min(pgrid, b.max_grid);
-        warp_engine_kernel<G, Pairs, 3><<<pgrid, wpb * 32, smem, st>>>(b, rw, tw);
-        e = cudaGetLastError();
-        return e == cudaSuccess ? KMC_OK : fail_cuda(e, "engine launch");
-    }
-    if (grid <= rich_blocks) {
-        static int configured_rich = 0;
-        const int rc = set_smem(warp_engine_kernel<G, Pairs, 2>, smem, configured_rich);
-        if (rc != KMC_OK) return rc;
-        warp_engine_kernel<G, Pairs, 2><<<grid, wpb * 32, smem, st>>>(b, rw, tw);
-    } else {
-        static int configured = 0;
-        const int rc = set_smem(warp_engine_kernel<G, Pairs, 3>, smem, configured);
-        if (rc != KMC_OK) return rc;
-        warp_engine_kernel<G, Pairs, 3><<<grid, wpb * 32, smem, st>>>(b, rw, tw);
-    }
-    cudaError_t e = cudaGetLastError();
-    return e == cudaSuccess ? KMC_OK : fail_cuda(e, "engine launch");
-}
-
-template <int G, typename Pairs>
-int preload_warp_kernels()
-{
-    int rc;
-    if ((rc = touch_kernel(warp_engine_kernel<G, Pairs, 2>)) != KMC_OK) return rc;
-    return touch_kernel(warp_engine_kernel<G, Pairs, 3>);
-}
-template <int G, typename Pairs>
-int launch_warp(const kmc_batch &b, cudaStream_t st)
-{
-    constexpr int CPW = 32 / G;
-    const int wpb = b.warps_per_block;
-    const int lw = chain_list_words<typename Pairs::Rec>(b.max_sites);
-    int rw = rate_buffer_words(b.max_sites, G);
-    // Pad each chain's area to G words modulo 32: the 32/G chains of a warp
-    // then store their running sums (row i of the transposed layout) to
-    // disjoint banks.
-    if (G < 32) rw += ((G - (lw + rw)) % 32 + 32) % 32;
-    if (static_cast<size_t>(wpb) * CPW * (lw + rw) * 4 > kSmemBudget) rw = 0;   // recompute instead
-    const size_t chains = static_cast<size_t>(wpb) * CPW * (lw + rw) * 4;
-    const int tw = table_stage_words<Pairs>(b, chains);
-    const size_t smem = chains + static_cast<size_t>(tw) * 4;
-    if (smem > kSmemBudget)
-        return fail(KMC_ERR_INVALID, "engine: %zu bytes of shared memory per block (max_sites %d, G %d, %d warps) exceeds the budget",
-                    smem, b.max_sites, G, wpb);
-    const int grid = (b.n_work + wpb - 1) / wpb;
-    if (grid <= 0) return KMC_OK;
-    if (tw > 0 && b.uniform_kT > 0.0f) {
-        // every chain has kT = uniform_kT: stage (L, L + c B) and B (3 S^2 words)
-        const int tw3 = ((3 * b.max_sites * b.max_sites) + 3) & ~3;
-        const size_t smem3 = chains + static_cast<size_t>(tw3) * 4;
-        if (smem3 <= kSmemBudget && static_cast<size_t>(tw3) * 4 <= 96 * 1024)
-            return launch_warp_kernel<G, TablePairs<true, true>>(b, st, grid, smem3, rw, tw3);
-    }
-    if (tw > 0) return launch_warp_kernel<G, TablePairs<true>>(b, st, grid, smem, rw, tw);
-    return launch_warp_kernel<G, Pairs>(b, st, grid, smem, rw, tw);
-}
-
 template <int T, typename Pairs>
 int launch_block_kernel(const kmc_batch &b, cudaStream_t st, size_t smem, int rw, int tw)
 {
@@ -1831,26 +1590,32 @@ int preload_block_kernel()
 {
     return touch_kernel(block_engine_kernel<T, Pairs>);
 }
+// Words of the running-sum buffer of a block group's chain, or 0: the event
+// search then re-evaluates the chosen thread's run, for a block group a chunk
+// or two of rates.
+template <int T, typename Pairs>
+int block_rate_words(const kmc_batch &b)
+{
+    const int lw = chain_list_words<typename Pairs::Rec>(b.max_sites);
+    const int rw = rate_buffer_words(b.max_sites, T);
+    if (static_cast<size_t>(lw + rw) * 4 > kSmemBudget) return 0;
+    // Drop the buffer when it is what limits the blocks an SM holds and the
+    // launch has more chains than the SMs then hold at once (a 512-chain
+    // request of N=240 networks at 512 threads: one wave of blocks instead
+    // of two).
+    const int per_sm_threads = 2048 / T;
+    const int per_sm_with = static_cast<int>((227 * 1024) / (static_cast<size_t>(lw + rw) * 4));
+    const int per_sm_without = static_cast<int>((227 * 1024) / (static_cast<size_t>(lw) * 4));
+    if (per_sm_with < per_sm_threads && per_sm_without > per_sm_with && b.n_work > per_sm_with * sm_count())
+        return 0;
+    return rw;
+}
+
 template <int T, typename Pairs>
 int launch_block(const kmc_batch &b, cudaStream_t st)
 {
     const int lw = chain_list_words<typename Pairs::Rec>(b.max_sites);
-    int rw = rate_buffer_words(b.max_sites, T);
-    if (static_cast<size_t>(lw + rw) * 4 > kSmemBudget) rw = 0;
-    if (rw > 0) {
-        // Without the running-sum buffer the event search re-evaluates the
-        // chosen thread's run, for a block group a chunk or two of rates.
-        // Drop the buffer when it is what limits the blocks an SM holds and
-        // the launch has more chains than the SMs then hold at once (a
-        // 512-chain request of N=240 networks at 512 threads: one wave of
-        // blocks instead of two).
-        const int per_sm_threads = 2048 / T;
-        const int per_sm_with = static_cast<int>((227 * 1024) / (static_cast<size_t>(lw + rw) * 4));
-        const int per_sm_without = static_cast<int>((227 * 1024) / (static_cast<size_t>(lw) * 4));
-        if (per_sm_with < per_sm_threads && per_sm_without > per_sm_with &&
-            b.n_work > per_sm_with * sm_count())
-            rw = 0;
-    }
+    const int rw = block_rate_words<T, Pairs>(b);
     const size_t chain = static_cast<size_t>(lw + rw) * 4;
     const int tw = table_stage_words<Pairs>(b, chain);
     const size_t smem = chain + static_cast<size_t>(tw) * 4;

@@ -1,5 +1,5 @@
 // kmc_f32_warp_positions.cu -- warp-slice engine kernels, positions mode
-#include "kmc_f32_engine.cuh"
+#include "kmc_f32_warp.cuh"
 
 namespace kmc {
 

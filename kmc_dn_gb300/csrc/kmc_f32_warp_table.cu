@@ -1,5 +1,5 @@
 // kmc_f32_warp_table.cu -- warp-slice engine kernels, table mode
-#include "kmc_f32_engine.cuh"
+#include "kmc_f32_warp.cuh"
 
 namespace kmc {
 

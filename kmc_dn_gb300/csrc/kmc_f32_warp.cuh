@@ -430,6 +430,10 @@ __device__ void run_warp(const kmc_batch &B, const Slice<G> &sl, ChainSmem<typen
                 }
             }
             KMC_SECTION(4);
+            // (record: when the hole that leaves came, read while the lists are
+            // rebuilt)
+            double since = 0.0;
+            if (record && run && g == 0 && from < N) since = occ_since[from];
             // ---- clock ----
             const float dt = e1 * rcp_approx(totf);
             const double t_before = t;
@@ -506,10 +510,12 @@ __device__ void run_warp(const kmc_batch &B, const Slice<G> &sl, ChainSmem<typen
                     if (tb) sm.occw[to >> 5] |= 1u << (to & 31);
                     else sm.eo[to - N] += 1;
                     if (record) {
-                        traffic[from * S + to] += 1;
-                        if (record == KMC_RECORD_GO) traffic[to * S + from] -= 1;
+                        // fire and forget: this thread alone updates the chain's
+                        // entries, and nothing waits for them
+                        atomicAdd(&traffic[from * S + to], 1);
+                        if (record == KMC_RECORD_GO) atomicAdd(&traffic[to * S + from], -1);
                         const double tx = (record == KMC_RECORD_GO) ? t : t_before;
-                        if (fa) occ_time[from] += tx - occ_since[from];
+                        if (fa) atomicAdd(&occ_time[from], tx - since);
                         if (tb) occ_since[to] = tx;
                     }
                 }

@@ -51,6 +51,7 @@
 #include <cuda_runtime.h>
 
 #include "kmc_common.cuh"
+#include "kmc_exp64.cuh"
 #include "kmc_internal.h"
 
 namespace kmc {
@@ -58,90 +59,12 @@ namespace {
 
 constexpr int kThreads = 128;
 constexpr int kWarps = kThreads / 32;
-// x > 0 for finite and infinite x, false for NaN (as the comparison is), on
-// the integer pipe.
-__device__ __forceinline__ bool positive(double x)
-{
-    return static_cast<unsigned long long>(__double_as_longlong(x)) - 1ull < 0x7ff0000000000000ull;
-}
-
-// x >= y of positive finite values, on the integer pipe.
-__device__ __forceinline__ bool not_less(double x, long long y_bits)
-{
-    return __double_as_longlong(x) >= y_bits;
-}
-
-// exp(x + y) = m * 2^k, 1 <= m <= 2, y a small correction of x, by table and
-// short polynomial (Tang, "Table-driven implementation of the exponential
-// function in IEEE floating-point arithmetic", ACM TOMS 15, 1989):
-// x = (128 k + j) ln2/128 + r, |r| <= ln2/256, m = 2^(j/128) (1 + p(r)), the
-// table entries with their low parts.  |x| < 2^17.  Within 0.51 ulp (largest
-// of 4e6 arguments in (-708, 0]; exp() there 0.87) while |x| < 5000; beyond,
-// the reduction rounds by 2^-53 |x|, as the energies themselves do.
-constexpr int kExpTable = 128;
-__device__ __forceinline__ double exp_split(double x, double y, const double2 *table, int &k)
-{
-    const double shift = 0x1.8p52;
-    const double t = fma(x, 0x1.71547652b82fep+7, shift);        // 128/ln2
-    const int n = __double2loint(t);
-    const double nf = t - shift;
-    // ln2/128 in a 33-bit part, whose products with small n are exact, and the rest
-    double r = fma(nf, -0x1.473de6af278edp-41, fma(nf, -0x1.62e42fefp-8, x));
-    if (__double_as_longlong(y) << 1) r += y;      // not for a zero: an add saved
-    double q = fma(r, 1.0 / 120.0, 1.0 / 24.0);
-    q = fma(fma(q, r, 1.0 / 6.0), r, 0.5);
-    const double p = fma(q, r * r, r);
-    const double2 T = table[n & (kExpTable - 1)];
-    k = n >> 7;
-    return T.x + fma(T.x, p, T.y);
-}
-
-// Entry j of that table, 2^(j/128) as hi + lo: the product of 2^(2^b/128)
-// over the bits of j in double-double arithmetic.
-__device__ double2 exp_table_entry(int j)
-{
-    const double hi[7] = {0x1.0163da9fb3335p+0, 0x1.02c9a3e778061p+0, 0x1.059b0d3158574p+0, 0x1.0b5586cf9890fp+0,
-                          0x1.172b83c7d517bp+0, 0x1.306fe0a31b715p+0, 0x1.6a09e667f3bcdp+0};
-    const double lo[7] = {0x1.b61299ab8cdb7p-54,  -0x1.19083535b085dp-56, 0x1.d73e2a475b465p-55,
-                          0x1.8a62e4adc610bp-54,  -0x1.19041b9d78a76p-55, 0x1.6f46ad23182e4p-55,
-                          -0x1.bdd3413b26456p-54};
-    double x = 1.0, y = 0.0;
-#pragma unroll
-    for (int b = 0; b < 7; ++b) {
-        if ((j >> b) & 1) {
-            const double m = x * hi[b];
-            const double e = fma(x, hi[b], -m) + (x * lo[b] + y * hi[b]);
-            x = m + e;
-            y = e - (x - m);
-        }
-    }
-    return make_double2(x, y);
-}
-
 // A site in a list: exp(+-E/kT) = m 2^k (a source's +, a target's -).
 struct __align__(16) Site {
     double m;
     int id;
     int k;
 };
-
-// |x| at and beyond which the split exponential is not used.
-__device__ __forceinline__ bool splittable(double x)
-{
-    return (__double2hiint(x) & 0x7fffffff) < 0x41000000;
-}
-
-// x / kT as the correctly rounded quotient (reciprocal product and one
-// residual, Markstein) and what it misses; `unit`: kT = 1.
-__device__ __forceinline__ double over_kT(double x, bool unit, double kT, double inv_kT, double &rest)
-{
-    rest = 0.0;
-    if (unit) return x;
-    const double y0 = x * inv_kT;
-    const double y = fma(fma(-y0, kT, x), inv_kT, y0);
-    rest = fma(-y, kT, x) * inv_kT;
-    return y;
-}
 
 // Exact n / T for 0 <= n < 2^22 from inv ~ 1/T: float quotient, one
 // correction step.
@@ -409,21 +332,7 @@ __device__ __forceinline__ void f64_chain(
             for (int a = 0; a < kAhead; ++a) {
                 const int k = k0 + 32 * a + lane;
                 if (k < kwe) {
-                    // min(cap, g 2^ex): a NaN energy difference counts as
-                    // downhill, as the comparison dE > 0 has it
-                    double r = g[a];
-                    if (ex[a] != INT_MIN) {
-                        const int er = __double2hiint(r) >> 20, e = er + ex[a];
-                        if (er == 0 || (er < 2047 && e <= 0))
-                            r = scalbn(r, ex[a]);      // zero, subnormal or about to be
-                        else if (e < 2047 && er < 2047)
-                            r = __hiloint2double(__double2hiint(r) + (ex[a] << 20), __double2loint(r));
-                        else
-                            r = cap[a];
-                        if (static_cast<unsigned long long>(__double_as_longlong(r)) >
-                            static_cast<unsigned long long>(__double_as_longlong(cap[a])))
-                            r = cap[a];
-                    }
+                    const double r = ex[a] == INT_MIN ? g[a] : scaled_min(g[a], ex[a], cap[a]);
                     rates[k] = r;
                 }
             }

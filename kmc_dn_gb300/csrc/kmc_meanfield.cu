@@ -20,8 +20,10 @@
 // site sums its row (outflow) or its column (inflow) in a fixed order, so a
 // run is deterministic and a network's result does not depend on the batch.
 // Two rate precisions:
-//   KMC_MF_RATES_F64  everything in FP64, exp() per pair (the reference's
-//                     arithmetic up to rounding order),
+//   KMC_MF_RATES_F64  everything in FP64 (the reference's arithmetic up to
+//                     rounding order), the exponentials as products of site
+//                     and pair factors (mf_factors; very large networks:
+//                     exp() per pair),
 //   KMC_MF_RATES_F32  FP32 energies and rates (one ex2.approx per pair),
 //                     compensated FP32 row/column sums, FP64 state, step
 //                     and clock: GB300 runs FP64 at 1/64 of FP32, so only
@@ -32,12 +34,14 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "kmc_exp64.cuh"
 #include "kmc_internal.h"
 
 namespace kmc {
 namespace {
 
-constexpr int kMfThreads = 128;
+constexpr int kMfThreads = 128;       // FP32-rate kernel
+constexpr int kMfThreads64 = 256;     // FP64 kernel: two warps a quarter of the SM overlap FP64 and integer work
 constexpr int kMfSmemLimit = 226 * 1024;   // dynamic; leaves room for the static words
 
 __device__ __forceinline__ double warp_sum(double x)
@@ -124,18 +128,53 @@ __device__ __host__ __forceinline__ int row_stride(int S) { return S | 1; }
 
 }  // namespace
 
-size_t mf_smem_bytes(int S, int rates)
+// Largest network of the FP64 path that keeps exponential factors beside the
+// pair constants (36 bytes a pair); larger ones, up to kmc_mf_max_sites,
+// take an exponential per pair (24 bytes).
+constexpr int kMfFactorSites = 77;
+
+static size_t factor_smem_bytes(int S)
+{
+    const size_t pairs = static_cast<size_t>(S) * row_stride(S);
+    return pairs * (16 + 8 + 8 + 4) + 16 * kExpTable + static_cast<size_t>(S) * (14 * 8 + 2 * 4) + 64;
+}
+
+static size_t pair_smem_bytes(int S, int rates)
 {
     const size_t pairs = static_cast<size_t>(S) * row_stride(S);
     const size_t per_pair = rates == KMC_MF_RATES_F64 ? 16 + 8 : 8 + 4;
-    // occ, out, in, avg, eo (double) + e (Real) + occ, e (float) per site, + scalars
+    // occ, out, in, avg, eo (double) + e (Real) + occ, 1 - occ (float) per site, + scalars
     return pairs * per_pair + static_cast<size_t>(S) * (6 * 8 + 2 * 4) + 64;
+}
+
+size_t mf_smem_bytes(int S, int rates)
+{
+    if (rates != KMC_MF_RATES_F64) return pair_smem_bytes(S, rates);
+    const size_t f = factor_smem_bytes(S < kMfFactorSites ? S : kMfFactorSites);
+    const size_t p = S > kMfFactorSites ? pair_smem_bytes(S, rates) : 0;
+    return f > p ? f : p;
 }
 
 namespace {
 
-template <bool F64>
-__global__ void __launch_bounds__(kMfThreads, F64 ? 4 : 8) mf_kernel(kmc_mf_batch b)
+// Steps of a thread's walk over the S x S pairs, T apart: no division per
+// pair.
+template <int T>
+struct PairStep {
+    int i, j, di, dj;
+    __device__ __forceinline__ PairStep(int p, int S) : i(p / S), j(p - (p / S) * S), di(T / S), dj(T - (T / S) * S) {}
+    __device__ __forceinline__ void next(int S)
+    {
+        i += di;
+        j += dj;
+        if (j >= S) { j -= S; ++i; }
+    }
+};
+
+// One network, an exponential per pair: all of the FP32-rate mode, and the
+// FP64 mode of networks beyond kMfFactorSites.
+template <bool F64, int T>
+__device__ void mf_pairs(const kmc_mf_batch &b)
 {
     using Real = typename MfTypes<F64>::Real;
     using Pair = typename MfTypes<F64>::Pair;
@@ -166,20 +205,24 @@ __global__ void __launch_bounds__(kMfThreads, F64 ? 4 : 8) mf_kernel(kmc_mf_batc
     double *avg = ins + S;
     double *eo = avg + S;
     Real *e = reinterpret_cast<Real *>(eo + S);   // site energies (electrodes: voltages)
-    float *of = reinterpret_cast<float *>(e + S);  // FP32 copy of the probabilities
+    float *of = reinterpret_cast<float *>(e + S);  // FP32 copy of the probabilities (1 for electrodes)
+    float *nf = of + S;                            // and of one minus them (1 for electrodes)
     __shared__ double sh_f, sh_ts, sh_time;
     __shared__ int sh_stop;
 
     // pair tables: K = nu*tc, B = I_0 R / d between acceptors (0 otherwise)
-    for (int p = tid; p < SS; p += kMfThreads) {
+    // (and on the diagonal, where the rate is K either way), no rate between
+    // electrodes
+    for (int p = tid; p < SS; p += T) {
         const int i = p / S, j = p - (p / S) * S;
-        const double K = nu * tcon[p];
-        const double B = (i < N && j < N) ? I0R / dist[p] : 0.0;
+        const double K = (i >= N && j >= N) ? 0.0 : nu * tcon[p];
+        const double B = (i < N && j < N && i != j) ? I0R / dist[p] : 0.0;
         KB[i * SP + j] = Pair{static_cast<Real>(K), static_cast<Real>(B)};
     }
-    for (int k = tid; k < S; k += kMfThreads) {
+    for (int k = tid; k < S; k += T) {
         occ[k] = k < N ? occ_io[k] : 0.0;
-        of[k] = static_cast<float>(occ[k]);
+        of[k] = k < N ? static_cast<float>(occ[k]) : 1.0f;
+        nf[k] = k < N ? 1.0f - of[k] : 1.0f;
         e[k] = k < N ? Real(0) : static_cast<Real>(se_out[k]);
         avg[k] = (b.record && k < N) ? b.average_occupation[b.site_off[c] + k] : 0.0;
         eo[k] = 0.0;
@@ -195,53 +238,62 @@ __global__ void __launch_bounds__(kMfThreads, F64 ? 4 : 8) mf_kernel(kmc_mf_batc
     int64_t it = 0;
     for (; it < hops; ++it) {
         // (1) energies from the probabilities, a thread per acceptor
-        for (int i = tid; i < N; i += kMfThreads) {
+        for (int i = tid; i < N; i += T) {
+            // (the diagonal's B is 0)
             Real acc = 0;
+            const Pair *row = KB + i * SP;
+#pragma unroll 4
             for (int j = 0; j < N; ++j) {
-                const Real w = F64 ? static_cast<Real>(1.0 - occ[j]) : static_cast<Real>(1.0f - of[j]);
-                if (j != i) acc += w * KB[i * SP + j].y;
+                if constexpr (F64) acc += (1.0 - occ[j]) * row[j].y;
+                else acc = fmaf(nf[j], row[j].y, acc);
             }
             e[i] = (i == tid ? ec_i : static_cast<Real>(Ec[i])) - acc;
         }
         __syncthreads();
 
         // (2) the S x S expected rates, a thread per pair
-        for (int p = tid; p < SS; p += kMfThreads) {
-            const int i = p / S, j = p - (p / S) * S;
-            const Pair kb = KB[i * SP + j];
-            Real r;
-            if (F64) {
-                double w;
-                if (i >= N && j >= N) w = 0.0;
-                else if (i >= N) w = 1.0 - occ[j];
-                else if (j >= N) w = occ[i];
-                else w = (1.0 - occ[j]) * occ[i];
-                const double dE = static_cast<double>(e[j]) - static_cast<double>(e[i]) - static_cast<double>(kb.y);
-                r = static_cast<Real>(w * static_cast<double>(kb.x) * exp(-fmax(dE, 0.0) * inv_kT));
-            } else {
-                float w;
-                if (i >= N && j >= N) w = 0.0f;
-                else if (i >= N) w = 1.0f - of[j];
-                else if (j >= N) w = of[i];
-                else w = (1.0f - of[j]) * of[i];
-                const float dE = static_cast<float>(e[j]) - static_cast<float>(e[i]) - static_cast<float>(kb.y);
-                r = static_cast<Real>(w * static_cast<float>(kb.x) * ex2_approx(-c2 * fmaxf(dE, 0.0f)));
+        PairStep<T> at(tid, S);
+        if constexpr (F64) {
+            for (int p = tid; p < SS; p += T, at.next(S)) {
+                const int i = at.i, j = at.j;
+                const Pair kb = KB[i * SP + j];
+                const double w = (j < N ? 1.0 - occ[j] : 1.0) * (i < N ? occ[i] : 1.0);
+                const double dE = e[j] - e[i] - kb.y;
+                rt[i * SP + j] = w * kb.x * exp(-fmax(dE, 0.0) * inv_kT);
             }
-            rt[i * SP + j] = r;
+        } else {
+            constexpr int U = 4;      // pairs in flight
+            for (int p = tid; p < SS; p += U * T) {
+                float r[U];
+                int to[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    if (p + u * T < SS) {
+                        const int i = at.i, j = at.j;
+                        to[u] = i * SP + j;
+                        const Pair kb = KB[to[u]];
+                        const float dE = e[j] - e[i] - kb.y;
+                        r[u] = nf[j] * of[i] * kb.x * ex2_approx(-c2 * fmaxf(dE, 0.0f));
+                    }
+                    at.next(S);
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (p + u * T < SS) rt[to[u]] = r[u];
+            }
         }
         __syncthreads();
 
         // (3) outflows (threads 0..S-1, along rows) and inflows (threads
         // S..2S-1, down columns), each a sequential sum in a fixed order
         // (FP32-rate mode: kept as two-float pairs in the same slots)
-        for (int q = tid; q < 2 * S; q += kMfThreads) {
+        for (int q = tid; q < 2 * S; q += T) {
             Acc<F64> a;
             const int k = q < S ? q : q - S;
-            if (q < S) {
-                for (int j = 0; j < S; ++j) a.add(rt[q * SP + j]);
-            } else {
-                for (int i = 0; i < S; ++i) a.add(rt[i * SP + k]);
-            }
+            const Real *v = q < S ? rt + q * SP : rt + k;
+            const int step = q < S ? 1 : SP;
+#pragma unroll 4
+            for (int n = 0; n < S; ++n) a.add(v[n * step]);
             double *dst = q < S ? outs : ins;
             if constexpr (F64) dst[k] = a.value();
             else reinterpret_cast<F2 *>(dst)[k] = a.pair();
@@ -281,23 +333,25 @@ __global__ void __launch_bounds__(kMfThreads, F64 ? 4 : 8) mf_kernel(kmc_mf_batc
             if (sh_stop) break;
             // (5') move the expected charge (the state stays FP64), record, clamp
             const float f = static_cast<float>(sh_f);
-            for (int k = tid; k < S; k += kMfThreads) {
+            for (int k = tid; k < S; k += T) {
                 const double d = static_cast<double>(df_add(ins2[k], F2{-outs2[k].hi, -outs2[k].lo}).hi * f);
                 if (k < N) {
                     if (b.record) avg[k] += occ[k] * sh_ts;
                     const double o = fmin(fmax(occ[k] + d, 0.0), 1.0);
                     occ[k] = o;
                     of[k] = static_cast<float>(o);
+                    nf[k] = 1.0f - of[k];
                 } else {
                     eo[k] += d;
                 }
             }
-            if (traffic)
-                for (int p = tid; p < SS; p += kMfThreads) {
-                    const int i = p / S, j = p - (p / S) * S;
-                    if (i >= N && j >= N) continue;
-                    traffic[p] += static_cast<double>((rt[i * SP + j] - rt[j * SP + i]) * f);
+            if (traffic) {
+                PairStep<T> at(tid, S);
+                for (int p = tid; p < SS; p += T, at.next(S)) {
+                    if (at.i >= N && at.j >= N) continue;
+                    traffic[p] += static_cast<double>((rt[at.i * SP + at.j] - rt[at.j * SP + at.i]) * f);
                 }
+            }
             __syncthreads();
             continue;
         }
@@ -332,29 +386,29 @@ __global__ void __launch_bounds__(kMfThreads, F64 ? 4 : 8) mf_kernel(kmc_mf_batc
         // (5) move the expected charge, record, clamp
         const double f = sh_f;
         const double ts = sh_ts;
-        for (int k = tid; k < S; k += kMfThreads) {
+        for (int k = tid; k < S; k += T) {
             const double net = ins[k] - outs[k];
             if (k < N) {
                 if (b.record) avg[k] += occ[k] * ts;
                 double o = occ[k] + net * f;
                 o = o < 0.0 ? 0.0 : (o > 1.0 ? 1.0 : o);
                 occ[k] = o;
-                of[k] = static_cast<float>(o);
             } else {
                 eo[k] += net * f;
             }
         }
-        if (traffic)
-            for (int p = tid; p < SS; p += kMfThreads) {
-                const int i = p / S, j = p - (p / S) * S;
-                if (i >= N && j >= N) continue;
-                traffic[p] += (static_cast<double>(rt[i * SP + j]) - static_cast<double>(rt[j * SP + i])) * f;
+        if (traffic) {
+            PairStep<T> at(tid, S);
+            for (int p = tid; p < SS; p += T, at.next(S)) {
+                if (at.i >= N && at.j >= N) continue;
+                traffic[p] += (static_cast<double>(rt[at.i * SP + at.j]) - static_cast<double>(rt[at.j * SP + at.i])) * f;
             }
+        }
         __syncthreads();
     }
 
     // outputs
-    for (int k = tid; k < S; k += kMfThreads) {
+    for (int k = tid; k < S; k += T) {
         if (k < N) {
             occ_io[k] = occ[k];
             se_out[k] = static_cast<double>(e[k]);
@@ -368,6 +422,278 @@ __global__ void __launch_bounds__(kMfThreads, F64 ? 4 : 8) mf_kernel(kmc_mf_batc
         if (b.status) b.status[c] = sh_stop ? KMC_ERR_NONFINITE : KMC_OK;
         if (b.iterations_done) b.iterations_done[c] = it;
     }
+}
+
+// One network, FP64, with the exponentials as products (networks of at most
+// kMfFactorSites): exp(-dE/kT) = exp(e_i/kT) exp(-e_j/kT) exp(B_ij/kT), one
+// exponential a site and iteration, the coupling factor tabulated with K.  A
+// pair then costs two multiplications, and its weights are taken out of the
+// sums (out_i = o_i sum_j (1 - o_j) t_ij, in_j = (1 - o_j) sum_i o_i t_ij):
+// four FP64 instructions a pair for the exponential's and the weights' thirty.
+// The FP64 unit's time is the kernel's (64 cycles a warp instruction and SM
+// quarter), so the rest is spread over the block, and compared as
+// integers.  Mantissa and exponent are kept apart
+// (kmc_exp64.cuh); energies beyond its range take the exponential.
+// 64 networks of N = 30, P = 8, 1000 iterations: 5.9 ms (18.9 ms with an
+// exponential per pair).
+__device__ void mf_factors(const kmc_mf_batch &b)
+{
+    constexpr int T = kMfThreads64;
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int c = blockIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int N = b.N[c], P = b.P[c], S = N + P;
+    const int SS = S * S;
+    const int SP = row_stride(S);
+    const double nu = b.nu[c], kT = b.kT[c], I0R = b.I_0[c] * b.R[c];
+    const double *dist = b.distances + b.pair_off[c];
+    const double *tcon = b.transitions_constant + b.pair_off[c];
+    const double *Ec = b.E_constant + b.site_off[c];
+    double *se_out = b.site_energies + b.site_off[c];
+    double *occ_io = b.occupation + b.site_off[c];
+
+    double2 *KW = reinterpret_cast<double2 *>(smem);          // K, mantissa of K exp(B/kT)
+    double2 *exp_tab = KW + S * SP;
+    double *Bt = reinterpret_cast<double *>(exp_tab + kExpTable);   // B
+    double *rt = Bt + S * SP;                                 // t_ij
+    double *occ = rt + S * SP;                                // probabilities (1 for electrodes)
+    double *emp = occ + S;                                    // one minus them (1 for electrodes)
+    double *um = emp + S;                                     // exp(e/kT), mantissas
+    double *vm = um + S;                                      // exp(-e/kT)
+    double *outs = vm + S;
+    double *ins = outs + S;
+    double *net = ins + S;
+    double *avg = net + S;
+    double *eo = avg + S;
+    double *e = eo + S;                                       // site energies (electrodes: voltages)
+    double *part = e + S;                                     // [4 S] parts of the sums
+    int *W_k = reinterpret_cast<int *>(part + 4 * S);         // exponents beside KW
+    int *uk = W_k + S * SP;
+    int *vk = uk + S;
+    __shared__ double sh_f, sh_ts, sh_time;
+    __shared__ int sh_stop, wide_always, wide_now[2];
+
+    const bool unit = kT == 1.0;
+    const double inv_kT = 1.0 / kT;
+    if (tid == 0) {
+        sh_time = 0.0;
+        sh_stop = wide_always = wide_now[0] = wide_now[1] = 0;
+    }
+    for (int j = tid; j < kExpTable; j += T) exp_tab[j] = exp_table_entry(j);
+    __syncthreads();
+    for (int p = tid; p < SS; p += T) {
+        const int i = p / S, j = p - (p / S) * S, q = i * SP + j;
+        const double K = (i >= N && j >= N) ? 0.0 : nu * tcon[p];
+        const double B = (i < N && j < N && i != j) ? I0R / dist[p] : 0.0;
+        double rest, f = 1.0;
+        int k = 0;
+        const double x = over_kT(B, unit, kT, inv_kT, rest);
+        if (splittable(x)) f = exp_split(x, rest, exp_tab, k);
+        else wide_always = 1;
+        Bt[q] = B;
+        KW[q] = make_double2(K, K * f);
+        W_k[q] = k;
+    }
+    for (int k = tid; k < S; k += T) {
+        occ[k] = k < N ? occ_io[k] : 1.0;
+        emp[k] = k < N ? 1.0 - occ[k] : 1.0;
+        e[k] = k < N ? 0.0 : se_out[k];
+        avg[k] = (b.record && k < N) ? b.average_occupation[b.site_off[c] + k] : 0.0;
+        eo[k] = 0.0;
+        um[k] = vm[k] = 1.0;
+        uk[k] = vk[k] = 0;
+        if (k >= N) {
+            double rest;
+            const double x = over_kT(e[k], unit, kT, inv_kT, rest);
+            if (splittable(x)) {
+                um[k] = exp_split(x, rest, exp_tab, uk[k]);
+                vm[k] = exp_split(-x, -rest, exp_tab, vk[k]);
+            } else {
+                wide_always = 1;
+            }
+        }
+    }
+    __syncthreads();
+
+    const int64_t hops = b.hops[c];
+    double *traffic = b.record ? b.traffic + b.traffic_off[c] : nullptr;
+    const double Ec0 = (tid >> 2) < N ? Ec[tid >> 2] : 0.0;
+    const int p0 = tid / (2 * S), q0 = tid - p0 * 2 * S;
+    int64_t it = 0;
+    for (; it < hops; ++it) {
+        // (1) energies from the probabilities and their exponentials: four
+        // threads an acceptor, two of which take one exponential each
+        for (int q = tid; q < 4 * ((N + 7) & ~7); q += T) {
+            const int i = q >> 2;
+            double acc = 0.0;
+            if (i < N) {
+                const double *row = Bt + i * SP;      // (the diagonal's B is 0)
+#pragma unroll 4
+                for (int j = q & 3; j < N; j += 4) acc = fma(emp[j], row[j], acc);
+            }
+            acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+            acc += __shfl_xor_sync(0xffffffffu, acc, 2);
+            if (i < N && (q & 3) < 2) {
+                const double ei = (q == tid ? Ec0 : Ec[i]) - acc;
+                const bool leave = (q & 3) == 0;
+                double rest;
+                double x = over_kT(ei, unit, kT, inv_kT, rest);
+                if (!leave) {
+                    x = -x;
+                    rest = -rest;
+                }
+                if (leave) e[i] = ei;
+                if (splittable(x)) (leave ? um : vm)[i] = exp_split(x, rest, exp_tab, (leave ? uk : vk)[i]);
+                else wide_now[it & 1] = 1;
+            }
+        }
+        __syncthreads();
+        const bool wide = wide_always | wide_now[it & 1];
+        if (tid == 0) wide_now[(it + 1) & 1] = 0;
+
+        // (2) t_ij = K min(1, exp(-dE/kT)), a thread per pair
+        PairStep<T> at(tid, S);
+        constexpr int U = 4;      // pairs in flight
+        for (int p = tid; p < SS; p += U * T) {
+            double t[U];
+            int to[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if (p + u * T < SS) {
+                    const int i = at.i, j = at.j;
+                    to[u] = i * SP + j;
+                    const double2 kw = KW[to[u]];
+                    if (!wide) {
+                        t[u] = scaled_min(kw.y * (um[i] * vm[j]), W_k[to[u]] + uk[i] + vk[j], kw.x);
+                    } else {
+                        const double dE = e[j] - e[i] - Bt[to[u]];
+                        t[u] = kw.x * exp(-fmax(dE, 0.0) * inv_kT);
+                    }
+                }
+                at.next(S);
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (p + u * T < SS) rt[to[u]] = t[u];
+        }
+        __syncthreads();
+
+        // (3) outflows along rows (items 0..S-1) and inflows down columns
+        // (S..2S-1), each in three parts
+        const int third = (S + 2) / 3;
+        for (int q = tid, item = q0, pt = p0; q < 6 * S; q += T) {
+            const int k = item < S ? item : item - S;
+            const double *v = item < S ? rt + k * SP : rt + k;
+            const double *w = item < S ? emp : occ;
+            const int step = item < S ? 1 : SP;
+            const int n1 = min(S, (pt + 1) * third);
+            double s = 0.0;
+#pragma unroll 4
+            for (int n = pt * third; n < n1; ++n) s = fma(w[n], v[n * step], s);
+            if (pt == 0) (item < S ? outs : ins)[k] = s;
+            else part[(pt - 1) * 2 * S + item] = s;
+            item += T;
+            while (item >= 2 * S) { item -= 2 * S; ++pt; }
+        }
+        __syncthreads();
+        for (int k = tid; k < S; k += T) {
+            const double o = occ[k] * (outs[k] + part[k] + part[2 * S + k]);
+            const double in = emp[k] * (ins[k] + part[S + k] + part[3 * S + k]);
+            outs[k] = o;
+            net[k] = in - o;
+        }
+        __syncthreads();
+
+        // (4) total and step size (one warp; one FP64 division per iteration)
+        if (warp == 0) {
+            double tot = lane < S ? outs[lane] : 0.0;
+            for (int k = lane + 32; k < S; k += 32) tot += outs[k];
+            tot = warp_sum(tot);
+            const double inv = __drcp_rn(tot);
+            double mc = 1.0;
+            bool less = false;
+            for (int k = lane; k < N; k += 32) {
+                const double nv = fma(net[k], inv, occ[k]);
+                // below 0 or above 1, by its bits (values above 1 have larger
+                // bit patterns; NaN compares as neither)
+                const long long bits = __double_as_longlong(nv);
+                if (bits < 0 || bits > __double_as_longlong(1.0)) {
+                    const double q = net[k] * inv;
+                    if (nv < 0) mc = fmin(mc, occ[k] / -q);
+                    if (nv > 1) mc = fmin(mc, (1.0 - occ[k]) / q);
+                    less = true;
+                }
+            }
+            if (__any_sync(0xffffffffu, less)) mc = warp_min(mc);
+            if (lane == 0) {
+                if (!positive(tot) || __double_as_longlong(tot) >= __double_as_longlong(1.0e300)) {
+                    sh_stop = 1;
+                } else {
+                    sh_f = mc * inv;              // fraction of each expected flow moved
+                    sh_ts = 0.98 * mc * inv;      // time step
+                    sh_time += sh_ts;
+                }
+            }
+        }
+        __syncthreads();
+        if (sh_stop) break;
+
+        // (5) record, move the expected charge, clamp
+        const double f = sh_f;
+        if (traffic) {
+            PairStep<T> tr(tid, S);
+            for (int p = tid; p < SS; p += T, tr.next(S)) {
+                const int i = tr.i, j = tr.j;
+                if (i >= N && j >= N) continue;
+                traffic[p] += (occ[i] * emp[j] * rt[i * SP + j] - occ[j] * emp[i] * rt[j * SP + i]) * f;
+            }
+            __syncthreads();
+        }
+        for (int k = tid; k < S; k += T) {
+            if (k < N) {
+                if (b.record) avg[k] += occ[k] * sh_ts;
+                double o = fma(net[k], f, occ[k]);
+                const long long bits = __double_as_longlong(o);
+                if (bits < 0 || bits > __double_as_longlong(1.0)) o = o < 0.0 ? 0.0 : (o > 1.0 ? 1.0 : o);
+                occ[k] = o;
+                emp[k] = 1.0 - o;
+            } else {
+                eo[k] += net[k] * f;
+            }
+        }
+        __syncthreads();
+    }
+
+    // outputs
+    for (int k = tid; k < S; k += T) {
+        if (k < N) {
+            occ_io[k] = occ[k];
+            se_out[k] = e[k];
+            if (b.record) b.average_occupation[b.site_off[c] + k] = avg[k];
+        } else {
+            b.electrode_occupation[b.el_off[c] + (k - N)] = eo[k];
+        }
+    }
+    if (tid == 0) {
+        b.time[c] = sh_time;
+        if (b.status) b.status[c] = sh_stop ? KMC_ERR_NONFINITE : KMC_OK;
+        if (b.iterations_done) b.iterations_done[c] = it;
+    }
+}
+
+// One block per network.
+__global__ void __launch_bounds__(kMfThreads, 8) mf_kernel_f32(kmc_mf_batch b)
+{
+    mf_pairs<false, kMfThreads>(b);
+}
+
+// The path is chosen by each network's own size, so that its result does not
+// depend on the batch.
+__global__ void __launch_bounds__(kMfThreads64, 2) mf_kernel_f64(kmc_mf_batch b)
+{
+    const int S = b.N[blockIdx.x] + b.P[blockIdx.x];
+    if (S >= 1 && S <= kMfFactorSites && S <= b.max_sites) mf_factors(b);
+    else mf_pairs<true, kMfThreads64>(b);
 }
 
 }  // namespace
@@ -409,13 +735,13 @@ extern "C" int kmc_mf_run(const kmc_mf_batch *b, void *stream)
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     cudaError_t e;
     if (b->rates == KMC_MF_RATES_F64) {
-        e = cudaFuncSetAttribute(mf_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        e = cudaFuncSetAttribute(mf_kernel_f64, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
         if (e != cudaSuccess) return fail_cuda(e, "mf_run smem attribute");
-        mf_kernel<true><<<b->n_chains, kMfThreads, smem, st>>>(*b);
+        mf_kernel_f64<<<b->n_chains, kMfThreads64, smem, st>>>(*b);
     } else {
-        e = cudaFuncSetAttribute(mf_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        e = cudaFuncSetAttribute(mf_kernel_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
         if (e != cudaSuccess) return fail_cuda(e, "mf_run smem attribute");
-        mf_kernel<false><<<b->n_chains, kMfThreads, smem, st>>>(*b);
+        mf_kernel_f32<<<b->n_chains, kMfThreads, smem, st>>>(*b);
     }
     e = cudaGetLastError();
     return e == cudaSuccess ? KMC_OK : fail_cuda(e, "mf_run launch");
@@ -533,8 +859,8 @@ namespace kmc {
 int preload_meanfield()
 {
     int rc;
-    if ((rc = touch_kernel(mf_kernel<true>)) != KMC_OK) return rc;
-    return touch_kernel(mf_kernel<false>);
+    if ((rc = touch_kernel(mf_kernel_f64)) != KMC_OK) return rc;
+    return touch_kernel(mf_kernel_f32);
 }
 
 }  // namespace kmc

@@ -526,6 +526,17 @@ size_t kmc_laplace_workspace_size(int32_t nx, int32_t ny, int32_t n_fields);
 int kmc_laplace_basis(int32_t nx, int32_t ny, double hx, double hy, int32_t n_fields,
                       double *grid, void *workspace, size_t workspace_bytes, void *stream);
 
+/*
+ * Boundary data of a layout's basis fields on the device: grid (n_electrodes
+ * + 1 nodal grids of (ny+1) x (nx+1)) gets 1 on electrode e's boundary nodes
+ * in field e and on the rest of the boundary in the last one, 0 elsewhere.
+ * An electrode is the segment within `surplus` of its position along its
+ * edge; the first that matches a node has it (the boundary expression of
+ * kmc_dopant_networks.py:733-763).  xy: device, 2 doubles per electrode.
+ */
+int kmc_laplace_boundary(int32_t nx, int32_t ny, double xdim, double ydim, double surplus,
+                         int32_t n_electrodes, const double *xy, double *grid, void *stream);
+
 /* P1 interpolation of n_fields nodal grids at n_points (x, y) points
  * (device xy[2*n_points]); out[f*n_points + p].  The point evaluation of the
  * FEniCS function V(x, y) (kmc_dopant_networks.py:851-853). */

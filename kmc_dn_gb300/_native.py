@@ -131,6 +131,7 @@ _SIGS = {
     "kmc_mf_run_host": (C.c_int, [C.POINTER(KmcMfBatch), _vp]),
     "kmc_laplace_workspace_size": (_sz, [_i32, _i32, _i32]),
     "kmc_laplace_basis": (C.c_int, [_i32, _i32, _f64, _f64, _i32, _vp, _vp, _sz, _vp]),
+    "kmc_laplace_boundary": (C.c_int, [_i32, _i32, _f64, _f64, _f64, _i32, _vp, _vp, _vp]),
     "kmc_p1_sample": (C.c_int, [_i32, _i32, _f64, _f64, _i32, _vp, _i32, _vp, _vp, _vp]),
 }
 EXPORTED = tuple(_SIGS)

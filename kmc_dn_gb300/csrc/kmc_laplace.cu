@@ -11,11 +11,21 @@
 //     T_n = Q_n diag(lambda) Q_n,  Q_n[a][b] = sqrt(2/n) sin(pi (a+1)(b+1)/n),
 //     lambda_b = 2 - 2 cos(pi (b+1)/n)   (n = cells, size n-1).
 // So U = Q_y ((Q_y F Q_x) ./ (cx lambda_x + cy lambda_y)) Q_x, F the
-// right-hand side carrying the boundary data: four small FP64 matrix
-// products per field, exact up to rounding (no iteration, no tolerance).
-// All fields of one mesh are solved in one batch; P1 sampling at the
-// acceptors follows.  This replaces the per-geometry CPU solve when
-// geometries churn (serving).
+// right-hand side carrying the boundary data: exact up to rounding (no
+// iteration, no tolerance).  All fields of one mesh are solved in one batch;
+// P1 sampling at the acceptors follows.  This replaces the per-geometry CPU
+// solve when geometries churn (serving).
+//
+// F is zero but for the nodes beside the boundary, so its transform is four
+// matrix-vector products a field (the sides' data) and four outer products.
+// The inverse transform is the work: two products with Q a field, FP64, whose
+// unit takes 64 cycles a warp instruction and SM quarter, spread over one
+// wave of blocks.  Q itself is never stored: its entries are the 2n values
+// sin(pi q/n), q = (k+1)(j+1) mod 2n, in shared memory.  (Half the products
+// could be had from Q's mirror symmetry Q[k][m-1-j] = (-1)^k Q[k][j]; that
+// moved the result by 7e-15, where this is within 1e-15 of the plain products.)
+// Four launches; 9 fields of 99 x 99 cells: 84 us (134 us in nine launches
+// with Q and dense products in 16 x 16 tiles).
 #include <cmath>
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -25,96 +35,168 @@
 namespace kmc {
 namespace {
 
-constexpr int kTile = 16;
+constexpr int kSides = 4;              // left, right (along y), bottom, top (along x)
+constexpr int kThreads = 128;
+constexpr int kRows = 6;               // rows of a field per block of a product: 147 blocks for 9 fields of 98 rows
 
-// Q[a][b] = sqrt(2/n) sin(pi (a+1)(b+1)/n), (n-1) x (n-1); lam[b].
-__global__ void dst_basis_kernel(int n, double *Q, double *lam)
+// Per direction: sqrt(2/n) sin(pi q/n), q = 0 .. 2n-1, and the eigenvalues
+// 2 - 2 cos(pi (k+1)/n).
+struct Tables {
+    double *sx, *sy, *lx, *ly;
+};
+
+__global__ void table_kernel(int nx, int ny, Tables t)
 {
-    const int m = n - 1;
     const double pi = 3.14159265358979323846;
-    const double s = sqrt(2.0 / n);
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < m * m; k += gridDim.x * blockDim.x) {
-        const int a = k / m, b = k - (k / m) * m;
-        // (a+1)(b+1) mod 2n keeps the sine argument small and exact
-        const long long p = (static_cast<long long>(a + 1) * (b + 1)) % (2LL * n);
-        Q[k] = s * sin(pi * static_cast<double>(p) / n);
-        if (a == 0) lam[b] = 2.0 - 2.0 * cos(pi * (b + 1) / n);
+    const int total = 2 * nx + 2 * ny + (nx - 1) + (ny - 1);
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < total; k += gridDim.x * blockDim.x) {
+        int q = k;
+        if (q < 2 * nx) { t.sx[q] = sqrt(2.0 / nx) * sin(pi * static_cast<double>(q) / nx); continue; }
+        q -= 2 * nx;
+        if (q < 2 * ny) { t.sy[q] = sqrt(2.0 / ny) * sin(pi * static_cast<double>(q) / ny); continue; }
+        q -= 2 * ny;
+        if (q < nx - 1) { t.lx[q] = 2.0 - 2.0 * cos(pi * (q + 1) / nx); continue; }
+        q -= nx - 1;
+        t.ly[q] = 2.0 - 2.0 * cos(pi * (q + 1) / ny);
     }
 }
 
-// Right-hand side of the interior system from the boundary values of each
-// field's nodal grid ((ny+1) x (nx+1), row = y index).
-__global__ void rhs_kernel(int nx, int ny, double cx, double cy, int nf, const double *grid, double *F)
+// The table of n cells in shared memory, or (no room: very fine meshes) where
+// it is.
+__device__ __forceinline__ const double *staged(const double *tab, int n, double *sh)
 {
-    const int mi = ny - 1, mj = nx - 1;
-    const long long per = static_cast<long long>(mi) * mj;
-    for (long long k = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; k < per * nf;
-         k += static_cast<long long>(gridDim.x) * blockDim.x) {
-        const int f = static_cast<int>(k / per);
-        const long long r = k - f * per;
-        const int i = static_cast<int>(r / mj) + 1, j = static_cast<int>(r % mj) + 1;   // node indices
-        const double *g = grid + static_cast<long long>(f) * (ny + 1) * (nx + 1);
-        double b = 0.0;
-        if (j == 1) b += cx * g[i * (nx + 1) + 0];
-        if (j == nx - 1) b += cx * g[i * (nx + 1) + nx];
-        if (i == 1) b += cy * g[0 * (nx + 1) + j];
-        if (i == ny - 1) b += cy * g[ny * (nx + 1) + j];
-        F[k] = b;
-    }
+    if (!sh) return tab;
+    for (int q = threadIdx.x; q < 2 * n; q += blockDim.x) sh[q] = tab[q];
+    return sh;
 }
 
-// C_f = op(A) * B_f or B_f * op(A) for every field f (blockIdx.z), FP64,
-// shared-memory tiles.  left: C = A (m x m) * X (m x n); else C = X (m x n) * A (n x n).
-__global__ void gemm_kernel(int m, int n, const double *A, const double *X, double *C, int left)
+// (a * b) mod m for a, b < m
+__device__ __forceinline__ int mulmod(int a, int b, int m)
 {
-    __shared__ double ta[kTile][kTile + 1];
-    __shared__ double tb[kTile][kTile + 1];
-    const long long off = static_cast<long long>(blockIdx.z) * m * n;
-    const double *Xf = X + off;
-    double *Cf = C + off;
-    const int row = blockIdx.y * kTile + threadIdx.y;
-    const int col = blockIdx.x * kTile + threadIdx.x;
-    const int K = left ? m : n;
-    double acc = 0.0;
-    for (int k0 = 0; k0 < K; k0 += kTile) {
-        const int ka = k0 + threadIdx.x, kb = k0 + threadIdx.y;
-        if (left) {
-            ta[threadIdx.y][threadIdx.x] = (row < m && ka < K) ? A[row * m + ka] : 0.0;
-            tb[threadIdx.y][threadIdx.x] = (kb < K && col < n) ? Xf[kb * n + col] : 0.0;
-        } else {
-            ta[threadIdx.y][threadIdx.x] = (row < m && ka < K) ? Xf[row * n + ka] : 0.0;
-            tb[threadIdx.y][threadIdx.x] = (kb < K && col < n) ? A[kb * n + col] : 0.0;
+    return static_cast<int>((static_cast<long long>(a) * b) % m);
+}
+
+// The transforms of the boundary data beside each side: G[f][side][l] =
+// sum_i Q[l][i] g_i, a warp a value.
+__global__ void __launch_bounds__(kThreads) side_kernel(int nx, int ny, int nf, Tables t, const double *grid,
+                                                        double *G, int in_smem)
+{
+    extern __shared__ double sh[];
+    const int f = blockIdx.z, side = blockIdx.y;
+    const int n = side < 2 ? ny : nx, m = n - 1, stride = max(nx, ny) - 1;
+    const double *g = grid + static_cast<long long>(f) * (ny + 1) * (nx + 1);
+    const double *tab = staged(side < 2 ? t.sy : t.sx, n, in_smem ? sh : nullptr);
+    // the side's interior nodes: data[i * step]
+    const long long step = side < 2 ? nx + 1 : 1;
+    const double *data = side == 0 ? g + nx + 1 : side == 1 ? g + nx + 1 + nx : side == 2 ? g + 1
+                                                          : g + static_cast<long long>(ny) * (nx + 1) + 1;
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    for (int l = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5); l < m; l += gridDim.x * (kThreads / 32)) {
+        double acc = 0.0;
+        int q = mulmod(l + 1, lane + 1, 2 * n);
+        const int dq = mulmod(l + 1, 32, 2 * n);
+        for (int i = lane; i < m; i += 32) {
+            acc = fma(tab[q], data[i * step], acc);
+            q += dq;
+            if (q >= 2 * n) q -= 2 * n;
         }
-        __syncthreads();
 #pragma unroll
-        for (int k = 0; k < kTile; ++k) acc = fma(ta[threadIdx.y][k], tb[k][threadIdx.x], acc);
+        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        if (lane == 0) G[(static_cast<long long>(f) * kSides + side) * stride + l] = acc;
+    }
+}
+
+// kRows rows of in (a row of m values each) times Q of n = m + 1 cells: a
+// thread a value.
+template <typename Store>
+__device__ __forceinline__ void rows_times_q(const double *in, int rows, int m, const double *tab, Store store)
+{
+    const int n2 = 2 * (m + 1);
+    for (int it = threadIdx.x; it < rows * m; it += blockDim.x) {
+        const int r = it / m, j = it - (it / m) * m;
+        const double *v = in + r * m;
+        double acc = 0.0;
+        int q = j + 1;                      // (k+1)(j+1) mod 2n
+#pragma unroll 4
+        for (int k = 0; k < m; ++k) {
+            acc = fma(v[k], tab[q], acc);
+            q += j + 1;
+            if (q >= n2) q -= n2;
+        }
+        store(r, j, acc);
+    }
+}
+
+// Y = W Qx, W[l][k] the transformed right-hand side over the eigenvalues.
+__global__ void __launch_bounds__(kThreads) x_kernel(int nx, int ny, double cx, double cy, Tables t, const double *G,
+                                                     double *Y, double *W, int in_smem)
+{
+    extern __shared__ double sh[];
+    const int f = blockIdx.y, mj = nx - 1, mi = ny - 1, stride = max(nx, ny) - 1;
+    const int l0 = blockIdx.x * kRows, rows = min(kRows, mi - l0);
+    const long long at = static_cast<long long>(f) * mi * mj;
+    double *w = in_smem ? sh + 2 * nx : W + at + static_cast<long long>(l0) * mj;
+    const double *tab = staged(t.sx, nx, in_smem ? sh : nullptr);
+    const double *g = G + static_cast<long long>(f) * kSides * stride;
+    for (int it = threadIdx.x; it < rows * mj; it += blockDim.x) {
+        const int r = it / mj, k = it - (it / mj) * mj, l = l0 + r;
+        // Qx[0][k], Qx[mj-1][k], Qy[l][0], Qy[l][mi-1]
+        const double x0 = t.sx[k + 1], x1 = t.sx[mulmod(mj, k + 1, 2 * nx)];
+        const double y0 = t.sy[l + 1], y1 = t.sy[mulmod(mi, l + 1, 2 * ny)];
+        const double num = cx * (g[l] * x0 + g[stride + l] * x1) + cy * (g[2 * stride + k] * y0 + g[3 * stride + k] * y1);
+        w[it] = num / (cx * t.lx[k] + cy * t.ly[l]);
+    }
+    __syncthreads();
+    // transposed (j, l): the next product reads its rows
+    double *out = Y + at;
+    rows_times_q(w, rows, mj, tab, [&](int r, int j, double v) { out[static_cast<long long>(j) * mi + l0 + r] = v; });
+}
+
+// U = Qy Y into the interior of the nodal grids: columns of U are rows of the
+// transposed Y times Qy (symmetric).
+__global__ void __launch_bounds__(kThreads) y_kernel(int nx, int ny, Tables t, const double *Y, double *grid,
+                                                     int in_smem)
+{
+    extern __shared__ double sh[];
+    const int f = blockIdx.y, mj = nx - 1, mi = ny - 1;
+    const int j0 = blockIdx.x * kRows, rows = min(kRows, mj - j0);
+    const double *tab = staged(t.sy, ny, in_smem ? sh : nullptr);
+    const double *w = Y + static_cast<long long>(f) * mi * mj + static_cast<long long>(j0) * mi;
+    if (in_smem) {
+        double *copy = sh + 2 * ny;
+        for (int it = threadIdx.x; it < rows * mi; it += blockDim.x) copy[it] = w[it];
+        w = copy;
         __syncthreads();
     }
-    if (row < m && col < n) Cf[row * n + col] = acc;
+    double *g = grid + static_cast<long long>(f) * (ny + 1) * (nx + 1);
+    rows_times_q(w, rows, mi, tab,
+                 [&](int r, int i, double v) { g[static_cast<long long>(i + 1) * (nx + 1) + j0 + r + 1] = v; });
 }
 
-__global__ void scale_kernel(int mi, int mj, double cx, double cy, const double *lamx, const double *lamy,
-                             int nf, double *W)
+// Boundary data of every basis field: field e < P is 1 on electrode e's
+// nodes, field P on the rest of the boundary.  The node coordinates and
+// comparisons are the host's (boundary_owner in laplace.py), operation for
+// operation; interior nodes are set to 0.
+__global__ void boundary_kernel(int nx, int ny, double hx, double hy, double xdim, double surplus, int P,
+                                const double *xy, double *grid)
 {
-    const long long per = static_cast<long long>(mi) * mj;
-    for (long long k = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; k < per * nf;
-         k += static_cast<long long>(gridDim.x) * blockDim.x) {
-        const long long r = k % per;
-        const int l = static_cast<int>(r / mj), kk = static_cast<int>(r % mj);
-        W[k] /= (cx * lamx[kk] + cy * lamy[l]);
-    }
-}
-
-__global__ void scatter_kernel(int nx, int ny, int nf, const double *U, double *grid)
-{
-    const int mi = ny - 1, mj = nx - 1;
-    const long long per = static_cast<long long>(mi) * mj;
-    for (long long k = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; k < per * nf;
-         k += static_cast<long long>(gridDim.x) * blockDim.x) {
-        const int f = static_cast<int>(k / per);
-        const long long r = k - f * per;
-        const int i = static_cast<int>(r / mj) + 1, j = static_cast<int>(r % mj) + 1;
-        grid[static_cast<long long>(f) * (ny + 1) * (nx + 1) + i * (nx + 1) + j] = U[k];
+    const int nodes = (nx + 1) * (ny + 1);
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nodes; k += gridDim.x * blockDim.x) {
+        const int i = k / (nx + 1), j = k - i * (nx + 1);
+        const bool edge = i == 0 || j == 0 || i == ny || j == nx;
+        int owner = P;
+        if (edge) {
+            const double x = __dmul_rn(static_cast<double>(j), hx), y = __dmul_rn(static_cast<double>(i), hy);
+            for (int e = 0; e < P; ++e) {
+                const double ex = xy[2 * e], ey = xy[2 * e + 1];
+                const bool mine = (ex == 0 || ex == xdim)
+                                      ? (x == ex && y >= __dsub_rn(ey, surplus) && y <= __dadd_rn(ey, surplus))
+                                      : (x >= __dsub_rn(ex, surplus) && x <= __dadd_rn(ex, surplus) && y == ey);
+                if (mine) { owner = e; break; }      // the first match wins
+            }
+        }
+        for (int f = 0; f <= P; ++f) grid[static_cast<long long>(f) * nodes + k] = edge && owner == f ? 1.0 : 0.0;
     }
 }
 
@@ -138,10 +220,35 @@ __global__ void p1_sample_kernel(int nx, int ny, double hx, double hy, int nf, c
     }
 }
 
+template <typename K>
+int allow_smem(K *kernel, size_t smem)
+{
+    if (smem <= 48 * 1024) return KMC_OK;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               static_cast<int>(smem));
+    return e == cudaSuccess ? KMC_OK : fail_cuda(e, "laplace_basis: shared memory");
+}
+
 int grid_for(long long n)
 {
     const long long b = (n + 255) / 256;
     return static_cast<int>(b < 1 ? 1 : (b > 4096 ? 4096 : b));
+}
+
+// Doubles of workspace: Y, the sides' transforms, the transformed right-hand
+// side where a block's rows do not fit its shared memory (0: they do), tables.
+struct LaplaceSpace {
+    size_t fields, sides, copy, tables;
+};
+LaplaceSpace laplace_space(int nx, int ny, int nf)
+{
+    const size_t mi = ny - 1, mj = nx - 1, longest = nx > ny ? nx : ny;
+    LaplaceSpace s;
+    s.fields = mi * mj * nf;
+    s.sides = kSides * (longest - 1) * nf;
+    s.copy = sizeof(double) * (kRows + 2) * longest > 200 * 1024 ? s.fields : 0;
+    s.tables = 2 * (static_cast<size_t>(nx) + ny) + mi + mj;
+    return s;
 }
 
 }  // namespace
@@ -152,8 +259,8 @@ using namespace kmc;
 extern "C" size_t kmc_laplace_workspace_size(int32_t nx, int32_t ny, int32_t n_fields)
 {
     if (nx < 2 || ny < 2 || n_fields < 1) return 0;
-    const size_t mi = ny - 1, mj = nx - 1;
-    return sizeof(double) * (mi * mi + mj * mj + mi + mj + 2 * mi * mj * static_cast<size_t>(n_fields));
+    const LaplaceSpace s = laplace_space(nx, ny, n_fields);
+    return sizeof(double) * (s.fields + s.sides + s.copy + s.tables);
 }
 
 extern "C" int kmc_laplace_basis(int32_t nx, int32_t ny, double hx, double hy, int32_t n_fields,
@@ -166,26 +273,39 @@ extern "C" int kmc_laplace_basis(int32_t nx, int32_t ny, double hx, double hy, i
         return fail(KMC_ERR_INVALID, "laplace_basis: workspace too small");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int mi = ny - 1, mj = nx - 1;
-    double *Qy = static_cast<double *>(workspace);
-    double *Qx = Qy + static_cast<size_t>(mi) * mi;
-    double *ly = Qx + static_cast<size_t>(mj) * mj;
-    double *lx = ly + mi;
-    double *W1 = lx + mj;
-    double *W2 = W1 + static_cast<size_t>(mi) * mj * n_fields;
+    const LaplaceSpace sp = laplace_space(nx, ny, n_fields);
+    double *ws = static_cast<double *>(workspace);
+    double *Y = ws, *G = Y + sp.fields, *W = G + sp.sides, *tab = W + sp.copy;
+    const Tables t{tab, tab + 2 * nx, tab + 2 * nx + 2 * ny, tab + 2 * nx + 2 * ny + mj};
     const double cx = hy / hx, cy = hx / hy;
-    dst_basis_kernel<<<grid_for(static_cast<long long>(mi) * mi), 256, 0, st>>>(ny, Qy, ly);
-    dst_basis_kernel<<<grid_for(static_cast<long long>(mj) * mj), 256, 0, st>>>(nx, Qx, lx);
-    const long long tot = static_cast<long long>(mi) * mj * n_fields;
-    rhs_kernel<<<grid_for(tot), 256, 0, st>>>(nx, ny, cx, cy, n_fields, grid, W1);
-    const dim3 blk(kTile, kTile), grd((mj + kTile - 1) / kTile, (mi + kTile - 1) / kTile, n_fields);
-    gemm_kernel<<<grd, blk, 0, st>>>(mi, mj, Qy, W1, W2, 1);      // Qy F
-    gemm_kernel<<<grd, blk, 0, st>>>(mi, mj, Qx, W2, W1, 0);      // (Qy F) Qx
-    scale_kernel<<<grid_for(tot), 256, 0, st>>>(mi, mj, cx, cy, lx, ly, n_fields, W1);
-    gemm_kernel<<<grd, blk, 0, st>>>(mi, mj, Qy, W1, W2, 1);
-    gemm_kernel<<<grd, blk, 0, st>>>(mi, mj, Qx, W2, W1, 0);
-    scatter_kernel<<<grid_for(tot), 256, 0, st>>>(nx, ny, n_fields, W1, grid);
+    const int longest = nx > ny ? nx : ny, in_smem = sp.copy == 0;
+    const size_t smem_side = in_smem ? sizeof(double) * 2 * longest : 0;
+    const size_t smem_x = in_smem ? sizeof(double) * (2 * static_cast<size_t>(nx) + static_cast<size_t>(kRows) * mj) : 0;
+    const size_t smem_y = in_smem ? sizeof(double) * (2 * static_cast<size_t>(ny) + static_cast<size_t>(kRows) * mi) : 0;
+    int rc;
+    if ((rc = allow_smem(side_kernel, smem_side)) != KMC_OK || (rc = allow_smem(x_kernel, smem_x)) != KMC_OK ||
+        (rc = allow_smem(y_kernel, smem_y)) != KMC_OK)
+        return rc;
+    table_kernel<<<grid_for(3LL * (nx + ny)), 128, 0, st>>>(nx, ny, t);
+    side_kernel<<<dim3((longest + 7) / 8, kSides, n_fields), kThreads, smem_side, st>>>(nx, ny, n_fields, t, grid, G, in_smem);
+    x_kernel<<<dim3((mi + kRows - 1) / kRows, n_fields), kThreads, smem_x, st>>>(nx, ny, cx, cy, t, G, Y, W, in_smem);
+    y_kernel<<<dim3((mj + kRows - 1) / kRows, n_fields), kThreads, smem_y, st>>>(nx, ny, t, Y, grid, in_smem);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? KMC_OK : fail_cuda(e, "laplace_basis launch");
+}
+
+extern "C" int kmc_laplace_boundary(int32_t nx, int32_t ny, double xdim, double ydim, double surplus,
+                                    int32_t n_electrodes, const double *xy, double *grid, void *stream)
+{
+    if (nx < 1 || ny < 1 || n_electrodes < 0 || !(xdim > 0) || !(ydim > 0))
+        return fail(KMC_ERR_INVALID, "laplace_boundary: bad mesh (nx %d, ny %d, electrodes %d)", nx, ny, n_electrodes);
+    if (!grid || (!xy && n_electrodes > 0)) return fail(KMC_ERR_INVALID, "laplace_boundary: NULL pointer");
+    const long long nodes = static_cast<long long>(nx + 1) * (ny + 1);
+    if (nodes > (1LL << 30)) return fail(KMC_ERR_INVALID, "laplace_boundary: mesh too large");
+    boundary_kernel<<<grid_for(nodes), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+        nx, ny, xdim / nx, ydim / ny, xdim, surplus, n_electrodes, xy, grid);
+    cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? KMC_OK : fail_cuda(e, "laplace_boundary launch");
 }
 
 extern "C" int kmc_p1_sample(int32_t nx, int32_t ny, double hx, double hy, int32_t n_fields,
@@ -208,11 +328,11 @@ namespace kmc {
 int preload_laplace()
 {
     int rc;
-    if ((rc = touch_kernel(dst_basis_kernel)) != KMC_OK) return rc;
-    if ((rc = touch_kernel(rhs_kernel)) != KMC_OK) return rc;
-    if ((rc = touch_kernel(gemm_kernel)) != KMC_OK) return rc;
-    if ((rc = touch_kernel(scale_kernel)) != KMC_OK) return rc;
-    if ((rc = touch_kernel(scatter_kernel)) != KMC_OK) return rc;
+    if ((rc = touch_kernel(table_kernel)) != KMC_OK) return rc;
+    if ((rc = touch_kernel(side_kernel)) != KMC_OK) return rc;
+    if ((rc = touch_kernel(x_kernel)) != KMC_OK) return rc;
+    if ((rc = touch_kernel(y_kernel)) != KMC_OK) return rc;
+    if ((rc = touch_kernel(boundary_kernel)) != KMC_OK) return rc;
     return touch_kernel(p1_sample_kernel);
 }
 

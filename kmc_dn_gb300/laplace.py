@@ -236,14 +236,19 @@ def solve_basis_fields_gpu(xdim, ydim, electrodes, nx, ny=None, surplus=None, de
     if ydim == 0:
         return solve_basis_fields(xdim, ydim, electrodes, nx)
     ny = nx if ny is None else ny
-    grids = boundary_grids(xdim, ydim, electrodes, nx, ny, surplus)
+    electrodes = np.asarray(electrodes, dtype=np.float64)
+    electrodes = electrodes.reshape(-1, electrodes.shape[-1] if electrodes.ndim == 2 else 2)
+    P = electrodes.shape[0]
     d = torch.device(dev if dev is not None else "cuda")
-    g = torch.as_tensor(grids, dtype=torch.float64).to(d).contiguous()
     L = lib()
-    wsb = L.kmc_laplace_workspace_size(nx, ny, grids.shape[0])
-    ws = torch.empty(max(int(wsb), 8), dtype=torch.uint8, device=d)
-    st = C.c_void_p(torch.cuda.current_stream(d).cuda_stream)
-    check(L.kmc_laplace_basis(nx, ny, xdim / nx, ydim / ny, grids.shape[0], C.c_void_p(g.data_ptr()),
-                              C.c_void_p(ws.data_ptr()), wsb, st))
-    torch.cuda.synchronize(d)
+    with torch.cuda.device(d):
+        xy = torch.as_tensor(np.ascontiguousarray(electrodes[:, :2])).to(d)
+        g = torch.empty((P + 1, ny + 1, nx + 1), dtype=torch.float64, device=d)
+        wsb = L.kmc_laplace_workspace_size(nx, ny, P + 1)
+        ws = torch.empty(max(int(wsb), 8), dtype=torch.uint8, device=d)
+        st = C.c_void_p(torch.cuda.current_stream(d).cuda_stream)
+        check(L.kmc_laplace_boundary(nx, ny, float(xdim), float(ydim), float(xdim / 10 if surplus is None else surplus),
+                                     P, C.c_void_p(xy.data_ptr()), C.c_void_p(g.data_ptr()), st))
+        check(L.kmc_laplace_basis(nx, ny, xdim / nx, ydim / ny, P + 1, C.c_void_p(g.data_ptr()),
+                                  C.c_void_p(ws.data_ptr()), wsb, st))
     return BasisFields(g.cpu().numpy(), xdim, ydim, nx, ny, 2)

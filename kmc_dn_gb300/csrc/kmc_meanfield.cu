@@ -20,10 +20,8 @@
 // site sums its row (outflow) or its column (inflow) in a fixed order, so a
 // run is deterministic and a network's result does not depend on the batch.
 // Two rate precisions:
-//   KMC_MF_RATES_F64  everything in FP64 (the reference's arithmetic up to
-//                     rounding order), the exponentials as products of site
-//                     and pair factors (mf_factors; very large networks:
-//                     exp() per pair),
+//   KMC_MF_RATES_F64  everything in FP64, exp() per pair (the reference's
+//                     arithmetic up to rounding order),
 //   KMC_MF_RATES_F32  FP32 energies and rates (one ex2.approx per pair),
 //                     compensated FP32 row/column sums, FP64 state, step
 //                     and clock: GB300 runs FP64 at 1/64 of FP32, so only
@@ -40,8 +38,12 @@
 namespace kmc {
 namespace {
 
-constexpr int kMfThreads = 128;       // FP32-rate kernel
-constexpr int kMfThreads64 = 256;     // FP64 kernel: two warps a quarter of the SM overlap FP64 and integer work
+constexpr int kMfThreads = 128;
+// FP64 mode, while every network has an SM of its own: two warps a quarter of
+// the SM overlap FP64 and other work (64 networks of N = 30: 10.2 us an
+// iteration, 11.9 with 128 threads; 1024 networks: 76 against 67, whose fewer
+// warps leave fewer exponentials to evaluate in part-filled warps).
+constexpr int kMfThreadsWide = 256;
 constexpr int kMfSmemLimit = 226 * 1024;   // dynamic; leaves room for the static words
 
 __device__ __forceinline__ double warp_sum(double x)
@@ -49,6 +51,13 @@ __device__ __forceinline__ double warp_sum(double x)
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
     return x;
+}
+
+// Whether x may lie outside [0, 1], by its bits (an FP64 comparison costs the
+// unit's 64 cycles): false for every value inside but -0.
+__device__ __forceinline__ bool outside_unit(double x)
+{
+    return static_cast<unsigned long long>(__double_as_longlong(x)) > 0x3ff0000000000000ull;
 }
 
 __device__ __forceinline__ double warp_min(double x)
@@ -128,31 +137,29 @@ __device__ __host__ __forceinline__ int row_stride(int S) { return S | 1; }
 
 }  // namespace
 
-// Largest network of the FP64 path that keeps exponential factors beside the
-// pair constants (36 bytes a pair); larger ones, up to kmc_mf_max_sites,
-// take an exponential per pair (24 bytes).
-constexpr int kMfFactorSites = 77;
+// Exponentials of the FP64 mode waiting to be taken, one warp's: at most 31
+// left over and 32 new ones.
+struct __align__(16) MfQueue {
+    double x[64];   // argument
+    int to[64];     // position in the rates
+};
 
-static size_t factor_smem_bytes(int S)
+// The FP64 mode's queues, where the block has room beside its tables (all
+// but the largest networks; without them every warp takes exponentials for
+// all its lanes, with the same results).
+__host__ __device__ static size_t queue_bytes(int S)
 {
-    const size_t pairs = static_cast<size_t>(S) * row_stride(S);
-    return pairs * (16 + 8 + 8 + 4) + 16 * kExpTable + static_cast<size_t>(S) * (14 * 8 + 2 * 4) + 64;
-}
-
-static size_t pair_smem_bytes(int S, int rates)
-{
-    const size_t pairs = static_cast<size_t>(S) * row_stride(S);
-    const size_t per_pair = rates == KMC_MF_RATES_F64 ? 16 + 8 : 8 + 4;
-    // occ, out, in, avg, eo (double) + e (Real) + occ, 1 - occ (float) per site, + scalars
-    return pairs * per_pair + static_cast<size_t>(S) * (6 * 8 + 2 * 4) + 64;
+    return S <= 95 ? sizeof(MfQueue) * (kMfThreadsWide / 32) : 0;
 }
 
 size_t mf_smem_bytes(int S, int rates)
 {
-    if (rates != KMC_MF_RATES_F64) return pair_smem_bytes(S, rates);
-    const size_t f = factor_smem_bytes(S < kMfFactorSites ? S : kMfFactorSites);
-    const size_t p = S > kMfFactorSites ? pair_smem_bytes(S, rates) : 0;
-    return f > p ? f : p;
+    const size_t pairs = static_cast<size_t>(S) * row_stride(S);
+    const size_t per_pair = rates == KMC_MF_RATES_F64 ? 16 + 8 : 8 + 4;
+    // occ, out, in, avg, eo (double) + e (Real) + FP32: occ, 1 - occ (float);
+    // FP64: 1 - occ (double) per site, + scalars
+    return pairs * per_pair + static_cast<size_t>(S) * (6 * 8 + 2 * 4) + 64 +
+           (rates == KMC_MF_RATES_F64 ? queue_bytes(S) : 0);
 }
 
 namespace {
@@ -171,8 +178,15 @@ struct PairStep {
     }
 };
 
-// One network, an exponential per pair: all of the FP32-rate mode, and the
-// FP64 mode of networks beyond kMfFactorSites.
+// One network.  The FP64 mode's arithmetic is the first version's operation
+// for operation: some networks amplify a rounding by 1e12 and more over a
+// thousand iterations (an occupation that keeps meeting its bound), so a sum
+// in another order or an exponential in factors, both as accurate, end
+// elsewhere.  What it does without is work: an exponential of 0 is 1, and only
+// the pairs with dE > 0, collected 32 at a time in a queue, take one (twenty
+// FP64 instructions, and a warp's FP64 instruction holds its SM quarter's
+// unit for 64 cycles on this part).  64 networks of N = 30, P = 8, 1000
+// iterations: 10.2 ms (18.9 ms with an exponential for every pair).
 template <bool F64, int T>
 __device__ void mf_pairs(const kmc_mf_batch &b)
 {
@@ -207,6 +221,10 @@ __device__ void mf_pairs(const kmc_mf_batch &b)
     Real *e = reinterpret_cast<Real *>(eo + S);   // site energies (electrodes: voltages)
     float *of = reinterpret_cast<float *>(e + S);  // FP32 copy of the probabilities (1 for electrodes)
     float *nf = of + S;                            // and of one minus them (1 for electrodes)
+    double *emp = reinterpret_cast<double *>(e + S);   // FP64: one minus the probabilities (1 for electrodes)
+    MfQueue *queue = nullptr;
+    if (F64 && queue_bytes(S) > 0)
+        queue = reinterpret_cast<MfQueue *>((reinterpret_cast<uintptr_t>(emp + S) + 15) & ~static_cast<uintptr_t>(15)) + warp;
     __shared__ double sh_f, sh_ts, sh_time;
     __shared__ int sh_stop;
 
@@ -220,9 +238,13 @@ __device__ void mf_pairs(const kmc_mf_batch &b)
         KB[i * SP + j] = Pair{static_cast<Real>(K), static_cast<Real>(B)};
     }
     for (int k = tid; k < S; k += T) {
-        occ[k] = k < N ? occ_io[k] : 0.0;
-        of[k] = k < N ? static_cast<float>(occ[k]) : 1.0f;
-        nf[k] = k < N ? 1.0f - of[k] : 1.0f;
+        occ[k] = k < N ? occ_io[k] : F64 ? 1.0 : 0.0;
+        if constexpr (F64) {
+            emp[k] = k < N ? 1.0 - occ[k] : 1.0;
+        } else {
+            of[k] = k < N ? static_cast<float>(occ[k]) : 1.0f;
+            nf[k] = k < N ? 1.0f - of[k] : 1.0f;
+        }
         e[k] = k < N ? Real(0) : static_cast<Real>(se_out[k]);
         avg[k] = (b.record && k < N) ? b.average_occupation[b.site_off[c] + k] : 0.0;
         eo[k] = 0.0;
@@ -232,6 +254,7 @@ __device__ void mf_pairs(const kmc_mf_batch &b)
 
     const Real ec_i = tid < N ? static_cast<Real>(Ec[tid]) : Real(0);
     const double inv_kT = 1.0 / kT;
+    const bool unit = kT == 1.0;
     const float c2 = static_cast<float>(1.4426950408889634 / kT);
     const int64_t hops = b.hops[c];
     double *traffic = b.record ? b.traffic + b.traffic_off[c] : nullptr;
@@ -244,7 +267,7 @@ __device__ void mf_pairs(const kmc_mf_batch &b)
             const Pair *row = KB + i * SP;
 #pragma unroll 4
             for (int j = 0; j < N; ++j) {
-                if constexpr (F64) acc += (1.0 - occ[j]) * row[j].y;
+                if constexpr (F64) acc = fma(emp[j], row[j].y, acc);
                 else acc = fmaf(nf[j], row[j].y, acc);
             }
             e[i] = (i == tid ? ec_i : static_cast<Real>(Ec[i])) - acc;
@@ -254,13 +277,52 @@ __device__ void mf_pairs(const kmc_mf_batch &b)
         // (2) the S x S expected rates, a thread per pair
         PairStep<T> at(tid, S);
         if constexpr (F64) {
-            for (int p = tid; p < SS; p += T, at.next(S)) {
-                const int i = at.i, j = at.j;
-                const Pair kb = KB[i * SP + j];
-                const double w = (j < N ? 1.0 - occ[j] : 1.0) * (i < N ? occ[i] : 1.0);
-                const double dE = e[j] - e[i] - kb.y;
-                rt[i * SP + j] = w * kb.x * exp(-fmax(dE, 0.0) * inv_kT);
+            int queued = 0;
+            auto flush = [&](int n) {     // the first n <= 32 queued exponentials
+                __syncwarp();
+                if (lane < n) rt[queue->to[lane]] *= exp(queue->x[lane]);
+                __syncwarp();
+            };
+            const int rounds = (SS + T - 1) / T;      // (the same for every lane of a warp)
+            for (int n = 0; n < rounds; ++n, at.next(S)) {
+                const bool in = n * T + tid < SS;
+                bool up = false;
+                double x = 0.0;
+                int to = 0;
+                if (in) {
+                    const int i = at.i, j = at.j;
+                    to = i * SP + j;
+                    const Pair kb = KB[to];
+                    const double wk = emp[j] * occ[i] * kb.x;
+                    const double dE = e[j] - e[i] - kb.y;
+                    up = positive(dE) && __double_as_longlong(kb.x) != 0;
+                    x = unit ? -dE : -dE * inv_kT;
+                    if (queue) {
+                        rt[to] = wk;
+                    } else {
+                        rt[to] = up ? wk * exp(x) : wk;
+                    }
+                }
+                if (queue) {
+                    const unsigned ups = __ballot_sync(0xffffffffu, up);
+                    if (up) {
+                        const int q = queued + __popc(ups & ((1u << lane) - 1u));
+                        queue->x[q] = x;
+                        queue->to[q] = to;
+                    }
+                    queued += __popc(ups);
+                    if (queued >= 32) {
+                        flush(32);
+                        queued -= 32;
+                        if (lane < queued) {
+                            queue->x[lane] = queue->x[32 + lane];
+                            queue->to[lane] = queue->to[32 + lane];
+                        }
+                        __syncwarp();
+                    }
+                }
             }
+            if (queued > 0) flush(queued);
         } else {
             constexpr int U = 4;      // pairs in flight
             for (int p = tid; p < SS; p += U * T) {
@@ -361,15 +423,19 @@ __device__ void mf_pairs(const kmc_mf_batch &b)
             double tot = 0.0;
             for (int k = lane; k < S; k += 32) tot += outs[k];
             tot = warp_sum(tot);
-            const double inv = 1.0 / tot;
+            const double inv = __drcp_rn(tot);
             double mc = 1.0;
+            bool less = false;
             for (int k = lane; k < N; k += 32) {
                 const double q = (ins[k] - outs[k]) * inv;
                 const double nv = occ[k] + q;
-                if (nv < 0) mc = fmin(mc, occ[k] / -q);
-                if (nv > 1) mc = fmin(mc, (1.0 - occ[k]) / q);
+                if (outside_unit(nv)) {
+                    if (nv < 0) mc = fmin(mc, occ[k] / -q);
+                    if (nv > 1) mc = fmin(mc, (1.0 - occ[k]) / q);
+                    less = true;
+                }
             }
-            mc = warp_min(mc);
+            if (__any_sync(0xffffffffu, less)) mc = warp_min(mc);
             if (lane == 0) {
                 if (!(tot > 0.0) || !(tot < 1.0e300)) {
                     sh_stop = 1;
@@ -390,9 +456,10 @@ __device__ void mf_pairs(const kmc_mf_batch &b)
             const double net = ins[k] - outs[k];
             if (k < N) {
                 if (b.record) avg[k] += occ[k] * ts;
-                double o = occ[k] + net * f;
-                o = o < 0.0 ? 0.0 : (o > 1.0 ? 1.0 : o);
+                double o = fma(net, f, occ[k]);
+                if (outside_unit(o)) o = o < 0.0 ? 0.0 : (o > 1.0 ? 1.0 : o);
                 occ[k] = o;
+                if constexpr (F64) emp[k] = 1.0 - o;
             } else {
                 eo[k] += net * f;
             }
@@ -424,276 +491,16 @@ __device__ void mf_pairs(const kmc_mf_batch &b)
     }
 }
 
-// One network, FP64, with the exponentials as products (networks of at most
-// kMfFactorSites): exp(-dE/kT) = exp(e_i/kT) exp(-e_j/kT) exp(B_ij/kT), one
-// exponential a site and iteration, the coupling factor tabulated with K.  A
-// pair then costs two multiplications, and its weights are taken out of the
-// sums (out_i = o_i sum_j (1 - o_j) t_ij, in_j = (1 - o_j) sum_i o_i t_ij):
-// four FP64 instructions a pair for the exponential's and the weights' thirty.
-// The FP64 unit's time is the kernel's (64 cycles a warp instruction and SM
-// quarter), so the rest is spread over the block, and compared as
-// integers.  Mantissa and exponent are kept apart
-// (kmc_exp64.cuh); energies beyond its range take the exponential.
-// 64 networks of N = 30, P = 8, 1000 iterations: 5.9 ms (18.9 ms with an
-// exponential per pair).
-__device__ void mf_factors(const kmc_mf_batch &b)
-{
-    constexpr int T = kMfThreads64;
-    extern __shared__ __align__(16) unsigned char smem[];
-    const int c = blockIdx.x;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int N = b.N[c], P = b.P[c], S = N + P;
-    const int SS = S * S;
-    const int SP = row_stride(S);
-    const double nu = b.nu[c], kT = b.kT[c], I0R = b.I_0[c] * b.R[c];
-    const double *dist = b.distances + b.pair_off[c];
-    const double *tcon = b.transitions_constant + b.pair_off[c];
-    const double *Ec = b.E_constant + b.site_off[c];
-    double *se_out = b.site_energies + b.site_off[c];
-    double *occ_io = b.occupation + b.site_off[c];
-
-    double2 *KW = reinterpret_cast<double2 *>(smem);          // K, mantissa of K exp(B/kT)
-    double2 *exp_tab = KW + S * SP;
-    double *Bt = reinterpret_cast<double *>(exp_tab + kExpTable);   // B
-    double *rt = Bt + S * SP;                                 // t_ij
-    double *occ = rt + S * SP;                                // probabilities (1 for electrodes)
-    double *emp = occ + S;                                    // one minus them (1 for electrodes)
-    double *um = emp + S;                                     // exp(e/kT), mantissas
-    double *vm = um + S;                                      // exp(-e/kT)
-    double *outs = vm + S;
-    double *ins = outs + S;
-    double *net = ins + S;
-    double *avg = net + S;
-    double *eo = avg + S;
-    double *e = eo + S;                                       // site energies (electrodes: voltages)
-    double *part = e + S;                                     // [4 S] parts of the sums
-    int *W_k = reinterpret_cast<int *>(part + 4 * S);         // exponents beside KW
-    int *uk = W_k + S * SP;
-    int *vk = uk + S;
-    __shared__ double sh_f, sh_ts, sh_time;
-    __shared__ int sh_stop, wide_always, wide_now[2];
-
-    const bool unit = kT == 1.0;
-    const double inv_kT = 1.0 / kT;
-    if (tid == 0) {
-        sh_time = 0.0;
-        sh_stop = wide_always = wide_now[0] = wide_now[1] = 0;
-    }
-    for (int j = tid; j < kExpTable; j += T) exp_tab[j] = exp_table_entry(j);
-    __syncthreads();
-    for (int p = tid; p < SS; p += T) {
-        const int i = p / S, j = p - (p / S) * S, q = i * SP + j;
-        const double K = (i >= N && j >= N) ? 0.0 : nu * tcon[p];
-        const double B = (i < N && j < N && i != j) ? I0R / dist[p] : 0.0;
-        double rest, f = 1.0;
-        int k = 0;
-        const double x = over_kT(B, unit, kT, inv_kT, rest);
-        if (splittable(x)) f = exp_split(x, rest, exp_tab, k);
-        else wide_always = 1;
-        Bt[q] = B;
-        KW[q] = make_double2(K, K * f);
-        W_k[q] = k;
-    }
-    for (int k = tid; k < S; k += T) {
-        occ[k] = k < N ? occ_io[k] : 1.0;
-        emp[k] = k < N ? 1.0 - occ[k] : 1.0;
-        e[k] = k < N ? 0.0 : se_out[k];
-        avg[k] = (b.record && k < N) ? b.average_occupation[b.site_off[c] + k] : 0.0;
-        eo[k] = 0.0;
-        um[k] = vm[k] = 1.0;
-        uk[k] = vk[k] = 0;
-        if (k >= N) {
-            double rest;
-            const double x = over_kT(e[k], unit, kT, inv_kT, rest);
-            if (splittable(x)) {
-                um[k] = exp_split(x, rest, exp_tab, uk[k]);
-                vm[k] = exp_split(-x, -rest, exp_tab, vk[k]);
-            } else {
-                wide_always = 1;
-            }
-        }
-    }
-    __syncthreads();
-
-    const int64_t hops = b.hops[c];
-    double *traffic = b.record ? b.traffic + b.traffic_off[c] : nullptr;
-    const double Ec0 = (tid >> 2) < N ? Ec[tid >> 2] : 0.0;
-    const int p0 = tid / (2 * S), q0 = tid - p0 * 2 * S;
-    int64_t it = 0;
-    for (; it < hops; ++it) {
-        // (1) energies from the probabilities and their exponentials: four
-        // threads an acceptor, two of which take one exponential each
-        for (int q = tid; q < 4 * ((N + 7) & ~7); q += T) {
-            const int i = q >> 2;
-            double acc = 0.0;
-            if (i < N) {
-                const double *row = Bt + i * SP;      // (the diagonal's B is 0)
-#pragma unroll 4
-                for (int j = q & 3; j < N; j += 4) acc = fma(emp[j], row[j], acc);
-            }
-            acc += __shfl_xor_sync(0xffffffffu, acc, 1);
-            acc += __shfl_xor_sync(0xffffffffu, acc, 2);
-            if (i < N && (q & 3) < 2) {
-                const double ei = (q == tid ? Ec0 : Ec[i]) - acc;
-                const bool leave = (q & 3) == 0;
-                double rest;
-                double x = over_kT(ei, unit, kT, inv_kT, rest);
-                if (!leave) {
-                    x = -x;
-                    rest = -rest;
-                }
-                if (leave) e[i] = ei;
-                if (splittable(x)) (leave ? um : vm)[i] = exp_split(x, rest, exp_tab, (leave ? uk : vk)[i]);
-                else wide_now[it & 1] = 1;
-            }
-        }
-        __syncthreads();
-        const bool wide = wide_always | wide_now[it & 1];
-        if (tid == 0) wide_now[(it + 1) & 1] = 0;
-
-        // (2) t_ij = K min(1, exp(-dE/kT)), a thread per pair
-        PairStep<T> at(tid, S);
-        constexpr int U = 4;      // pairs in flight
-        for (int p = tid; p < SS; p += U * T) {
-            double t[U];
-            int to[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                if (p + u * T < SS) {
-                    const int i = at.i, j = at.j;
-                    to[u] = i * SP + j;
-                    const double2 kw = KW[to[u]];
-                    if (!wide) {
-                        t[u] = scaled_min(kw.y * (um[i] * vm[j]), W_k[to[u]] + uk[i] + vk[j], kw.x);
-                    } else {
-                        const double dE = e[j] - e[i] - Bt[to[u]];
-                        t[u] = kw.x * exp(-fmax(dE, 0.0) * inv_kT);
-                    }
-                }
-                at.next(S);
-            }
-#pragma unroll
-            for (int u = 0; u < U; ++u)
-                if (p + u * T < SS) rt[to[u]] = t[u];
-        }
-        __syncthreads();
-
-        // (3) outflows along rows (items 0..S-1) and inflows down columns
-        // (S..2S-1), each in three parts
-        const int third = (S + 2) / 3;
-        for (int q = tid, item = q0, pt = p0; q < 6 * S; q += T) {
-            const int k = item < S ? item : item - S;
-            const double *v = item < S ? rt + k * SP : rt + k;
-            const double *w = item < S ? emp : occ;
-            const int step = item < S ? 1 : SP;
-            const int n1 = min(S, (pt + 1) * third);
-            double s = 0.0;
-#pragma unroll 4
-            for (int n = pt * third; n < n1; ++n) s = fma(w[n], v[n * step], s);
-            if (pt == 0) (item < S ? outs : ins)[k] = s;
-            else part[(pt - 1) * 2 * S + item] = s;
-            item += T;
-            while (item >= 2 * S) { item -= 2 * S; ++pt; }
-        }
-        __syncthreads();
-        for (int k = tid; k < S; k += T) {
-            const double o = occ[k] * (outs[k] + part[k] + part[2 * S + k]);
-            const double in = emp[k] * (ins[k] + part[S + k] + part[3 * S + k]);
-            outs[k] = o;
-            net[k] = in - o;
-        }
-        __syncthreads();
-
-        // (4) total and step size (one warp; one FP64 division per iteration)
-        if (warp == 0) {
-            double tot = lane < S ? outs[lane] : 0.0;
-            for (int k = lane + 32; k < S; k += 32) tot += outs[k];
-            tot = warp_sum(tot);
-            const double inv = __drcp_rn(tot);
-            double mc = 1.0;
-            bool less = false;
-            for (int k = lane; k < N; k += 32) {
-                const double nv = fma(net[k], inv, occ[k]);
-                // below 0 or above 1, by its bits (values above 1 have larger
-                // bit patterns; NaN compares as neither)
-                const long long bits = __double_as_longlong(nv);
-                if (bits < 0 || bits > __double_as_longlong(1.0)) {
-                    const double q = net[k] * inv;
-                    if (nv < 0) mc = fmin(mc, occ[k] / -q);
-                    if (nv > 1) mc = fmin(mc, (1.0 - occ[k]) / q);
-                    less = true;
-                }
-            }
-            if (__any_sync(0xffffffffu, less)) mc = warp_min(mc);
-            if (lane == 0) {
-                if (!positive(tot) || __double_as_longlong(tot) >= __double_as_longlong(1.0e300)) {
-                    sh_stop = 1;
-                } else {
-                    sh_f = mc * inv;              // fraction of each expected flow moved
-                    sh_ts = 0.98 * mc * inv;      // time step
-                    sh_time += sh_ts;
-                }
-            }
-        }
-        __syncthreads();
-        if (sh_stop) break;
-
-        // (5) record, move the expected charge, clamp
-        const double f = sh_f;
-        if (traffic) {
-            PairStep<T> tr(tid, S);
-            for (int p = tid; p < SS; p += T, tr.next(S)) {
-                const int i = tr.i, j = tr.j;
-                if (i >= N && j >= N) continue;
-                traffic[p] += (occ[i] * emp[j] * rt[i * SP + j] - occ[j] * emp[i] * rt[j * SP + i]) * f;
-            }
-            __syncthreads();
-        }
-        for (int k = tid; k < S; k += T) {
-            if (k < N) {
-                if (b.record) avg[k] += occ[k] * sh_ts;
-                double o = fma(net[k], f, occ[k]);
-                const long long bits = __double_as_longlong(o);
-                if (bits < 0 || bits > __double_as_longlong(1.0)) o = o < 0.0 ? 0.0 : (o > 1.0 ? 1.0 : o);
-                occ[k] = o;
-                emp[k] = 1.0 - o;
-            } else {
-                eo[k] += net[k] * f;
-            }
-        }
-        __syncthreads();
-    }
-
-    // outputs
-    for (int k = tid; k < S; k += T) {
-        if (k < N) {
-            occ_io[k] = occ[k];
-            se_out[k] = e[k];
-            if (b.record) b.average_occupation[b.site_off[c] + k] = avg[k];
-        } else {
-            b.electrode_occupation[b.el_off[c] + (k - N)] = eo[k];
-        }
-    }
-    if (tid == 0) {
-        b.time[c] = sh_time;
-        if (b.status) b.status[c] = sh_stop ? KMC_ERR_NONFINITE : KMC_OK;
-        if (b.iterations_done) b.iterations_done[c] = it;
-    }
-}
-
 // One block per network.
 __global__ void __launch_bounds__(kMfThreads, 8) mf_kernel_f32(kmc_mf_batch b)
 {
     mf_pairs<false, kMfThreads>(b);
 }
 
-// The path is chosen by each network's own size, so that its result does not
-// depend on the batch.
-__global__ void __launch_bounds__(kMfThreads64, 2) mf_kernel_f64(kmc_mf_batch b)
+template <int T>
+__global__ void __launch_bounds__(T, 512 / T) mf_kernel_f64(kmc_mf_batch b)
 {
-    const int S = b.N[blockIdx.x] + b.P[blockIdx.x];
-    if (S >= 1 && S <= kMfFactorSites && S <= b.max_sites) mf_factors(b);
-    else mf_pairs<true, kMfThreads64>(b);
+    mf_pairs<true, T>(b);
 }
 
 }  // namespace
@@ -734,15 +541,21 @@ extern "C" int kmc_mf_run(const kmc_mf_batch *b, void *stream)
     const size_t smem = mf_smem_bytes(b->max_sites, b->rates);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     cudaError_t e;
-    if (b->rates == KMC_MF_RATES_F64) {
-        e = cudaFuncSetAttribute(mf_kernel_f64, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    int dev = 0, sms = 0;
+    if ((e = cudaGetDevice(&dev)) != cudaSuccess ||
+        (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
+        return fail_cuda(e, "mf_run: device query");
+    auto launch = [&](auto *kernel, int threads) -> int {
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
         if (e != cudaSuccess) return fail_cuda(e, "mf_run smem attribute");
-        mf_kernel_f64<<<b->n_chains, kMfThreads64, smem, st>>>(*b);
-    } else {
-        e = cudaFuncSetAttribute(mf_kernel_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-        if (e != cudaSuccess) return fail_cuda(e, "mf_run smem attribute");
-        mf_kernel_f32<<<b->n_chains, kMfThreads, smem, st>>>(*b);
-    }
+        kernel<<<b->n_chains, threads, smem, st>>>(*b);
+        return KMC_OK;
+    };
+    // (a network's result does not depend on the threads that share it)
+    const int rc = b->rates != KMC_MF_RATES_F64 ? launch(mf_kernel_f32, kMfThreads)
+                   : b->n_chains <= sms ? launch(mf_kernel_f64<kMfThreadsWide>, kMfThreadsWide)
+                                        : launch(mf_kernel_f64<kMfThreads>, kMfThreads);
+    if (rc != KMC_OK) return rc;
     e = cudaGetLastError();
     return e == cudaSuccess ? KMC_OK : fail_cuda(e, "mf_run launch");
 }
@@ -859,7 +672,8 @@ namespace kmc {
 int preload_meanfield()
 {
     int rc;
-    if ((rc = touch_kernel(mf_kernel_f64)) != KMC_OK) return rc;
+    if ((rc = touch_kernel(mf_kernel_f64<kMfThreads>)) != KMC_OK) return rc;
+    if ((rc = touch_kernel(mf_kernel_f64<kMfThreadsWide>)) != KMC_OK) return rc;
     return touch_kernel(mf_kernel_f32);
 }
 

@@ -330,6 +330,19 @@ typedef struct kmc_batch {
 int kmc_build_table(int32_t n_acceptors, int32_t n_electrodes, double nu, double I_0, double R,
                     const double *distances, const double *transitions_constant,
                     float *tab_LB, void *stream);
+/*
+ * kmc_build_table for n_tables geometries whose FP64 tables are HOST arrays:
+ * table t (S = n_acceptors[t] + n_electrodes[t]) goes to tab_LB +
+ * tab_off[t] floats.  All arguments but tab_LB are host arrays, distances
+ * and transitions_constant arrays of n_tables host pointers.  One launch for
+ * all of them.  Returns when the tables are built (the host arrays are free
+ * then).
+ */
+int kmc_build_tables(int32_t n_tables, const int32_t *n_acceptors, const int32_t *n_electrodes,
+                     const double *nu, const double *I_0, const double *R,
+                     const double *const *distances, const double *const *transitions_constant,
+                     const int64_t *tab_off, float *tab_LB, void *stream);
+
 
 /*
  * Constant site energies of many chains on one geometry from the Laplace

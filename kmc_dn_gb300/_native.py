@@ -110,6 +110,7 @@ _SIGS = {
     "kmc_simulate_f64_static": (C.c_int, [_i32, _i32, _f64, _f64, _f64, _f64, _vp, _vp, _vp, _vp, _vp,
                                           _vp, _i64, _i32, _vp, _vp, _vp, _u64, _vp, _vp, _vp, _vp]),
     "kmc_build_table": (C.c_int, [_i32, _i32, _f64, _f64, _f64, _vp, _vp, _vp, _vp]),
+    "kmc_build_tables": (C.c_int, [_i32, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
     "kmc_site_energies": (C.c_int, [_i32, _i32, _i32, _vp, _vp, _f64, _vp, _vp, _vp, _vp]),
     "kmc_run_batch": (C.c_int, [C.POINTER(KmcBatch), _vp]),
     "kmc_engine_lane_options": (C.c_int, []),

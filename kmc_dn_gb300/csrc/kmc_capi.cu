@@ -601,6 +601,15 @@ int kmc_build_table(int32_t n_acceptors, int32_t n_electrodes, double nu, double
                        tab_LB, static_cast<cudaStream_t>(stream));
 }
 
+int kmc_build_tables(int32_t n_tables, const int32_t *n_acceptors, const int32_t *n_electrodes,
+                     const double *nu, const double *I_0, const double *R, const double *const *distances,
+                     const double *const *transitions_constant, const int64_t *tab_off, float *tab_LB,
+                     void *stream)
+{
+    return build_tables(n_tables, n_acceptors, n_electrodes, nu, I_0, R, distances, transitions_constant,
+                        tab_off, tab_LB, static_cast<cudaStream_t>(stream));
+}
+
 int kmc_site_energies(int32_t n_chains, int32_t n_acceptors, int32_t n_electrodes,
                       const double *basis, const double *voltages, double mu, const double *comp,
                       float *E_constant, float *el_energy, void *stream)

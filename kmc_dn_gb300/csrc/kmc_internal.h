@@ -48,6 +48,8 @@ inline int touch_kernel(K *kernel)
 int section_clocks(uint64_t *out, int reset);
 int build_table(int N, int P, double nu, double I0, double R, const double *d, const double *tc,
                 float *tab, cudaStream_t st);
+int build_tables(int n, const int32_t *N, const int32_t *P, const double *nu, const double *I0, const double *R,
+                 const double *const *d, const double *const *tc, const int64_t *off, float *tab, cudaStream_t st);
 int site_energies(int n_chains, int N, int P, const double *basis, const double *V, double mu,
                   const double *comp, float *Ec, float *Vel, cudaStream_t st);
 int simulate_f64(int N, int P, double nu, double kT, double I0, double R, uint8_t *occ,

@@ -64,6 +64,70 @@ def _dev(a, dtype, dev):
     return torch.as_tensor(np.require(a, requirements=("C", "W")), dtype=dtype).to(dev)
 
 
+def _version(t):
+    """A tensor's count of in-place writes; None where it has none (inference mode)."""
+    try:
+        return t._version
+    except RuntimeError:
+        return None
+
+
+class _Pack:
+    """Arrays of one launch in one device buffer: the inputs go over in one
+    copy, the zeroed state behind them is one fill, and a run of neighbouring
+    arrays (the results) comes back in one copy.  (A copy of its own for each
+    array cost 30 us apiece, 1 ms of a 1000-hop call.)
+
+    ``add`` / ``zeros`` name the arrays in buffer order (all inputs before the
+    first zeros); ``upload`` returns the tensors by name, views of the
+    buffer."""
+    _NP = {torch.uint8: np.uint8, torch.int32: np.int32, torch.int64: np.int64, torch.float32: np.float32,
+           torch.float64: np.float64}
+
+    def __init__(self):
+        self._items = []          # (name, offset, bytes, dtype, shape, array or None)
+        self._size = 0
+        self._inputs = 0
+
+    def _place(self, name, count, dtype, shape, a):
+        nbytes = count * np.dtype(self._NP[dtype]).itemsize
+        self._items.append((name, self._size, nbytes, dtype, shape, a))
+        self._size += (nbytes + 255) & ~255
+
+    def add(self, name, a, dtype):
+        a = np.ascontiguousarray(np.asarray(a).astype(self._NP[dtype], copy=False))
+        self._place(name, a.size, dtype, a.shape, a)
+        self._inputs = self._size
+
+    def zeros(self, name, shape, dtype):
+        shape = (shape,) if isinstance(shape, int) else tuple(shape)
+        self._place(name, int(np.prod(shape, dtype=np.int64)), dtype, shape, None)
+
+    def upload(self, dev):
+        host = np.empty(self._inputs, np.uint8)
+        for _, off, nb, _, _, a in self._items:
+            if a is not None:
+                host[off:off + nb] = a.reshape(-1).view(np.uint8)
+        self.buffer = torch.empty(max(self._size, 256), dtype=torch.uint8, device=dev)
+        # the fill first: the copy from pageable memory waits for the stream,
+        # so the buffer is complete for launches on any stream
+        if self._size > self._inputs:
+            self.buffer[self._inputs:].zero_()
+        if self._inputs:
+            self.buffer[:self._inputs].copy_(torch.from_numpy(host))
+        return {name: self.buffer[off:off + nb].view(dt).view(shape) for name, off, nb, dt, shape, _ in self._items}
+
+    def download(self, first, last):
+        """The arrays from `first` to `last` (in buffer order) on the host, by
+        name, in one copy."""
+        names = [it[0] for it in self._items]
+        part = self._items[names.index(first):names.index(last) + 1]
+        base = part[0][1]
+        host = self.buffer[base:part[-1][1] + part[-1][2]].cpu().numpy()
+        return {name: host[off - base:off - base + nb].view(self._NP[dt]).reshape(shape)
+                for name, off, nb, dt, shape, _ in part}
+
+
 # ---------------------------------------------------------------------------
 # plain FP64 single chain
 # ---------------------------------------------------------------------------
@@ -81,44 +145,52 @@ def simulate_f64(N, P, nu, kT, I_0, R, occupation, distances, E_constant, site_e
     S = N + P
     hops = int(hops)
     f64 = torch.float64
-    occ = _dev(np.asarray(occupation, dtype=np.uint8).reshape(N), torch.uint8, d)
-    dist = _dev(np.asarray(distances, np.float64).reshape(S, S), f64, d)
-    tc = _dev(np.asarray(transitions_constant, np.float64).reshape(S, S), f64, d)
-    ec = _dev(np.asarray(E_constant, np.float64).reshape(N), f64, d)
-    se = _dev(np.asarray(site_energies, np.float64).reshape(S), f64, d)
-    eo0 = np.zeros(P, np.int64) if electrode_occupation is None else np.asarray(electrode_occupation, np.int64)
-    eo = _dev(eo0.reshape(P), torch.int64, d)
-    traffic = torch.zeros((S, S), dtype=f64, device=d) if record else None
-    oit = torch.zeros(max(N, 1), dtype=f64, device=d) if record else None
     u = None
     if uniforms is not None:
-        u = _dev(np.asarray(uniforms, np.float64), f64, d)
-        if u.numel() < 2 * hops:
+        u = np.asarray(uniforms, np.float64).reshape(-1)
+        if u.size < 2 * hops:
             raise ValueError("replay stream shorter than 2*hops")
-    log = torch.zeros(2 * max(hops, 1), dtype=torch.int32, device=d) if hop_log else None
-    t_out = torch.zeros(1, dtype=f64, device=d)
-    st_out = torch.zeros(1, dtype=torch.int32, device=d)
+    eo0 = np.zeros(P, np.int64) if electrode_occupation is None else np.asarray(electrode_occupation, np.int64)
+    pk = _Pack()
+    pk.add("dist", np.asarray(distances, np.float64).reshape(S, S), f64)
+    pk.add("tc", np.asarray(transitions_constant, np.float64).reshape(S, S), f64)
+    pk.add("ec", np.asarray(E_constant, np.float64).reshape(N), f64)
+    pk.add("se", np.asarray(site_energies, np.float64).reshape(S), f64)
+    if u is not None:
+        pk.add("u", u, f64)
+    pk.add("eo", eo0.reshape(P), torch.int64)
+    pk.add("occ", np.asarray(occupation, dtype=np.uint8).reshape(N), torch.uint8)
+    pk.zeros("time", 1, f64)
+    pk.zeros("status", 1, torch.int32)
+    if record:
+        pk.zeros("oit", max(N, 1), f64)
+        pk.zeros("traffic", (S, S), f64)
+    if hop_log:
+        pk.zeros("log", 2 * max(hops, 1), torch.int32)
+    if flux:
+        pk.zeros("flux", max(P, 1), f64)
+    t = pk.upload(d)
     L = lib()
     wsb = L.kmc_simulate_f64_workspace_size(S)
     ws = torch.empty(max(wsb, 8), dtype=torch.uint8, device=d)
-    fx = torch.zeros(max(P, 1), dtype=f64, device=d) if flux else None
-    args = (N, P, float(nu), float(kT), float(I_0), float(R), _ptr(occ), _ptr(dist),
-            _ptr(ec), _ptr(se), _ptr(tc), _ptr(eo), hops, int(bool(record)),
-            _ptr(traffic), _ptr(oit), _ptr(u), int(seed) & (2**64 - 1), _ptr(log),
-            _ptr(t_out), _ptr(st_out), _ptr(ws), wsb, _stream_handle(stream))
+    args = (N, P, float(nu), float(kT), float(I_0), float(R), _ptr(t["occ"]), _ptr(t["dist"]),
+            _ptr(t["ec"]), _ptr(t["se"]), _ptr(t["tc"]), _ptr(t["eo"]), hops, int(bool(record)),
+            _ptr(t.get("traffic")), _ptr(t.get("oit")), _ptr(t.get("u")), int(seed) & (2**64 - 1), _ptr(t.get("log")),
+            _ptr(t["time"]), _ptr(t["status"]), _ptr(ws), wsb, _stream_handle(stream))
     if flux:
-        check(L.kmc_simulate_f64_flux(*args, _ptr(fx)))
+        check(L.kmc_simulate_f64_flux(*args, _ptr(t["flux"])))
     else:
         check(L.kmc_simulate_f64(*args))
     torch.cuda.synchronize(d)
-    out = dict(time=float(t_out.item()), occupation=occ.cpu().numpy().astype(bool),
-               electrode_occupation=eo.cpu().numpy(), status=int(st_out.item()))
-    out["traffic"] = traffic.cpu().numpy() if record else np.zeros((S, S))
-    out["occupations_in_time"] = oit.cpu().numpy()[:N] if record else np.zeros(N)
+    r = pk.download("eo", pk._items[-1][0])
+    out = dict(time=float(r["time"][0]), occupation=r["occ"].astype(bool), electrode_occupation=r["eo"],
+               status=int(r["status"][0]))
+    out["traffic"] = r["traffic"] if record else np.zeros((S, S))
+    out["occupations_in_time"] = r["oit"][:N] if record else np.zeros(N)
     if hop_log:
-        out["hop_log"] = log.cpu().numpy()[: 2 * hops].reshape(hops, 2)
+        out["hop_log"] = r["log"][: 2 * hops].reshape(hops, 2)
     if flux:
-        out["flux_time"] = fx.cpu().numpy()[:P]
+        out["flux_time"] = r["flux"][:P]
     return out
 
 
@@ -195,20 +267,28 @@ def simulate_f64_many(chains, hops, seeds, *, dev=None, record=False, flux=False
     el_off = np.concatenate([[0], np.cumsum(Ps)[:-1]]).astype(np.int64)
     tr_off = np.concatenate([[0], np.cumsum(Ss.astype(np.int64) ** 2)[:-1]]).astype(np.int64)
     smax = int(Ss.max())
-    T = lambda a, dt: _dev(a, dt, d)  # noqa: E731
-    keep = dict(
-        N=T(Ns, torch.int32), P=T(Ps, torch.int32),
-        nu=T([float(ch["nu"]) for ch in chains], f64), kT=T([float(ch["kT"]) for ch in chains], f64),
-        I_0=T([float(ch["I_0"]) for ch in chains], f64), R=T([float(ch["R"]) for ch in chains], f64),
-        pair_off=T(pair_off, i64), distances=T(cat([b[0] for b in blocks], np.float64), f64),
-        tc=T(cat([b[1] for b in blocks], np.float64), f64),
-        site_off=T(site_off, i64), Ec=T(cat([ch["E_constant"] for ch in chains], np.float64), f64),
-        se_off=T(se_off, i64), se=T(cat([ch["site_energies"] for ch in chains], np.float64), f64),
-        occ=T(cat([ch["occupation"] for ch in chains], np.uint8), torch.uint8),
-        el_off=T(el_off, i64), eo=torch.zeros(max(int(Ps.sum()), 1), dtype=i64, device=d),
-        hops=T(np.broadcast_to(np.asarray(hops, np.int64), (n,)), i64),
-        seeds=T(np.asarray([int(s_) & (2**64 - 1) for s_ in seeds], np.uint64).view(np.int64), i64),
-        t_out=torch.zeros(n, dtype=f64, device=d), s_out=torch.zeros(n, dtype=torch.int32, device=d))
+    pk = _Pack()
+    i32 = torch.int32
+    for k, a, dt in (("N", Ns, i32), ("P", Ps, i32), ("nu", [float(ch["nu"]) for ch in chains], f64),
+                     ("kT", [float(ch["kT"]) for ch in chains], f64), ("I_0", [float(ch["I_0"]) for ch in chains], f64),
+                     ("R", [float(ch["R"]) for ch in chains], f64), ("pair_off", pair_off, i64),
+                     ("distances", cat([b[0] for b in blocks], np.float64), f64),
+                     ("tc", cat([b[1] for b in blocks], np.float64), f64), ("site_off", site_off, i64),
+                     ("Ec", cat([ch["E_constant"] for ch in chains], np.float64), f64), ("se_off", se_off, i64),
+                     ("se", cat([ch["site_energies"] for ch in chains], np.float64), f64), ("el_off", el_off, i64),
+                     ("hops", np.broadcast_to(np.asarray(hops, np.int64), (n,)), i64),
+                     ("seeds", np.asarray([int(s_) & (2**64 - 1) for s_ in seeds], np.uint64).view(np.int64), i64),
+                     ("tr_off", tr_off, i64),
+                     ("occ", cat([ch["occupation"] for ch in chains], np.uint8), torch.uint8)):
+        pk.add(k, a, dt)
+    pk.zeros("t_out", n, f64)
+    pk.zeros("eo", max(int(Ps.sum()), 1), i64)
+    pk.zeros("s_out", n, i32)
+    if record:
+        pk.zeros("oit", max(int(Ns.sum()), 1), f64)
+    if flux:
+        pk.zeros("fx", max(int(Ps.sum()), 1), f64)
+    keep = pk.upload(d)
     L = lib()
     wsb = L.kmc_simulate_f64_batch_workspace_size(n, smax)
     keep["ws"] = torch.empty(max(wsb, 8), dtype=torch.uint8, device=d)
@@ -224,29 +304,21 @@ def simulate_f64_many(chains, hops, seeds, *, dev=None, record=False, flux=False
                                                       keep["eo"].data_ptr())
     b.hops, b.seeds = keep["hops"].data_ptr(), keep["seeds"].data_ptr()
     if record:
-        keep["tr_off"] = T(tr_off, i64)
         keep["tr"] = torch.zeros(max(int((Ss.astype(np.int64) ** 2).sum()), 1), dtype=f64, device=d)
-        keep["oit"] = torch.zeros(max(int(Ns.sum()), 1), dtype=f64, device=d)
         b.traffic_off, b.traffic, b.occupations_in_time = (keep["tr_off"].data_ptr(), keep["tr"].data_ptr(),
                                                            keep["oit"].data_ptr())
     if flux:
-        keep["fx"] = torch.zeros(max(int(Ps.sum()), 1), dtype=f64, device=d)
         b.flux_time = keep["fx"].data_ptr()
     b.time_out, b.status_out = keep["t_out"].data_ptr(), keep["s_out"].data_ptr()
     b.workspace, b.workspace_bytes = keep["ws"].data_ptr(), wsb
     check(L.kmc_simulate_f64_batch(C.byref(b), _stream_handle()))
     torch.cuda.synchronize(d)
-    times = keep["t_out"].cpu().numpy()
-    eo = keep["eo"].cpu().numpy()
-    eos = [eo[o:o + p] for o, p in zip(el_off, Ps)]
-    status = keep["s_out"].cpu().numpy()
-    res = [times, eos, status]
+    r = pk.download("t_out", pk._items[-1][0])
+    res = [r["t_out"], [r["eo"][o:o + p] for o, p in zip(el_off, Ps)], r["s_out"]]
     if record:
-        oit = keep["oit"].cpu().numpy()
-        res.append([oit[o:o + k] for o, k in zip(site_off, Ns)])
+        res.append([r["oit"][o:o + k] for o, k in zip(site_off, Ns)])
     if flux:
-        fx = keep["fx"].cpu().numpy()
-        res.append([fx[o:o + p] for o, p in zip(el_off, Ps)])
+        res.append([r["fx"][o:o + p] for o, p in zip(el_off, Ps)])
     return tuple(res)
 
 
@@ -408,26 +480,19 @@ class TableSet:
             raise ValueError("the engine supports at most 64 electrodes")
         if pair_mode not in ("table", "positions"):
             raise ValueError("pair_mode must be 'table' or 'positions'")
-        tab_off = np.zeros(len(self.specs), np.int64)
-        off = 0
+        SS = (Ns.astype(np.int64) + Ps) ** 2
         build = pair_mode == "table"          # positions mode never reads the pair tables
-        for i, t in enumerate(self.specs):
-            tab_off[i] = off
-            off += 2 * t.S * t.S if build else 0
-        self.tab_LB = torch.empty(max(off, 2), dtype=torch.float32, device=d)
-        L = lib()
-        sh = _stream_handle()
-        for i, t in enumerate(self.specs if build else []):
-            dd = _dev(np.asarray(t.distances, np.float64).reshape(t.S, t.S), torch.float64, d)
-            tc = _dev(np.asarray(t.transitions_constant, np.float64).reshape(t.S, t.S), torch.float64, d)
-            check(L.kmc_build_table(t.N, t.P, float(t.nu), float(t.I_0), float(t.R), _ptr(dd), _ptr(tc),
-                                    C.c_void_p(self.tab_LB.data_ptr() + 4 * int(tab_off[i])), sh))
-            torch.cuda.current_stream().synchronize()
-        self.tab_N = _dev(Ns, torch.int32, d)
-        self.tab_P = _dev(Ps, torch.int32, d)
-        self.tab_off = _dev(tab_off, torch.int64, d)
+        tab_off = np.zeros(len(self.specs), np.int64)
+        if build:
+            tab_off[1:] = np.cumsum(2 * SS)[:-1]
+        self.tab_LB = torch.empty(max(int(2 * SS.sum()) if build else 0, 2), dtype=torch.float32, device=d)
+        if build and self.specs:
+            build_tables(self.specs, Ns, Ps, tab_off, self.tab_LB)
+        pk = _Pack()
+        pk.add("N", Ns, torch.int32)
+        pk.add("P", Ps, torch.int32)
+        pk.add("off", tab_off, torch.int64)
         self.pair_mode = _native.PAIRS_POSITIONS if pair_mode == "positions" else _native.PAIRS_TABLE
-        self.tab_pos = self.tab_pos_off = self.tab_coef = None
         if pair_mode == "positions":
             pos_off = np.zeros(len(self.specs), np.int64)
             rows, coef, off = [], [], 0
@@ -440,9 +505,30 @@ class TableSet:
                 pos_off[i] = off
                 off += 4 * t.S
                 coef.append([-2.0 * np.log2(np.e) / t.ab, np.log2(t.nu * t.nu), t.I_0 * t.R, 0.0])
-            self.tab_pos = _dev(np.concatenate(rows), torch.float32, d)
-            self.tab_pos_off = _dev(pos_off, torch.int64, d)
-            self.tab_coef = _dev(np.asarray(coef, np.float32).reshape(-1), torch.float32, d)
+            pk.add("pos", np.concatenate(rows), torch.float32)
+            pk.add("pos_off", pos_off, torch.int64)
+            pk.add("coef", np.asarray(coef, np.float32).reshape(-1), torch.float32)
+        dv = pk.upload(d)
+        self.tab_N, self.tab_P, self.tab_off = dv["N"], dv["P"], dv["off"]
+        self.tab_pos, self.tab_pos_off, self.tab_coef = dv.get("pos"), dv.get("pos_off"), dv.get("coef")
+
+
+def build_tables(specs, Ns, Ps, tab_off, tab_LB):
+    """FP32 pair tables of all specs from their FP64 host tables
+    (kmc_build_tables), into tab_LB at tab_off (floats)."""
+    n = len(specs)
+    keep = [np.ascontiguousarray(np.asarray(a, np.float64).reshape(t.S, t.S))
+            for t in specs for a in (t.distances, t.transitions_constant)]
+    dist = (C.c_void_p * n)(*[a.ctypes.data for a in keep[0::2]])
+    tc = (C.c_void_p * n)(*[a.ctypes.data for a in keep[1::2]])
+    consts = np.array([[t.nu, t.I_0, t.R] for t in specs], np.float64)
+    cols = [np.ascontiguousarray(consts[:, k]) for k in range(3)]
+    off = np.ascontiguousarray(tab_off, np.int64)
+    Ns, Ps = np.ascontiguousarray(Ns, np.int32), np.ascontiguousarray(Ps, np.int32)
+    p = lambda a: C.c_void_p(a.ctypes.data)  # noqa: E731
+    with torch.cuda.device(tab_LB.device):
+        check(lib().kmc_build_tables(n, p(Ns), p(Ps), *[p(a) for a in cols], dist, tc, p(off), _ptr(tab_LB),
+                                     _stream_handle()))
 
 
 class Batch:
@@ -510,34 +596,56 @@ class Batch:
         nsite = int(self.N_c.sum())
         nel = int(self.P_c.sum())
 
-        def pool(vals, total, dtype, np_dtype):
+        def pool(vals, total, np_dtype):
             if isinstance(vals, np.ndarray) and vals.ndim == 2:
                 flat = vals.astype(np_dtype).reshape(-1)
             else:
                 flat = np.concatenate([np.asarray(v, np_dtype).reshape(-1) for v in vals]) if total else np.zeros(0, np_dtype)
             if flat.shape[0] != total:
                 raise ValueError(f"pool size {flat.shape[0]} != {total}")
-            return _dev(flat if total else np.zeros(1, np_dtype), dtype, d)
+            return flat if total else np.zeros(1, np_dtype)
 
-        self.E_constant = E_constant_dev if E_constant_dev is not None else pool(E_constant, nsite, torch.float32, np.float32)
-        self.el_energy = el_energy_dev if el_energy_dev is not None else pool(el_energy, nel, torch.float32, np.float32)
-        self.occupation = pool(occupation, nsite, torch.uint8, np.uint8)
-        self.chain_tab_d = _dev(ct, torch.int32, d)
+        hops_c = np.broadcast_to(np.asarray(hops, np.int64), (n,))
         kT32 = np.broadcast_to(np.asarray(kT, np.float32), (n,))
-        self.kT = _dev(kT32, torch.float32, d)
         # one temperature for every chain: the engine may fold it into a staged table
         self.uniform_kT = float(kT32[0]) if n and np.all(kT32 == kT32[0]) else 0.0
-        self.site_off_d = _dev(self.site_off, torch.int64, d)
-        self.el_off_d = _dev(self.el_off, torch.int64, d)
-        self.pair_off_d = _dev(self.pair_off, torch.int64, d)
-        self.electrode_occupation = torch.zeros(max(nel, 1), dtype=torch.int64, device=d)
-        self.time = torch.zeros(n, dtype=torch.float64, device=d)
-        self.hops_done = torch.zeros(n, dtype=torch.int64, device=d)
-        self.hops_total = _dev(np.broadcast_to(np.asarray(hops, np.int64), (n,)), torch.int64, d)
         sid = np.arange(n, dtype=np.uint64) if streams is None else np.asarray(streams, np.uint64)
-        self.stream_ids = _dev(sid.view(np.int64), torch.int64, d)
-        self.status = torch.zeros(n, dtype=torch.int32, device=d)
-        self.n_pairs = torch.zeros(n, dtype=torch.int64, device=d)
+        f32, i32, i64 = torch.float32, torch.int32, torch.int64
+        pk = self._pack = _Pack()
+        if E_constant_dev is None:
+            pk.add("E_constant", pool(E_constant, nsite, np.float32), f32)
+        if el_energy_dev is None:
+            pk.add("el_energy", pool(el_energy, nel, np.float32), f32)
+        pk.add("chain_tab", ct, i32)
+        pk.add("kT", kT32, f32)
+        pk.add("site_off", self.site_off, i64)
+        pk.add("el_off", self.el_off, i64)
+        pk.add("pair_off", self.pair_off, i64)
+        pk.add("hops_total", hops_c, i64)
+        pk.add("streams", sid.view(np.int64), i64)
+        bins = make_work_lists(self.S_c, hops_c, lanes, sms=self._sms)
+        for k, (_, work, _, _) in enumerate(bins):
+            pk.add(f"work{k}", work, i32)
+        # the state: from here on one copy brings it back
+        pk.add("occupation", pool(occupation, nsite, np.uint8), torch.uint8)
+        pk.zeros("electrode_occupation", max(nel, 1), i64)
+        pk.zeros("time", n, torch.float64)
+        pk.zeros("hops_done", n, i64)
+        pk.zeros("n_pairs", n, i64)
+        pk.zeros("status", n, i32)
+        dv = pk.upload(d)
+        self.E_constant = E_constant_dev if E_constant_dev is not None else dv["E_constant"]
+        self.el_energy = el_energy_dev if el_energy_dev is not None else dv["el_energy"]
+        self.occupation, self.chain_tab_d, self.kT = dv["occupation"], dv["chain_tab"], dv["kT"]
+        self.site_off_d, self.el_off_d, self.pair_off_d = dv["site_off"], dv["el_off"], dv["pair_off"]
+        self.electrode_occupation, self.time, self.hops_done = dv["electrode_occupation"], dv["time"], dv["hops_done"]
+        self.hops_total, self.stream_ids = dv["hops_total"], dv["streams"]
+        self.status, self.n_pairs = dv["status"], dv["n_pairs"]
+        # the largest budget, while nobody has written to the tensor since
+        self._budget = (int(hops_c.max()) if n else 1, self.hops_total, _version(self.hops_total))
+        self._state = {k: dv[k] for k in ("occupation", "electrode_occupation", "time", "hops_done", "n_pairs", "status")}
+        self._bins = [dict(G=G, n_work=len(work) // max(1, 32 // G), work=dv[f"work{k}"], max_sites=smax, chains=order)
+                      for k, (G, work, order, smax) in enumerate(bins)]
         if self.record:
             self.occ_time = torch.zeros(max(nsite, 1), dtype=torch.float64, device=d)
             self.occ_since = torch.zeros(max(nsite, 1), dtype=torch.float64, device=d)
@@ -574,7 +682,6 @@ class Batch:
         self.energy_drift = torch.zeros(n, dtype=torch.float32, device=d) if measure_drift else None
         self.cancel = None            # a CancelWord, or None
         self.time_budget_ns = 0       # per launch and chain; 0: none
-        self._bins = self._make_bins(lanes, np.broadcast_to(np.asarray(hops, np.int64), (n,)))
         # persistent launches: one work counter per bin, zeroed before each launch
         self.persistent = bool(persistent)
         self._counters = (torch.zeros(max(len(self._bins), 1), dtype=torch.int32, device=d)
@@ -589,14 +696,6 @@ class Batch:
         elif isinstance(w, dict):
             w = w.get(G, 4)
         return int(w) if w else 4
-
-    # -- work lists --------------------------------------------------------
-    def _make_bins(self, lanes, hops):
-        bins = []
-        for G, work, order, smax in make_work_lists(self.S_c, hops, lanes, sms=self._sms):
-            bins.append(dict(G=G, n_work=len(work) // max(1, 32 // G), work=_dev(work, torch.int32, self.dev),
-                             max_sites=smax, chains=order))
-        return bins
 
     def _struct(self, bin_, seg):
         b = _native.KmcBatch()
@@ -655,16 +754,37 @@ class Batch:
 
     def launch(self, max_hops_per_launch=None, stream=None, bin_streams=None):
         """One launch per size bin: advance every chain by up to
-        max_hops_per_launch hops (a multiple of the re-anchor period).  Bins
-        go to `stream`, or round-robin to `bin_streams` so that launches of
-        different sizes run side by side (the caller synchronises)."""
+        max_hops_per_launch hops (a multiple of the re-anchor period).  The
+        bins run side by side: the first on `stream` (default: the current
+        one), the others on streams forked from it and joined back to it, or
+        all round-robin on `bin_streams` (the caller synchronises)."""
         seg = max_hops_per_launch
         if seg is None:
-            seg = int(self.hops_total.max().item()) if self.n else 1
+            top, tensor, version = self._budget
+            if self.hops_total is not tensor or version is None or _version(tensor) != version:
+                top = int(self.hops_total.max().item()) if self.n else 1
+            seg = top
         seg = max(self.reanchor, ((int(seg) + self.reanchor - 1) // self.reanchor) * self.reanchor)
+        if len(self._bins) > 1 and not bin_streams:
+            main = stream if stream is not None else torch.cuda.current_stream(self.dev)
+            with torch.cuda.device(self.dev):
+                sides = [torch.cuda.Stream(self.dev) for _ in self._bins[1:]]
+                fork = torch.cuda.Event()
+                fork.record(main)
+                for s_ in sides:
+                    s_.wait_event(fork)
+                try:
+                    self._launch_bins(seg, [main] + sides)
+                finally:
+                    for s_ in sides:
+                        main.wait_stream(s_)
+            return self
+        return self._launch_bins(seg, bin_streams if bin_streams else [stream])
+
+    def _launch_bins(self, seg, streams):
         L = lib()
         for i, bin_ in enumerate(self._bins):
-            st = bin_streams[i % len(bin_streams)] if bin_streams else stream
+            st = streams[i % len(streams)]
             b = self._struct(bin_, seg)
             if self._counters is not None:
                 ctr = self._counters[i:i + 1]
@@ -691,10 +811,13 @@ class Batch:
         return self._results()
 
     def _results(self):
-        eo = self.electrode_occupation.cpu().numpy()
-        occ = self.occupation.cpu().numpy()
-        out = dict(time=self.time.cpu().numpy(), status=self.status.cpu().numpy(),
-                   hops_done=self.hops_done.cpu().numpy(), n_pairs=self.n_pairs.cpu().numpy())
+        st = self._state
+        if all(getattr(self, k) is v for k, v in st.items()):
+            r = self._pack.download("occupation", "status")
+        else:                     # the caller has put tensors of its own in place
+            r = {k: getattr(self, k).cpu().numpy() for k in st}
+        eo, occ = r["electrode_occupation"], r["occupation"]
+        out = {k: r[k] for k in ("time", "status", "hops_done", "n_pairs")}
         out["electrode_occupation"] = [eo[o:o + p] for o, p in zip(self.el_off, self.P_c)]
         out["occupation"] = [occ[o:o + n].astype(bool) for o, n in zip(self.site_off, self.N_c)]
         if self.select_mismatch is not None:
@@ -735,12 +858,14 @@ def superpose(basis, comp, voltages, mu=0.0, dev=None, stream=None):
     V = np.asarray(voltages, np.float64)
     C_, P = V.shape
     N = basis.shape[1]
-    b = _dev(basis, torch.float64, d)
-    v = _dev(V, torch.float64, d)
-    cp = _dev(np.asarray(comp, np.float64), torch.float64, d)
+    pk = _Pack()
+    pk.add("basis", basis, torch.float64)
+    pk.add("V", V, torch.float64)
+    pk.add("comp", np.asarray(comp, np.float64), torch.float64)
+    t = pk.upload(d)
     ec = torch.empty(max(C_ * N, 1), dtype=torch.float32, device=d)
     ve = torch.empty(max(C_ * P, 1), dtype=torch.float32, device=d)
-    check(lib().kmc_site_energies(C_, N, P, _ptr(b), _ptr(v), float(mu), _ptr(cp), _ptr(ec), _ptr(ve),
+    check(lib().kmc_site_energies(C_, N, P, _ptr(t["basis"]), _ptr(t["V"]), float(mu), _ptr(t["comp"]), _ptr(ec), _ptr(ve),
                                   _stream_handle(stream)))
     return ec, ve
 

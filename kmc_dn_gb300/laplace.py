@@ -88,7 +88,7 @@ class BasisFields:
         """Basis values at points: array (n_basis, n_points).  P1 interpolation
         on the reference's triangulation."""
         pts = np.asarray(points, dtype=np.float64)
-        return np.stack([interpolate_p1(f, self, pts) for f in self.fields])
+        return interpolate_p1(self.fields, self, pts)
 
 
 def solve_basis_fields(xdim, ydim, electrodes, nx, ny=None, surplus=None):
@@ -174,7 +174,8 @@ def solve_basis_fields(xdim, ydim, electrodes, nx, ny=None, surplus=None):
 
 
 def interpolate_p1(field, basis: BasisFields, pts, diagonal="right"):
-    """Evaluate the piecewise-linear interpolant of nodal ``field`` at points.
+    """Evaluate the piecewise-linear interpolant of nodal ``field`` (or of a
+    stack of fields, one row each) at points.
 
     2D: cell (ix, iy) is split along the diagonal from (ix, iy) to
     (ix+1, iy+1) ("right", the mesh generator's default) or from (ix+1, iy)
@@ -186,16 +187,16 @@ def interpolate_p1(field, basis: BasisFields, pts, diagonal="right"):
         s = x / h
         ix = np.clip(np.floor(s).astype(np.int64), 0, basis.nx - 1)
         t = s - ix
-        return field[ix] * (1 - t) + field[ix + 1] * t
+        return field[..., ix] * (1 - t) + field[..., ix + 1] * t
     hx, hy = basis.xdim / basis.nx, basis.ydim / basis.ny
     sx, sy = pts[:, 0] / hx, pts[:, 1] / hy
     ix = np.clip(np.floor(sx).astype(np.int64), 0, basis.nx - 1)
     iy = np.clip(np.floor(sy).astype(np.int64), 0, basis.ny - 1)
     xi, eta = sx - ix, sy - iy
-    f00 = field[iy, ix]
-    f10 = field[iy, ix + 1]
-    f01 = field[iy + 1, ix]
-    f11 = field[iy + 1, ix + 1]
+    f00 = field[..., iy, ix]
+    f10 = field[..., iy, ix + 1]
+    f01 = field[..., iy + 1, ix]
+    f11 = field[..., iy + 1, ix + 1]
     if diagonal == "right":
         lower = xi >= eta
         v_lo = f00 + xi * (f10 - f00) + eta * (f11 - f10)

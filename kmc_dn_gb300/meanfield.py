@@ -17,6 +17,7 @@ import numpy as np
 
 from . import _native
 from ._native import KmcMfBatch, check, lib
+from .engine import _Pack
 
 __all__ = ["Network", "MeanFieldBatch", "run", "simulate_probability", "max_sites"]
 
@@ -31,10 +32,17 @@ class Network:
         self.N, self.P = int(N), int(P)
         self.nu, self.kT, self.I_0, self.R = float(nu), float(kT), float(I_0), float(R)
         S = self.N + self.P
-        self.distances = np.ascontiguousarray(distances, np.float64).reshape(S, S)
-        self.transitions_constant = np.ascontiguousarray(transitions_constant, np.float64).reshape(S, S)
-        self.E_constant = np.ascontiguousarray(E_constant, np.float64).reshape(self.N)
-        self.voltages = np.ascontiguousarray(voltages, np.float64).reshape(self.P)
+
+        def as_shape(a, shape):
+            # the caller's own array where it has the form: networks given the
+            # same arrays keep sharing them
+            a = np.ascontiguousarray(a, np.float64)
+            return a if a.shape == shape else a.reshape(shape)
+
+        self.distances = as_shape(distances, (S, S))
+        self.transitions_constant = as_shape(transitions_constant, (S, S))
+        self.E_constant = as_shape(E_constant, (self.N,))
+        self.voltages = as_shape(voltages, (self.P,))
 
 
 def max_sites(rates="f64"):
@@ -68,47 +76,53 @@ class MeanFieldBatch:
         blocks, seen, off = [], {}, 0
         for c, x in enumerate(nets):
             key = (id(x.distances), id(x.transitions_constant))
-            if key not in seen:
-                seen[key] = off
+            at = seen.get(key)
+            if at is None:
+                seen[key] = at = off
                 blocks.append((x.distances, x.transitions_constant))
                 off += x.distances.size
-            pair_off[c] = seen[key]
+            pair_off[c] = at
         self.site_off = np.concatenate([[0], np.cumsum(Ss)[:-1]]).astype(np.int64)
         self.el_off = np.concatenate([[0], np.cumsum(Ps.astype(np.int64))[:-1]]).astype(np.int64)
         self.tr_off = np.concatenate([[0], np.cumsum(Ss * Ss)[:-1]]).astype(np.int64)
         self.S = Ss
         n_sites = int(Ss.sum())
+        # site pools: acceptors, then electrodes, of each network
+        acceptor = np.arange(n_sites) - np.repeat(self.site_off, Ss) < np.repeat(Ns, Ss)
         ec = np.zeros(n_sites)
         se = np.zeros(n_sites)
+        ec[acceptor] = np.concatenate([x.E_constant for x in nets])
+        se[~acceptor] = np.concatenate([x.voltages for x in nets])
         occ = np.zeros(n_sites)
-        for c, x in enumerate(nets):
-            o = self.site_off[c]
-            ec[o:o + x.N] = x.E_constant
-            se[o + x.N:o + x.N + x.P] = x.voltages
-            occ[o:o + x.N] = start
+        if np.ndim(start) == 0:
+            occ[acceptor] = start
+        else:                     # a vector for every network
+            for o, x in zip(self.site_off, nets):
+                occ[o:o + x.N] = start
         self.dev = d = torch.device(dev if dev is not None else "cuda")
         f64, i64, i32 = torch.float64, torch.int64, torch.int32
-        T = lambda a, dt: torch.as_tensor(np.ascontiguousarray(a)).to(device=d, dtype=dt)  # noqa: E731
-        self.t = t = {}
-        t["N"], t["P"] = T(Ns, i32), T(Ps, i32)
-        for k in ("nu", "kT", "I_0", "R"):
-            t[k] = T([getattr(x, k) for x in nets], f64)
-        t["pair_off"] = T(pair_off, i64)
-        t["distances"] = T(np.concatenate([b[0].ravel() for b in blocks]), f64)
-        t["transitions_constant"] = T(np.concatenate([b[1].ravel() for b in blocks]), f64)
-        t["site_off"], t["E_constant"] = T(self.site_off, i64), T(ec, f64)
-        self._se0, self._occ0 = T(se, f64), T(occ, f64)
-        t["site_energies"], t["occupation"] = self._se0.clone(), self._occ0.clone()
-        t["el_off"] = T(self.el_off, i64)
-        t["electrode_occupation"] = torch.zeros(max(int(Ps.sum()), 1), dtype=f64, device=d)
-        t["hops"] = T(h, i64)
-        t["time"] = torch.zeros(n, dtype=f64, device=d)
-        t["status"] = torch.zeros(n, dtype=i32, device=d)
-        t["iterations_done"] = torch.zeros(n, dtype=i64, device=d)
+        pk = self._pack = _Pack()
+        for k, a, dt in (("N", Ns, i32), ("P", Ps, i32), *((k, [getattr(x, k) for x in nets], f64)
+                                                           for k in ("nu", "kT", "I_0", "R")),
+                         ("pair_off", pair_off, i64), ("distances", np.concatenate([b[0].ravel() for b in blocks]), f64),
+                         ("transitions_constant", np.concatenate([b[1].ravel() for b in blocks]), f64),
+                         ("site_off", self.site_off, i64), ("E_constant", ec, f64), ("el_off", self.el_off, i64),
+                         ("hops", h, i64), ("traffic_off", self.tr_off, i64), ("se0", se, f64), ("occ0", occ, f64),
+                         # results from here on
+                         ("site_energies", se, f64), ("occupation", occ, f64)):
+            pk.add(k, a, dt)
+        pk.zeros("electrode_occupation", max(int(Ps.sum()), 1), f64)
+        pk.zeros("time", n, f64)
+        pk.zeros("iterations_done", n, i64)
+        pk.zeros("status", n, i32)
         if record:
-            t["traffic_off"] = T(self.tr_off, i64)
-            t["traffic"] = torch.zeros(int((Ss * Ss).sum()), dtype=f64, device=d)
-            t["average_occupation"] = torch.zeros(n_sites, dtype=f64, device=d)
+            pk.zeros("average_occupation", n_sites, f64)
+            pk.zeros("traffic", int((Ss * Ss).sum()), f64)
+        self.t = t = pk.upload(d)
+        self._se0, self._occ0 = t.pop("se0"), t.pop("occ0")
+        if not record:
+            t.pop("traffic_off")
+        self._last = "traffic" if record else "status"
         b = KmcMfBatch()
         b.n_chains, b.max_sites, b.rates, b.record = n, int(Ss.max()), self.mode, int(self.record)
         for name, _ in KmcMfBatch._fields_[4:]:
@@ -135,20 +149,17 @@ class MeanFieldBatch:
     def results(self):
         import torch
         torch.cuda.synchronize(self.dev)
-        t, nets, n = self.t, self.nets, self.n
-        so, eo_off = self.site_off, self.el_off
-        occ_h, se_h = t["occupation"].cpu().numpy(), t["site_energies"].cpu().numpy()
-        eo_h = t["electrode_occupation"].cpu().numpy()
-        out = dict(time=t["time"].cpu().numpy(), status=t["status"].cpu().numpy(),
-                   iterations=t["iterations_done"].cpu().numpy(),
-                   occupation=[occ_h[so[c]:so[c] + nets[c].N].copy() for c in range(n)],
-                   site_energies=[se_h[so[c]:so[c] + nets[c].N].copy() for c in range(n)],
-                   electrode_occupation=[eo_h[eo_off[c]:eo_off[c] + nets[c].P].copy() for c in range(n)])
+        r = self._pack.download("site_energies", self._last)
+        nets, so, eo_off = self.nets, self.site_off, self.el_off
+        occ_h, se_h, eo_h = r["occupation"], r["site_energies"], r["electrode_occupation"]
+        out = dict(time=r["time"], status=r["status"], iterations=r["iterations_done"],
+                   occupation=[occ_h[o:o + x.N] for o, x in zip(so, nets)],
+                   site_energies=[se_h[o:o + x.N] for o, x in zip(so, nets)],
+                   electrode_occupation=[eo_h[o:o + x.P] for o, x in zip(eo_off, nets)])
         if self.record:
-            tr_h, avg_h = t["traffic"].cpu().numpy(), t["average_occupation"].cpu().numpy()
-            S, to = self.S, self.tr_off
-            out["traffic"] = [tr_h[to[c]:to[c] + S[c] ** 2].reshape(S[c], S[c]).copy() for c in range(n)]
-            out["average_occupation"] = [avg_h[so[c]:so[c] + nets[c].N].copy() for c in range(n)]
+            tr_h, avg_h = r["traffic"], r["average_occupation"]
+            out["traffic"] = [tr_h[o:o + s * s].reshape(s, s) for o, s in zip(self.tr_off, self.S)]
+            out["average_occupation"] = [avg_h[o:o + x.N] for o, x in zip(so, nets)]
         return out
 
 

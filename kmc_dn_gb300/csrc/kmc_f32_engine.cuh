@@ -354,6 +354,7 @@ __device__ __forceinline__ void decode_pair(int k, int h, int A1, int T1, int T2
 template <bool kStaged, bool kUniform = false>
 struct TablePairs {
     using Rec = int2;
+    static constexpr bool kFarTable = !kStaged;   // Coulomb terms come from L2
     static constexpr bool kSiteInRec = true;    // rec.x is the site id
     static constexpr bool kUniformTable = kUniform;
     static constexpr bool kPairedTgt = false;
@@ -391,6 +392,7 @@ struct TablePairs {
 // Positions mode: records are {x, y, z, scaled energy}; d from coordinates.
 struct PositionPairs {
     using Rec = float4;
+    static constexpr bool kFarTable = false;
     static constexpr bool kSiteInRec = false;   // site ids kept beside the records
     static constexpr bool kUniformTable = false;
     static constexpr bool kPairedTgt = false;
@@ -937,6 +939,86 @@ __device__ __forceinline__ ChainSmem<Rec> carve(uint32_t *base, int S, int rate_
     return c;
 }
 
+// Applies a hop to the energies and lists of the acceptors in one pass: the
+// O(N) update (makeJump, simulation.go:107-130; kComp: compensated), then the
+// record to its place in the ordered source or target list.  The occupancy
+// bits are those before the hop.  R sites of a thread a step, both Coulomb
+// terms of each read before its energy is touched and nothing stored before
+// the last of them (no load moves across a store).  That pays where the terms
+// come from L2 (a search population of 384 networks: 1853 to 1266 cycles a
+// hop, 33.1 to 32.3 ms).  From shared memory or positions a hop is bound by
+// its instructions, and R = 4 costs more than it hides (512 N=240 chains 36.5
+// against 37.8 ms, 4096 N=30 chains 31.6 against 32.4): R = 1 there, where
+// the order of the reads alone took one N=30 chain from 2.46 to 2.38 ms and
+// one N=100 chain from 22.3 to 21.8.
+template <int G, int R, bool kComp, typename Pairs>
+__device__ __forceinline__ int rebuild_sites(const Pairs &pairs, const ChainSmem<typename Pairs::Rec> &sm, int g, int N,
+                                             float cs, int from, int to, int h_new)
+{
+    // (a plain add of a computed term is one fused multiply-add, so positions
+    // without compensation form it in place)
+    constexpr bool kFirst = kComp || Pairs::kFarTable;
+    const bool fa = from < N, tb = to < N;
+    int wcur = 0, cum = 0, bad = 0;
+    for (int j0 = g; j0 < N; j0 += R * G) {
+        float E[R], lo[R], cf[R], ct[R];
+        uint32_t word[R];
+        int below[R];
+        typename Pairs::Rec r[R];
+#pragma unroll
+        for (int u = 0; u < R; ++u) {
+            const int j = R > 1 ? min(j0 + u * G, N - 1) : j0;   // past the end: the last site again, not stored
+            E[u] = sm.E[j];
+            lo[u] = kComp ? sm.Elo[j] : 0.0f;
+            if constexpr (kFirst) {
+                cf[u] = fa ? pairs.coulomb(j, from) : 0.0f;
+                ct[u] = tb ? pairs.coulomb(j, to) : 0.0f;
+            }
+            const int w = j >> 5;
+            while (wcur < w) { cum += __popc(sm.occw[wcur]); ++wcur; }
+            word[u] = sm.occw[w];
+            below[u] = cum;
+        }
+#pragma unroll
+        for (int u = 0; u < R; ++u) {
+            const int j = R > 1 ? min(j0 + u * G, N - 1) : j0;
+            if constexpr (kComp) {
+                if (fa && j != from) comp_add(E[u], lo[u], -cf[u]);
+                if (tb && j != to) comp_add(E[u], lo[u], ct[u]);
+                r[u] = pairs.rec(j, cs * (E[u] + lo[u]));
+            } else {
+                if (fa && j != from) E[u] -= kFirst ? cf[u] : pairs.coulomb(j, from);
+                if (tb && j != to) E[u] += kFirst ? ct[u] : pairs.coulomb(j, to);
+                r[u] = pairs.rec(j, cs * E[u]);
+            }
+            // holes below j after the hop
+            below[u] += __popc(word[u] & ((1u << (j & 31)) - 1u)) - ((fa && from < j) ? 1 : 0) + ((tb && to < j) ? 1 : 0);
+        }
+#pragma unroll
+        for (int u = 0; u < R; ++u) {
+            const int j = j0 + u * G;
+            if (R > 1 && j >= N) break;
+            sm.E[j] = E[u];
+            if constexpr (kComp) sm.Elo[j] = lo[u];
+            const bool occ_j = (j == to && tb) || (j != from && ((word[u] >> (j & 31)) & 1u));
+#ifdef KMC_DEBUG_CHECKS
+            if (occ_j ? !(below[u] >= 0 && below[u] < h_new) : !(j - below[u] >= 0 && j - below[u] < N - h_new)) {
+                bad = 1;        // skip the store: the chain stops after this hop
+                continue;
+            }
+#endif
+            if (occ_j) {
+                sm.src[below[u]] = r[u];
+                if (!Pairs::kSiteInRec) sm.src_id[below[u]] = j;
+            } else {
+                tgt_store<Pairs>(sm.tgt, j - below[u], r[u]);
+                if (!Pairs::kSiteInRec) sm.tgt_id[j - below[u]] = j;
+            }
+        }
+    }
+    return bad;
+}
+
 // ---------------------------------------------------------------------------
 // The hop loop of one chain, run by one block
 // ---------------------------------------------------------------------------
@@ -1379,36 +1461,10 @@ __device__ void run_chain(const kmc_batch &B, const Grp &grp, ChainSmem<typename
         const int h_new = h + (tb ? 1 : 0) - (fa ? 1 : 0);
         const int z_new = N - h_new;
         {
-            int wcur = 0, cum = 0;
-            for (int j = g; j < N; j += G) {
-                // O(N) update (makeJump, simulation.go:107-130), compensated
-                float Ej = sm.E[j], Elo = sm.Elo[j];
-                if (fa && j != from) comp_add(Ej, Elo, -pairs.coulomb(j, from));
-                if (tb && j != to) comp_add(Ej, Elo, pairs.coulomb(j, to));
-                sm.E[j] = Ej;
-                sm.Elo[j] = Elo;
-                const int w = j >> 5;
-                while (wcur < w) { cum += __popc(sm.occw[wcur]); ++wcur; }
-                const uint32_t word = sm.occw[w];
-                // holes below j and the bit of j after the hop
-                const int below = cum + __popc(word & ((1u << (j & 31)) - 1u))
-                                  - ((fa && from < j) ? 1 : 0) + ((tb && to < j) ? 1 : 0);
-                const bool occ_j = (j == to && tb) || (j != from && ((word >> (j & 31)) & 1u));
+            [[maybe_unused]] const int reb = rebuild_sites<G, 1, true>(pairs, sm, g, N, cs, from, to, h_new);
 #ifdef KMC_DEBUG_CHECKS
-                if (occ_j ? !(below >= 0 && below < h_new) : !(j - below >= 0 && j - below < z_new)) {
-                    dbg_bad = 1;        // skip the store: the chain stops after this hop
-                    continue;
-                }
+            dbg_bad |= reb;
 #endif
-                const Rec r = pairs.rec(j, cs * (Ej + Elo));
-                if (occ_j) {
-                    sm.src[below] = r;
-                    if (!Pairs::kSiteInRec) sm.src_id[below] = j;
-                } else {
-                    tgt_store<Pairs>(sm.tgt, j - below, r);
-                    if (!Pairs::kSiteInRec) sm.tgt_id[j - below] = j;
-                }
-            }
             if (h_new != h) {
                 for (int e = g; e < P; e += G) {
                     const Rec r = (e == g) ? el_rec : pairs.rec(N + e, cs * Vel[e]);

@@ -462,35 +462,16 @@ __device__ void run_warp(const kmc_batch &B, const Slice<G> &sl, ChainSmem<typen
             const int h_new = h + (tb ? 1 : 0) - (fa ? 1 : 0);
             const int z_new = N - h_new;
             if (run) {
-                int wcur = 0, cum = 0;
-                for (int j = g; j < N; j += G) {
-                    // O(N) update (makeJump, simulation.go:107-130)
-                    float Ej = sm.E[j];
-                    if (fa && j != from) Ej -= pairs.coulomb(j, from);
-                    if (tb && j != to) Ej += pairs.coulomb(j, to);
-                    sm.E[j] = Ej;
-                    const int w = j >> 5;
-                    while (wcur < w) { cum += __popc(sm.occw[wcur]); ++wcur; }
-                    const uint32_t word = sm.occw[w];
-                    // holes below j and the bit of j after the hop
-                    const int below = cum + __popc(word & ((1u << (j & 31)) - 1u))
-                                      - ((fa && from < j) ? 1 : 0) + ((tb && to < j) ? 1 : 0);
-                    const bool occ_j = (j == to && tb) || (j != from && ((word >> (j & 31)) & 1u));
+                // tables read from L2: as many sites a step as the slice has,
+                // up to four a lane (rebuild_sites)
+                constexpr int kTwo = Pairs::kFarTable ? 2 : 1, kFour = Pairs::kFarTable ? 4 : 1;
+                [[maybe_unused]] const int reb =
+                    kFour > 1 && N > 2 * G ? rebuild_sites<G, kFour, false>(pairs, sm, g, N, cs, from, to, h_new)
+                    : kTwo > 1 && N > G    ? rebuild_sites<G, kTwo, false>(pairs, sm, g, N, cs, from, to, h_new)
+                                           : rebuild_sites<G, 1, false>(pairs, sm, g, N, cs, from, to, h_new);
 #ifdef KMC_DEBUG_CHECKS
-                    if (occ_j ? !(below >= 0 && below < h_new) : !(j - below >= 0 && j - below < z_new)) {
-                        dbg_bad = 1;        // skip the store: the chain stops after this hop
-                        continue;
-                    }
+                dbg_bad |= reb;
 #endif
-                    const Rec r = pairs.rec(j, cs * Ej);
-                    if (occ_j) {
-                        sm.src[below] = r;
-                        if (!Pairs::kSiteInRec) sm.src_id[below] = j;
-                    } else {
-                        sm.tgt[j - below] = r;
-                        if (!Pairs::kSiteInRec) sm.tgt_id[j - below] = j;
-                    }
-                }
                 if (h_new != h) {
                     for (int e = g; e < P; e += G) {
                         const Rec r = (e == g) ? el_rec : pairs.rec(N + e, cs * Vel[e]);

@@ -1,6 +1,7 @@
 // kmc_f32.cu -- batched FP32 hop-loop engine for sm_103a: launch validation
-// and dispatch (the kernels are in kmc_f32_engine.cuh, instantiated by
-// kmc_f32_warp_table.cu, kmc_f32_warp_positions.cu and kmc_f32_block.cu).
+// and dispatch (the kernels are in kmc_f32_engine.cuh and kmc_f32_warp.cuh,
+// instantiated by kmc_f32_warp_table.cu, kmc_f32_warp_positions.cu and
+// kmc_f32_block.cu).
 //
 // A chain is run by a group of threads: a G-lane slice of a warp (G = 4, 8,
 // 16, 32; 32/G chains per warp) for small networks, or a whole thread block

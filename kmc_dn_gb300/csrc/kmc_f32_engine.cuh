@@ -107,19 +107,17 @@ inline int section_clocks_read(uint64_t *out, int reset)
 #define KMC_SECTION(k) do { } while (0)
 #endif
 
+// Pairs a step of a balanced walk (walk_pairs).
 #ifndef KMC_PAIR_STEP
 #define KMC_PAIR_STEP 4
 #endif
 constexpr int kPairStep = KMC_PAIR_STEP;
 
+// Unroll of the block groups' row walks, two pairs a step; N = 1000 networks
+// are insensitive to it.
 #ifndef KMC_PAIR_UNROLL
 #define KMC_PAIR_UNROLL 4
 #endif
-// Unroll of the pair walk (four steps = eight pairs in flight per thread):
-// on the N=30 ensemble 10 % faster than no unrolling and 5 % faster than two
-// steps; the large networks are insensitive to it.  Steps of four or eight
-// pairs with all their loads issued before the running-sum stores measured
-// 1-2.5 % slower than two-pair steps.
 constexpr int kPairUnroll = KMC_PAIR_UNROLL;
 
 // a compile-time bool as a type (selects a lambda's instantiation)

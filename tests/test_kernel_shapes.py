@@ -96,6 +96,23 @@ def test_rebuild_from_l2_equals_staged(engine_lib, lanes, N):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("lanes,N,P", [(64, 40, 2), (64, 60, 8), (64, 61, 7), (64, 90, 1), (64, 120, 8), (128, 150, 9),
+                                       (64, 200, 5)])
+def test_runs_of_rows_in_part_replay(engine_lib, oracle_mod, lanes, N, P):
+    """Positions, block groups, balanced runs of at least a row.  The oracle's hops on a stream that keeps 1e-4 of the
+    total rate away from every boundary (the FP32 cumulative sums are within
+    2e-5 of it); odd rows, odd starts, few electrodes."""
+    n, hops = _net(N, P, seed=4), 400
+    occ = n.occupation.astype(np.uint8)
+    net = (n.N, n.P, n.nu, n.kT, n.I_0, n.R, occ, n.distances, n.E_constant(), n.site_energies(), n.transitions_constant)
+    u, _ = oracle_mod.clear_stream(*net, hops, 9)
+    o = oracle_mod.numba_replay(*net, u)
+    r = _batch([n], [hops], lanes=lanes, pair_mode="positions", replay=[u], hop_log=True).run().results()
+    np.testing.assert_array_equal(r["hop_log"][0], o["hop_log"])
+    assert abs(r["time"][0] - o["time"]) <= 1e-4 * o["time"]
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("mode,lanes,N", [("table", 4, 120), ("table", 4, 80), ("positions", 4, 80), ("table", 32, 120),
                                           ("positions", 32, 120), ("table", 4, 10), ("positions", 16, 30)])
 def test_slices_of_a_warp_end_alone(engine_lib, mode, lanes, N):

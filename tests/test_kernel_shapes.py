@@ -127,6 +127,23 @@ def test_slices_of_a_warp_end_alone(engine_lib, mode, lanes, N):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("mode", ["table", "positions"])
+@pytest.mark.parametrize("lanes,N", [(64, 200), (64, 203), (128, 240)])
+def test_block_search_without_stored_sums(engine_lib, lanes, N, mode):
+    """A launch of more chains than fit beside their running sums drops these
+    and re-evaluates the chosen run; alone a chain keeps them.  The two search
+    the same rates in sums that associate differently (1e-7 of a run), so the
+    hops of a few short chains are the same."""
+    import torch
+    n, count = _net(N, 7), 5 * torch.cuda.get_device_properties(0).multi_processor_count
+    many = _batch([n], [60] * count, chain_table=[0] * count, lanes=lanes, pair_mode=mode, hop_log=True).run().results()
+    assert not np.any(many["status"])
+    for k in (0, 1, count // 2, count - 1):
+        alone = _batch([n], [60], chain_table=[0], streams=[k], lanes=lanes, pair_mode=mode, hop_log=True).run().results()
+        np.testing.assert_array_equal(many["hop_log"][k], alone["hop_log"][0])
+
+
+@pytest.mark.gpu
 def test_bins_side_by_side(engine_lib):
     """Size bins on streams of their own give what they give one after the
     other, and budgets changed after construction are kept to."""

@@ -219,6 +219,7 @@ __device__ void run_warp(const kmc_batch &B, const Slice<G> &sl, ChainSmem<typen
         }
         const bool anchor = run && until_anchor == 0;
         if (__any_sync(kAll, anchor)) {
+            __syncwarp();      // the last hop's bits are visible: a vote orders no memory
             anchor_and_build(anchor, B.energy_drift != nullptr);
             if (anchor) until_anchor = reanchor;
         }

@@ -965,7 +965,9 @@ __device__ __forceinline__ int rebuild_sites(const Pairs &pairs, const ChainSmem
         typename Pairs::Rec r[R];
 #pragma unroll
         for (int u = 0; u < R; ++u) {
-            const int j = R > 1 ? min(j0 + u * G, N - 1) : j0;   // past the end: the last site again, not stored
+            // past the end: the step's first site again, not stored (another
+            // thread's site would be read while that thread writes it)
+            const int j = R > 1 && j0 + u * G < N ? j0 + u * G : j0;
             E[u] = sm.E[j];
             lo[u] = kComp ? sm.Elo[j] : 0.0f;
             if constexpr (kFirst) {
@@ -979,7 +981,7 @@ __device__ __forceinline__ int rebuild_sites(const Pairs &pairs, const ChainSmem
         }
 #pragma unroll
         for (int u = 0; u < R; ++u) {
-            const int j = R > 1 ? min(j0 + u * G, N - 1) : j0;
+            const int j = R > 1 && j0 + u * G < N ? j0 + u * G : j0;
             if constexpr (kComp) {
                 if (fa && j != from) comp_add(E[u], lo[u], -cf[u]);
                 if (tb && j != to) comp_add(E[u], lo[u], ct[u]);

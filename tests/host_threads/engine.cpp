@@ -135,6 +135,8 @@ int main(int, char **argv)
     case 2: return launch<64, Far>(40, 6, 5, 30, 1, true, true, true);
     case 3: return launch<64, PairedPositionPairs>(90, 6, 9, 20, 1, true, false, false);
     case 4: return launch<256, PairedPositionPairs>(70, 6, 5, 10, 1, true, true, false);
+    case 5: return launch<16, Far>(40, 4, 5, 40, 2, true, true, true);
+    case 6: return launch<32, Far>(40, 4, 9, 40, 1, false, true, true);
     }
     return 2;
 }

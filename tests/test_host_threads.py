@@ -16,7 +16,8 @@ CSRC = os.path.join(REPO, "kmc_dn_gb300", "csrc")
 HOST = {"ex2.approx": "y = exp2f(x);", "rcp.approx": "y = 1.0f / x;", "rsqrt.approx": "y = 1.0f / sqrtf(x);",
         "globaltimer": "t = 0;"}
 LAUNCHES = ["slices of 4, one temperature", "slices of 8, positions, recorded", "block of 64, recorded",
-            "block of 64, positions, no stored sums", "block of 256, positions"]
+            "block of 64, positions, no stored sums", "block of 256, positions",
+            "slices of 16, sites four a step, recorded", "whole warp, sites two a step"]
 
 
 def _cuda_include():

@@ -633,19 +633,8 @@ class Batch:
         pk.zeros("hops_done", n, i64)
         pk.zeros("n_pairs", n, i64)
         pk.zeros("status", n, i32)
-        dv = pk.upload(d)
-        self.E_constant = E_constant_dev if E_constant_dev is not None else dv["E_constant"]
-        self.el_energy = el_energy_dev if el_energy_dev is not None else dv["el_energy"]
-        self.occupation, self.chain_tab_d, self.kT = dv["occupation"], dv["chain_tab"], dv["kT"]
-        self.site_off_d, self.el_off_d, self.pair_off_d = dv["site_off"], dv["el_off"], dv["pair_off"]
-        self.electrode_occupation, self.time, self.hops_done = dv["electrode_occupation"], dv["time"], dv["hops_done"]
-        self.hops_total, self.stream_ids = dv["hops_total"], dv["streams"]
-        self.status, self.n_pairs = dv["status"], dv["n_pairs"]
-        # the largest budget, while nobody has written to the tensor since
-        self._budget = (int(hops_c.max()) if n else 1, self.hops_total, _version(self.hops_total))
-        self._state = {k: dv[k] for k in ("occupation", "electrode_occupation", "time", "hops_done", "n_pairs", "status")}
-        self._bins = [dict(G=G, n_work=len(work) // max(1, 32 // G), work=dv[f"work{k}"], max_sites=smax, chains=order)
-                      for k, (G, work, order, smax) in enumerate(bins)]
+        # The optional state is filled before the pack goes over: that copy waits
+        # for the stream, so the batch is complete for launches on any stream.
         if self.record:
             self.occ_time = torch.zeros(max(nsite, 1), dtype=torch.float64, device=d)
             self.occ_since = torch.zeros(max(nsite, 1), dtype=torch.float64, device=d)
@@ -684,8 +673,21 @@ class Batch:
         self.time_budget_ns = 0       # per launch and chain; 0: none
         # persistent launches: one work counter per bin, zeroed before each launch
         self.persistent = bool(persistent)
-        self._counters = (torch.zeros(max(len(self._bins), 1), dtype=torch.int32, device=d)
+        self._counters = (torch.zeros(max(len(bins), 1), dtype=torch.int32, device=d)
                           if self.persistent else None)
+        dv = pk.upload(d)
+        self.E_constant = E_constant_dev if E_constant_dev is not None else dv["E_constant"]
+        self.el_energy = el_energy_dev if el_energy_dev is not None else dv["el_energy"]
+        self.occupation, self.chain_tab_d, self.kT = dv["occupation"], dv["chain_tab"], dv["kT"]
+        self.site_off_d, self.el_off_d, self.pair_off_d = dv["site_off"], dv["el_off"], dv["pair_off"]
+        self.electrode_occupation, self.time, self.hops_done = dv["electrode_occupation"], dv["time"], dv["hops_done"]
+        self.hops_total, self.stream_ids = dv["hops_total"], dv["streams"]
+        self.status, self.n_pairs = dv["status"], dv["n_pairs"]
+        # the largest budget, while nobody has written to the tensor since
+        self._budget = (int(hops_c.max()) if n else 1, self.hops_total, _version(self.hops_total))
+        self._state = {k: dv[k] for k in ("occupation", "electrode_occupation", "time", "hops_done", "n_pairs", "status")}
+        self._bins = [dict(G=G, n_work=len(work) // max(1, 32 // G), work=dv[f"work{k}"], max_sites=smax, chains=order)
+                      for k, (G, work, order, smax) in enumerate(bins)]
 
     def _warps(self, G, n_work=None):
         w = self.warps_per_block

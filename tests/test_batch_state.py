@@ -1,0 +1,76 @@
+"""A batch's device state: complete when the constructor returns, and read as
+it is when a launch starts."""
+import types
+
+import numpy as np
+import pytest
+import torch
+
+from kmc_dn_gb300 import _native, engine, workloads
+
+
+def _positions_spec(N, P, seed=0):
+    L = float(np.sqrt(N / workloads.DENSITY))
+    rng = np.random.Generator(np.random.PCG64(seed))
+    return workloads.make_network(rng, N, N // 10, L, L, workloads.perimeter_electrodes(L, P),
+                                  voltages=rng.uniform(-1, 1, P), cells=30)
+
+
+def _make(net, hops, tables, **kw):
+    n = len(hops)
+    return engine.Batch(tables, [0] * n, [net.kT] * n, [net.E_constant()] * n, [net.electrodes[:, 3]] * n,
+                        [net.occupation.astype(np.uint8)] * n, hops, seed=3, **kw)
+
+
+EVERYTHING = dict(record=_native.RECORD_GO, hop_log=True, hop_rates=True, count_select_mismatch=True,
+                  measure_drift=True, persistent=True, flux=True)
+
+
+def test_fills_come_before_the_blocking_copy(monkeypatch):
+    """Every fill of optional state is queued before the one copy that waits
+    for the stream (here: plain tensors, calls in order)."""
+    monkeypatch.setattr(engine, "device", lambda dev=None: torch.device("cpu"))
+    monkeypatch.setattr(torch.cuda, "get_device_properties", lambda d: types.SimpleNamespace(multi_processor_count=152))
+    net = _positions_spec(12, 4)
+    tables = engine.TableSet([engine.TableSpec.from_network(net)], pair_mode="positions")
+    calls = []
+
+    def logged(owner, name):
+        f = getattr(owner, name)
+        monkeypatch.setattr(owner, name, lambda *a, **k: (calls.append(name), f(*a, **k))[1])
+
+    for owner, name in ((torch, "zeros"), (torch, "full"), (torch, "ones"), (engine._Pack, "upload")):
+        logged(owner, name)
+    u = np.full(40, 0.5)
+    b = _make(net, [20, 20], tables, replay=[u, u], **EVERYTHING)
+    assert calls.count("zeros") >= 8 and "full" in calls
+    assert calls[-1] == "upload" and calls.count("upload") == 1
+    assert torch.all(b.hop_log == -1) and not b.traffic.any() and not b.flux_time.any()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("lanes", [8, 32, 64])
+def test_batch_built_on_one_stream_runs_on_another(engine_lib, lanes, monkeypatch):
+    """With work queued on the constructing stream behind the upload, a launch
+    on a stream of its own keeps what it records."""
+    net, hops = _positions_spec(24, 5, seed=1), [300, 200]
+    tables = engine.TableSet([engine.TableSpec.from_network(net)])
+    want = _make(net, hops, tables, lanes=lanes, **EVERYTHING).run().results()
+    upload = engine._Pack.upload
+
+    def slow(self, dev):
+        t = upload(self, dev)
+        torch.cuda._sleep(40_000_000)       # 20 ms on the current stream
+        return t
+
+    monkeypatch.setattr(engine._Pack, "upload", slow)
+    build, other = torch.cuda.Stream(), torch.cuda.Stream()
+    with torch.cuda.stream(build):
+        b = _make(net, hops, tables, lanes=lanes, **EVERYTHING)
+    b.launch(stream=other)
+    got = b.results()
+    for k in ("time", "hops_done", "n_pairs", "status", "energy_drift"):
+        np.testing.assert_array_equal(got[k], want[k], err_msg=k)
+    for k in ("occupation", "electrode_occupation", "traffic", "occ_time", "flux_time", "hop_log", "hop_rates"):
+        for c in range(2):
+            np.testing.assert_array_equal(got[k][c], want[k][c], err_msg=k)

@@ -64,14 +64,6 @@ def _dev(a, dtype, dev):
     return torch.as_tensor(np.require(a, requirements=("C", "W")), dtype=dtype).to(dev)
 
 
-def _version(t):
-    """A tensor's count of in-place writes; None where it has none (inference mode)."""
-    try:
-        return t._version
-    except RuntimeError:
-        return None
-
-
 class _Pack:
     """Arrays of one launch in one device buffer: the inputs go over in one
     copy, the zeroed state behind them is one fill, and a run of neighbouring
@@ -683,8 +675,6 @@ class Batch:
         self.electrode_occupation, self.time, self.hops_done = dv["electrode_occupation"], dv["time"], dv["hops_done"]
         self.hops_total, self.stream_ids = dv["hops_total"], dv["streams"]
         self.status, self.n_pairs = dv["status"], dv["n_pairs"]
-        # the largest budget, while nobody has written to the tensor since
-        self._budget = (int(hops_c.max()) if n else 1, self.hops_total, _version(self.hops_total))
         self._state = {k: dv[k] for k in ("occupation", "electrode_occupation", "time", "hops_done", "n_pairs", "status")}
         self._bins = [dict(G=G, n_work=len(work) // max(1, 32 // G), work=dv[f"work{k}"], max_sites=smax, chains=order)
                       for k, (G, work, order, smax) in enumerate(bins)]
@@ -760,13 +750,9 @@ class Batch:
         bins run side by side: the first on `stream` (default: the current
         one), the others on streams forked from it and joined back to it, or
         all round-robin on `bin_streams` (the caller synchronises)."""
-        seg = max_hops_per_launch
-        if seg is None:
-            top, tensor, version = self._budget
-            if self.hops_total is not tensor or version is None or _version(tensor) != version:
-                top = int(self.hops_total.max().item()) if self.n else 1
-            seg = top
-        seg = max(self.reanchor, ((int(seg) + self.reanchor - 1) // self.reanchor) * self.reanchor)
+        # (None: every chain to the end of its budget, which the kernels read)
+        seg = 2**62 if max_hops_per_launch is None else int(max_hops_per_launch)
+        seg = max(self.reanchor, ((seg + self.reanchor - 1) // self.reanchor) * self.reanchor)
         if len(self._bins) > 1 and not bin_streams:
             main = stream if stream is not None else torch.cuda.current_stream(self.dev)
             with torch.cuda.device(self.dev):

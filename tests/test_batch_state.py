@@ -22,6 +22,12 @@ def _make(net, hops, tables, **kw):
                         [net.occupation.astype(np.uint8)] * n, hops, seed=3, **kw)
 
 
+def _on_cpu(monkeypatch):
+    """Batches of plain CPU tensors (nothing can be launched)."""
+    monkeypatch.setattr(engine, "device", lambda dev=None: torch.device("cpu"))
+    monkeypatch.setattr(torch.cuda, "get_device_properties", lambda d: types.SimpleNamespace(multi_processor_count=152))
+
+
 EVERYTHING = dict(record=_native.RECORD_GO, hop_log=True, hop_rates=True, count_select_mismatch=True,
                   measure_drift=True, persistent=True, flux=True)
 
@@ -29,8 +35,7 @@ EVERYTHING = dict(record=_native.RECORD_GO, hop_log=True, hop_rates=True, count_
 def test_fills_come_before_the_blocking_copy(monkeypatch):
     """Every fill of optional state is queued before the one copy that waits
     for the stream (here: plain tensors, calls in order)."""
-    monkeypatch.setattr(engine, "device", lambda dev=None: torch.device("cpu"))
-    monkeypatch.setattr(torch.cuda, "get_device_properties", lambda d: types.SimpleNamespace(multi_processor_count=152))
+    _on_cpu(monkeypatch)
     net = _positions_spec(12, 4)
     tables = engine.TableSet([engine.TableSpec.from_network(net)], pair_mode="positions")
     calls = []
@@ -46,6 +51,37 @@ def test_fills_come_before_the_blocking_copy(monkeypatch):
     assert calls.count("zeros") >= 8 and "full" in calls
     assert calls[-1] == "upload" and calls.count("upload") == 1
     assert torch.all(b.hop_log == -1) and not b.traffic.any() and not b.flux_time.any()
+
+
+def test_launch_covers_budgets_as_they_are(monkeypatch):
+    """Budgets written after construction count, also by a writer that torch
+    does not see (a kernel, another library, the tensor's .data)."""
+    _on_cpu(monkeypatch)
+    net = _positions_spec(12, 4)
+    tables = engine.TableSet([engine.TableSpec.from_network(net)], pair_mode="positions")
+    for reanchor in (1024, 700):
+        b = _make(net, [20, 30], tables, reanchor=reanchor)
+        segs = []
+        monkeypatch.setattr(b, "_launch_bins", lambda seg, streams: segs.append(b._struct(b._bins[0], seg)))
+        for write in (lambda: None, lambda: b.hops_total.data.fill_(10**6), lambda: b.hops_total.numpy().fill(10**7)):
+            write()
+            b.launch()
+            assert segs[-1].max_hops_per_launch >= b.hops_total.max()
+            assert segs[-1].max_hops_per_launch % reanchor == 0
+        b.launch(5000)
+        assert segs[-1].max_hops_per_launch == -(-5000 // reanchor) * reanchor
+
+
+@pytest.mark.gpu
+def test_budgets_raised_in_place_are_run(engine_lib):
+    net = _positions_spec(24, 5, seed=1)
+    tables = engine.TableSet([engine.TableSpec.from_network(net)])
+    want = _make(net, [3000, 1500], tables).run().results()
+    b = _make(net, [40, 20], tables)
+    b.hops_total.data.copy_(torch.tensor([3000, 1500]))
+    got = b.run().results()
+    assert got["hops_done"].tolist() == [3000, 1500] and not got["status"].any()
+    np.testing.assert_array_equal(got["time"], want["time"])
 
 
 @pytest.mark.gpu

@@ -149,25 +149,35 @@ int build_tables(int n, const int32_t *N, const int32_t *P, const double *nu, co
     // streams of their own took 8, the driver's part of the copies being
     // serial.  Reading the arrays in place over the coherent link took 4 once
     // their pages had been read a few times, but up to 16 the first time.)
+    // The FP64 tables pass through kTableStage bytes, or the largest one's,
+    // whatever their number: a launch a filling of it, in stream order.
+    constexpr size_t kTableStage = 64 << 20;
+    const size_t room = std::max(largest, std::min(pairs, kTableStage / 16));     // pairs
     char *buf = nullptr;
     const size_t head = (sizeof(TableSource) * n + 255) & ~static_cast<size_t>(255);
-    cudaError_t e = cudaMallocAsync(reinterpret_cast<void **>(&buf), head + 16 * pairs, st);
+    cudaError_t e = cudaMallocAsync(reinterpret_cast<void **>(&buf), head + 16 * room, st);
     if (e != cudaSuccess) return fail_cuda(e, "build_tables: device allocation");
-    double *at = reinterpret_cast<double *>(buf + head);
-    for (int t = 0; t < n && e == cudaSuccess; ++t) {
-        const size_t SS = static_cast<size_t>(N[t] + P[t]) * (N[t] + P[t]);
-        src[t] = TableSource{N[t], P[t], nu[t], I0[t] * R[t], at, at + SS, reinterpret_cast<float2 *>(tab + off[t])};
-        e = cudaMemcpyAsync(at, d[t], 8 * SS, cudaMemcpyHostToDevice, st);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(at + SS, tc[t], 8 * SS, cudaMemcpyHostToDevice, st);
-        at += 2 * SS;
-    }
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(buf, src.data(), sizeof(TableSource) * n, cudaMemcpyHostToDevice, st);
+    TableSource *dev = reinterpret_cast<TableSource *>(buf);
     const int bx = static_cast<int>(std::min<size_t>((largest + 255) / 256, 64));
-    for (int t0 = 0; t0 < n && e == cudaSuccess; t0 += 65535) {
-        build_tables_kernel<<<dim3(bx, std::min(n - t0, 65535)), 256, 0, st>>>(
-            reinterpret_cast<const TableSource *>(buf) + t0);
-        e = cudaGetLastError();
+    for (int t0 = 0, t1; t0 < n && e == cudaSuccess; t0 = t1) {
+        double *at = reinterpret_cast<double *>(buf + head);
+        size_t used = 0;
+        for (t1 = t0; t1 < n && t1 - t0 < 65535 && e == cudaSuccess; ++t1) {
+            const size_t SS = static_cast<size_t>(N[t1] + P[t1]) * (N[t1] + P[t1]);
+            if (used + SS > room) break;
+            used += SS;
+            src[t1] = TableSource{N[t1], P[t1], nu[t1], I0[t1] * R[t1], at, at + SS,
+                                  reinterpret_cast<float2 *>(tab + off[t1])};
+            e = cudaMemcpyAsync(at, d[t1], 8 * SS, cudaMemcpyHostToDevice, st);
+            if (e == cudaSuccess) e = cudaMemcpyAsync(at + SS, tc[t1], 8 * SS, cudaMemcpyHostToDevice, st);
+            at += 2 * SS;
+        }
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(dev + t0, &src[t0], sizeof(TableSource) * (t1 - t0), cudaMemcpyHostToDevice, st);
+        if (e == cudaSuccess) {
+            build_tables_kernel<<<dim3(bx, t1 - t0), 256, 0, st>>>(dev + t0);
+            e = cudaGetLastError();
+        }
     }
     const cudaError_t f = cudaFreeAsync(buf, st), w = cudaStreamSynchronize(st);
     if (e == cudaSuccess) e = f;

@@ -110,3 +110,31 @@ def test_batch_built_on_one_stream_runs_on_another(engine_lib, lanes, monkeypatc
     for k in ("occupation", "electrode_occupation", "traffic", "occ_time", "flux_time", "hop_log", "hop_rates"):
         for c in range(2):
             np.testing.assert_array_equal(got[k][c], want[k][c], err_msg=k)
+
+
+@pytest.mark.gpu
+def test_table_build_stages_a_bounded_part(engine_lib):
+    """The FP64 tables of a set pass through a staging buffer whose size does
+    not grow with their number (the high-water mark of the device's memory
+    pool), and each comes out as if it were built alone."""
+    import ctypes as C
+    cu = C.CDLL("libcuda.so.1")
+    pool, high, zero = C.c_void_p(), C.c_uint64(), C.c_uint64(0)
+    USED_MEM_HIGH = 8
+    S, n = 900, 16                              # 13 MB of FP64 tables a geometry, 207 MB in all
+    rng = np.random.default_rng(2)
+    N, P = S - 7, 7
+    d = [rng.uniform(0.1, 3.0, (S, S)) for _ in range(3)]
+    tc = [rng.uniform(0.0, 1.0, (S, S)) for _ in range(3)]
+    specs = [engine.TableSpec(N, P, 0.5 + k, 3.0, 0.25, d[k % 3], tc[(k + 1) % 3]) for k in range(n)]
+    specs.insert(5, engine.TableSpec(1, 2, 1.0, 1.0, 1.0, d[0][:3, :3], tc[0][:3, :3]))
+    engine.TableSet(specs[:1])
+    assert cu.cuDeviceGetDefaultMemPool(C.byref(pool), torch.cuda.current_device()) == 0
+    assert cu.cuMemPoolSetAttribute(pool, USED_MEM_HIGH, C.byref(zero)) == 0
+    ts = engine.TableSet(specs)
+    assert cu.cuMemPoolGetAttribute(pool, USED_MEM_HIGH, C.byref(high)) == 0
+    assert 16 * S * S <= high.value <= 70 << 20
+    off = ts.tab_off.cpu().numpy()
+    for k in (0, 4, 5, 6, 9, 16):
+        one = engine.TableSet(specs[k:k + 1]).tab_LB
+        assert torch.equal(ts.tab_LB[int(off[k]):int(off[k]) + one.numel()], one)

@@ -594,7 +594,7 @@ struct BlockScratch {
 // pairs (N = 30 alone: 23 barriers).  The hop loop therefore publishes the
 // per-thread sums once and lets every warp repeat the rest of the selection
 // by itself (select, and the search of one run's stored sums).
-template <int T>
+template <int T, bool kPerWarp = (T <= 128)>
 struct BlockGroup {
     static constexpr int kSize = T;
     static constexpr int kWarps = T / 32;
@@ -604,15 +604,17 @@ struct BlockGroup {
     BlockScratch<T> *sc;
 
     // The event's thread: exact fixed-point scan of the group's sums (see
-    // Selection).  Synchronises the block once (up to 128 threads: every warp
-    // reads all sums, T/32 a lane) or twice (each thread converts its own
-    // sum, which needs the largest one first).
+    // Selection).  Synchronises the block once (kPerWarp: every warp reads and
+    // converts all sums, T/32 a lane) or twice (each thread converts its own
+    // sum, which needs the largest one first: fewer instructions, which count
+    // where the SM is full of blocks).
     __device__ __forceinline__ Selection select(float lsum, uint64_t u_ev) const
     {
         constexpr int kShift = FixShift<T>::kShift;
         const int lane = g & 31;
         Selection r;
-        if constexpr (T <= 128) {
+        if constexpr (kPerWarp) {
+            static_assert(T <= 128, "a warp reads at most four sums a lane");
             constexpr int K = T / 32;
             float *s = reinterpret_cast<float *>(sc->sums);
             s[g] = lsum;
@@ -1547,18 +1549,23 @@ __device__ __forceinline__ const float2 *stage_table(const kmc_batch &B, uint32_
     return reinterpret_cast<const float2 *>(smem);
 }
 
-// Block kernel: one chain per block of T threads.  512 / T blocks an SM leave
-// 128 registers a thread; without the bound the compiler took 64 or 72 for
-// the positions kernels and spilled 150 to 390 bytes inside the hop loop.
-template <int T, typename Pairs>
-__global__ void __launch_bounds__(T, 512 / T) block_engine_kernel(const kmc_batch B, int rate_words,
-                                                         int table_words)
+// Block kernel: one chain per block of T threads, kBlocks of them an SM.
+// 512 / T blocks leave 128 registers a thread, which the pair walk uses: a
+// chain alone runs 1.1 to 2 times as fast as at 72 or 96 (one N = 120 chain of
+// 128 threads 2.0, N = 240 1.07).  But equal chains that need a second wave of
+// blocks for the last few take as long as two full waves (five N = 240 chains
+// of 128 threads an SM: 1.6 times the one wave), so leaner variants hold more
+// (launch_block_kernel chooses).
+template <int T, typename Pairs, int kBlocks>
+__global__ void __launch_bounds__(T, kBlocks) block_engine_kernel(const kmc_batch B, int rate_words, int table_words)
 {
     extern __shared__ __align__(16) uint32_t smem[];
     __shared__ BlockScratch<T> scratch;
     int *iscratch = scratch.si;
     const float2 *stab = stage_table(B, smem, table_words);
-    BlockGroup<T> grp;
+    // (a full SM of 128-thread blocks: 2 % faster with the fewer instructions)
+    using Grp = BlockGroup<T, (T == 64 || (T == 128 && kBlocks == 512 / T))>;
+    Grp grp;
     grp.init();
     grp.sd = scratch.sd;
     grp.si = scratch.si;
@@ -1575,14 +1582,14 @@ __global__ void __launch_bounds__(T, 512 / T) block_engine_kernel(const kmc_batc
             __syncthreads();
             if (item >= B.n_work) break;
             const int c = B.work[item];
-            if (c >= 0 && c < B.n_chains) run_chain<BlockGroup<T>, Pairs>(B, grp, sm, c, stab);
+            if (c >= 0 && c < B.n_chains) run_chain<Grp, Pairs>(B, grp, sm, c, stab);
             __syncthreads();
         }
         return;
     }
     const int c = B.work[blockIdx.x];
     if (c < 0 || c >= B.n_chains) return;   // uniform over the block
-    run_chain<BlockGroup<T>, Pairs>(B, grp, sm, c, stab);
+    run_chain<Grp, Pairs>(B, grp, sm, c, stab);
 }
 
 template <typename K>
@@ -1627,31 +1634,82 @@ int table_stage_words(const kmc_batch &b, size_t rest)
     return (w * 4 + rest <= kSmemBudget && w * 4 <= 64 * 1024) ? static_cast<int>(w) : 0;
 }
 
-template <int T, typename Pairs>
-int launch_block_kernel(const kmc_batch &b, cudaStream_t st, size_t smem, int rw, int tw)
+template <int T, typename Pairs, int kBlocks>
+int launch_block_variant(const kmc_batch &b, cudaStream_t st, size_t smem, int rw, int tw)
 {
     static int configured = 0;
-    const int rc = set_smem(block_engine_kernel<T, Pairs>, smem, configured);
+    auto *kernel = block_engine_kernel<T, Pairs, kBlocks>;
+    const int rc = set_smem(kernel, smem, configured);
     if (rc != KMC_OK) return rc;
     if (b.n_work <= 0) return KMC_OK;
     int grid = b.n_work;
     if (b.work_counter) {   // persistent: the resident blocks claim the chains
         int per_sm = 0;
-        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, block_engine_kernel<T, Pairs>, T, smem);
+        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, T, smem);
         if (e != cudaSuccess) return fail_cuda(e, "engine occupancy");
         grid = min(grid, max(1, per_sm) * sm_count());
         if (b.max_grid > 0) grid = min(grid, b.max_grid);
     }
-    block_engine_kernel<T, Pairs><<<grid, T, smem, st>>>(b, rw, tw);
+    kernel<<<grid, T, smem, st>>>(b, rw, tw);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? KMC_OK : fail_cuda(e, "engine launch");
+}
+
+// Blocks whose shared memory an SM holds, `bytes` of it dynamic.
+template <int T>
+int blocks_by_smem(size_t bytes)
+{
+    return max(1, static_cast<int>(228 * 1024 / (bytes + sizeof(BlockScratch<T>) + 1024)));
+}
+
+// Time of q equal blocks an SM, r at a time, in twentieths of a block's share
+// of a full SM: the same for every variant within 10 %, and a wave that is
+// not full takes no less than 17/20 of one of the 128-register kernel.
+inline int waves_cost(int q, int r, int rich)
+{
+    return 20 * (q / r * r) + (q % r ? max(20 * (q % r), 17 * rich) : 0);
+}
+
+// The variant for a launch of q blocks an SM.  64 and 128 threads: the one of
+// 96 registers (five chains of 128 threads an SM), or of 72 (seven) for tables
+// read from memory and no stored sums, where that shortens the waves; with
+// sums stored, seven chains leave the table reads too little L1 (N = 120, 128
+// threads, seven an SM: 3.6 ms, in two waves of four 2.0).  1024 chains of
+// N = 240, 128 threads, tables in memory: 6.6 ms, 8.3 with one variant.  512
+// threads: two chains of 64 registers an SM in positions mode (304 chains of
+// N = 240: 2.1 ms against 2.5 one at a time).
+template <int T, typename Pairs>
+int launch_block_kernel(const kmc_batch &b, cudaStream_t st, size_t smem, int rw, int tw)
+{
+    constexpr int kRich = 512 / T;
+    const int q = (b.n_work + sm_count() - 1) / sm_count(), fit = blocks_by_smem<T>(smem);
+    if constexpr (T == 512 && Pairs::kPairedTgt)
+        if (q > 1 && fit > 1) return launch_block_variant<T, Pairs, 2>(b, st, smem, rw, tw);
+    if constexpr (T <= 128) {
+        const bool most = Pairs::kFarTable && rw == 0;
+        const int rich = min(kRich, fit), lean = min((most ? 896 : 640) / T, fit);
+        if (waves_cost(q, lean, kRich) < waves_cost(q, rich, kRich)) {
+            if constexpr (Pairs::kFarTable)
+                if (most) return launch_block_variant<T, Pairs, 896 / T>(b, st, smem, rw, tw);
+            return launch_block_variant<T, Pairs, 640 / T>(b, st, smem, rw, tw);
+        }
+    }
+    return launch_block_variant<T, Pairs, kRich>(b, st, smem, rw, tw);
 }
 
 template <int T, typename Pairs>
 int preload_block_kernel()
 {
-    return touch_kernel(block_engine_kernel<T, Pairs>);
+    int rc = touch_kernel(block_engine_kernel<T, Pairs, 512 / T>);
+    if constexpr (T <= 128)
+        if (rc == KMC_OK) rc = touch_kernel(block_engine_kernel<T, Pairs, 640 / T>);
+    if constexpr (T <= 128 && Pairs::kFarTable)
+        if (rc == KMC_OK) rc = touch_kernel(block_engine_kernel<T, Pairs, 896 / T>);
+    if constexpr (T == 512 && Pairs::kPairedTgt)
+        if (rc == KMC_OK) rc = touch_kernel(block_engine_kernel<T, Pairs, 2>);
+    return rc;
 }
+
 // Words of the running-sum buffer of a block group's chain, or 0: the event
 // search then re-evaluates the chosen thread's run, for a block group a chunk
 // or two of rates.
@@ -1661,16 +1719,14 @@ int block_rate_words(const kmc_batch &b)
     const int lw = chain_list_words<typename Pairs::Rec>(b.max_sites);
     const int rw = rate_buffer_words(b.max_sites, T);
     if (static_cast<size_t>(lw + rw) * 4 > kSmemBudget) return 0;
-    // Drop the buffer when it is what limits the blocks an SM holds and the
-    // launch has more chains than the SMs then hold at once (a 512-chain
-    // request of N=240 networks at 512 threads: one wave of blocks instead
-    // of two).
-    const int per_sm_threads = 2048 / T;
-    const int per_sm_with = static_cast<int>((227 * 1024) / (static_cast<size_t>(lw + rw) * 4));
-    const int per_sm_without = static_cast<int>((227 * 1024) / (static_cast<size_t>(lw) * 4));
-    if (per_sm_with < per_sm_threads && per_sm_without > per_sm_with && b.n_work > per_sm_with * sm_count())
-        return 0;
-    return rw;
+    // Dropped for launches of more chains than the SMs hold with it, where
+    // that lets more blocks be resident (registers allow 640 / T of up to 128
+    // threads, 2 of more), or gives its place to the L1 for tables in memory (N = 240, 256 threads, 3 chains an SM: 2.2 ms, 2.4 with the
+    // buffer; in positions mode 1.9 with it, 2.0 without).
+    const int by_regs = Pairs::kFarTable ? 2048 / T : T <= 128 ? 640 / T : 2;
+    const int with = min(by_regs, blocks_by_smem<T>(4 * static_cast<size_t>(lw + rw)));
+    const int without = min(by_regs, blocks_by_smem<T>(4 * static_cast<size_t>(lw)));
+    return with < without && b.n_work > with * sm_count() ? 0 : rw;
 }
 
 template <int T, typename Pairs>

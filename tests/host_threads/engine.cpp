@@ -115,7 +115,7 @@ int launch(int N, int P, int reanchor, int hops, int chains, bool record, bool s
     for (int item = 0; item < B.n_work; ++item)
         run_block(kBlock ? G : 32, [&] {
             blockIdx.x = static_cast<unsigned>(item);
-            if constexpr (kBlock) block_engine_kernel<G, Pairs>(B, rate_words, table_words);
+            if constexpr (kBlock) block_engine_kernel<G, Pairs, 512 / G>(B, rate_words, table_words);
             else warp_engine_kernel<G, Pairs, 2>(B, rate_words, table_words);
         });
     for (int c = 0; c < chains; ++c)

@@ -79,7 +79,9 @@ struct Slice {
     }
 };
 
-template <int G, typename Pairs>
+// kLean: the 80-register kernel, whose list rebuild takes one site a step
+// (two or four spill).
+template <int G, typename Pairs, bool kLean>
 __device__ void run_warp(const kmc_batch &B, const Slice<G> &sl, ChainSmem<typename Pairs::Rec> sm, int c,
                          const float2 *shared_tab)
 {
@@ -465,7 +467,8 @@ __device__ void run_warp(const kmc_batch &B, const Slice<G> &sl, ChainSmem<typen
             if (run) {
                 // tables read from L2: as many sites a step as the slice has,
                 // up to four a lane (rebuild_sites)
-                constexpr int kTwo = Pairs::kFarTable ? 2 : 1, kFour = Pairs::kFarTable ? 4 : 1;
+                constexpr bool kMany = Pairs::kFarTable && !kLean;
+                constexpr int kTwo = kMany ? 2 : 1, kFour = kMany ? 4 : 1;
                 [[maybe_unused]] const int reb =
                     kFour > 1 && N > 2 * G ? rebuild_sites<G, kFour, false>(pairs, sm, g, N, cs, from, to, h_new)
                     : kTwo > 1 && N > G    ? rebuild_sites<G, kTwo, false>(pairs, sm, g, N, cs, from, to, h_new)
@@ -566,11 +569,11 @@ __device__ __forceinline__ const float2 *stage_table_uniform(const kmc_batch &B,
 
 
 // 32/G chains a warp, blockDim.x / 32 warps a block.  Two register budgets:
-// MinBlocks = 3 blocks of 256 threads keeps registers at or below 85 so that
-// 24 warps fit on an SM (launches with more blocks than the SMs hold at 2
-// each); MinBlocks = 2 allows 128 registers (16 warps per SM), which the pair
-// walk uses without spills: 5.6 % faster on 4096 N=30 chains, whose blocks
-// all fit.  table_words > 0: every chain of the launch uses table 0, staged
+// MinBlocks = 2 allows 128 registers (two blocks of 256 threads, 16 warps an
+// SM), which the pair walk uses without spills; MinBlocks = 3 allows 80 (24
+// warps an SM).  4096 N = 100 chains with tables in memory: 31.7 ms in two
+// waves at 128 registers, 51 in one and a part at 80 (launch_warp_kernel
+// chooses).  table_words > 0: every chain of the launch uses table 0, staged
 // in shared memory ahead of the per-chain areas.
 template <int G, typename Pairs, int MinBlocks>
 __global__ void __launch_bounds__(256, MinBlocks) warp_engine_kernel(const kmc_batch B, int rate_words,
@@ -601,54 +604,75 @@ __global__ void __launch_bounds__(256, MinBlocks) warp_engine_kernel(const kmc_b
             if ((threadIdx.x & 31) == 0) item = atomicAdd(B.work_counter, 1);
             item = __shfl_sync(kAll, item, 0);
             if (item >= B.n_work) break;
-            run_warp<G, Pairs>(B, sl, sm, chain_of(item), stab);
+            run_warp<G, Pairs, (MinBlocks > 2)>(B, sl, sm, chain_of(item), stab);
             __syncwarp();
         }
         return;
     }
     const int item = blockIdx.x * (blockDim.x >> 5) + warp;
     if (item >= B.n_work) return;      // the whole warp
-    run_warp<G, Pairs>(B, sl, sm, chain_of(item), stab);
+    run_warp<G, Pairs, (MinBlocks > 2)>(B, sl, sm, chain_of(item), stab);
+}
+
+// Whether a launch may take the 80-register kernel.  Not whole warps a chain,
+// nor slices of 16 with tables in memory: there its 24 warps an SM are slower
+// than two waves of 16 (N = 60, 3648 chains, tables in memory: 22.4 ms against
+// 10.4; N = 30 in slices of 16, 6000 chains: 6.8 against 5.9).
+template <int G, typename Pairs>
+constexpr bool lean_warps()
+{
+    return G <= (Pairs::kFarTable ? 8 : 16);
 }
 
 template <int G, typename Pairs>
 int launch_warp_kernel(const kmc_batch &b, cudaStream_t st, size_t smem, int rw, int tw)
 {
-    const int wpb = b.warps_per_block, grid = (b.n_work + wpb - 1) / wpb;
-    if (grid <= 0) return KMC_OK;
-    auto launch = [&](auto *kernel, int &configured) -> int {
-        const int rc = set_smem(kernel, smem, configured);
-        if (rc != KMC_OK) return rc;
-        int blocks = grid;
-        cudaError_t e;
+    const int wpb = b.warps_per_block, sms = sm_count();
+    int blocks = (b.n_work + wpb - 1) / wpb;
+    if (blocks <= 0) return KMC_OK;
+    auto *kernel = warp_engine_kernel<G, Pairs, 2>;
+    static int configured_rich = 0;
+    int rc = set_smem(kernel, smem, configured_rich);
+    if (rc != KMC_OK) return rc;
+    const bool crowded = blocks > (16 / wpb) * sms;      // more than the SMs hold at once
+    if (b.work_counter || (crowded && lean_warps<G, Pairs>())) {
+        int rich = 0, lean = 0;      // resident blocks an SM
+        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&rich, kernel, wpb * 32, smem);
+        if (e != cudaSuccess) return fail_cuda(e, "engine occupancy");
+        rich = max(1, rich);
         if (b.work_counter) {
             // persistent: as many blocks as stay resident at once, no more
             // than the work needs
-            int per_sm = 0;
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, wpb * 32, smem);
-            if (e != cudaSuccess) return fail_cuda(e, "engine occupancy");
-            blocks = min(blocks, max(1, per_sm) * sm_count());
+            blocks = min(blocks, rich * sms);
             if (b.max_grid > 0) blocks = min(blocks, b.max_grid);
+        } else if constexpr (lean_warps<G, Pairs>()) {
+            // The 80-register kernel where its residency saves more waves than
+            // its warps are slower: a wave of 24 takes 1/0.6 of one of 16
+            // (N = 12 in slices of 8, 12000 chains: 4.5 ms in one wave, 5.3 in
+            // two; N = 30 in slices of 16, positions, 6000: 5.5 and 6.1; N =
+            // 40, where shared memory holds no more than 16 warps: 10.1 and 8.2).
+            static int configured_lean = 0;
+            auto *small = warp_engine_kernel<G, Pairs, 3>;
+            if ((rc = set_smem(small, smem, configured_lean)) != KMC_OK) return rc;
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&lean, small, wpb * 32, smem);
+            if (e != cudaSuccess) return fail_cuda(e, "engine occupancy");
+            lean = max(1, lean);
+            const int q = (blocks + sms - 1) / sms, waves = (q + rich - 1) / rich, waves_lean = (q + lean - 1) / lean;
+            if (5 * waves_lean < 3 * waves) kernel = small;
         }
-        kernel<<<blocks, wpb * 32, smem, st>>>(b, rw, tw);
-        e = cudaGetLastError();
-        return e == cudaSuccess ? KMC_OK : fail_cuda(e, "engine launch");
-    };
-    // the register-rich variant when every block of the launch is resident at
-    // once with 16 warps per SM, else the one that fits 24
-    if (!b.work_counter && grid <= (16 / wpb) * sm_count()) {
-        static int configured_rich = 0;
-        return launch(warp_engine_kernel<G, Pairs, 2>, configured_rich);
     }
-    static int configured = 0;
-    return launch(warp_engine_kernel<G, Pairs, 3>, configured);
+    kernel<<<blocks, wpb * 32, smem, st>>>(b, rw, tw);
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? KMC_OK : fail_cuda(e, "engine launch");
 }
 
 template <int G, typename Pairs>
 int preload_warp_kernels()
 {
-    const int rc = touch_kernel(warp_engine_kernel<G, Pairs, 2>);
-    return rc == KMC_OK ? touch_kernel(warp_engine_kernel<G, Pairs, 3>) : rc;
+    int rc = touch_kernel(warp_engine_kernel<G, Pairs, 2>);
+    if constexpr (lean_warps<G, Pairs>())
+        if (rc == KMC_OK) rc = touch_kernel(warp_engine_kernel<G, Pairs, 3>);
+    return rc;
 }
 
 template <int G, typename Pairs>

@@ -49,3 +49,12 @@ def _same_as_alone(per_sm, N, P, lanes, mode, two, hops=40, **kw):
     (1, 100, 8, 512, "positions", False), (2, 100, 8, 512, "positions", False), (3, 240, 8, 256, "positions", False)])
 def test_block_groups_in_a_crowd(engine_lib, per_sm, N, P, lanes, mode, two):
     _same_as_alone(per_sm, N, P, lanes, mode, two)
+
+
+@pytest.mark.parametrize("per_sm,N,lanes,mode,two,kw", [
+    (20, 12, 8, "table", True, {}), (20, 12, 8, "table", False, {}), (20, 30, 16, "positions", False, {}),
+    (20, 40, 16, "positions", False, {}), (20, 30, 16, "table", True, {}), (17, 60, 32, "table", True, {}),
+    (20, 12, 8, "table", True, {"persistent": True}), (17, 60, 32, "positions", False, {"persistent": True})])
+def test_warp_slices_in_a_crowd(engine_lib, per_sm, N, lanes, mode, two, kw):
+    """More warps than the SMs hold at 128 registers."""
+    _same_as_alone(per_sm, N, 8, lanes, mode, two, **kw)

@@ -846,14 +846,12 @@ def superpose(basis, comp, voltages, mu=0.0, dev=None, stream=None):
     V = np.asarray(voltages, np.float64)
     C_, P = V.shape
     N = basis.shape[1]
-    pk = _Pack()
-    pk.add("basis", basis, torch.float64)
-    pk.add("V", V, torch.float64)
-    pk.add("comp", np.asarray(comp, np.float64), torch.float64)
-    t = pk.upload(d)
+    b = _dev(basis, torch.float64, d)
+    v = _dev(V, torch.float64, d)
+    cp = _dev(np.asarray(comp, np.float64), torch.float64, d)
     ec = torch.empty(max(C_ * N, 1), dtype=torch.float32, device=d)
     ve = torch.empty(max(C_ * P, 1), dtype=torch.float32, device=d)
-    check(lib().kmc_site_energies(C_, N, P, _ptr(t["basis"]), _ptr(t["V"]), float(mu), _ptr(t["comp"]), _ptr(ec), _ptr(ve),
+    check(lib().kmc_site_energies(C_, N, P, _ptr(b), _ptr(v), float(mu), _ptr(cp), _ptr(ec), _ptr(ve),
                                   _stream_handle(stream)))
     return ec, ve
 

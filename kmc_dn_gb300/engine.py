@@ -460,7 +460,7 @@ def make_work_lists(S_c, hops, lanes=None, sms=None):
 
 class TableSet:
     """Device-resident geometry data, built once and shared by batches:
-    FP32 pair tables (L, B) from the FP64 tables (kmc_build_table) and, in
+    FP32 pair tables (L, B) from the FP64 tables (build_tables) and, in
     positions mode, the site coordinates and rate constants."""
 
     def __init__(self, specs: Sequence[TableSpec], pair_mode="table", dev=None):
@@ -500,15 +500,25 @@ class TableSet:
             pk.add("pos", np.concatenate(rows), torch.float32)
             pk.add("pos_off", pos_off, torch.int64)
             pk.add("coef", np.asarray(coef, np.float32).reshape(-1), torch.float32)
-        dv = pk.upload(d)
+        dv = pk.upload(d)       # (waits for the stream: the tables are built too)
         self.tab_N, self.tab_P, self.tab_off = dv["N"], dv["P"], dv["off"]
         self.tab_pos, self.tab_pos_off, self.tab_coef = dv.get("pos"), dv.get("pos_off"), dv.get("coef")
 
 
 def build_tables(specs, Ns, Ps, tab_off, tab_LB):
-    """FP32 pair tables of all specs from their FP64 host tables
-    (kmc_build_tables), into tab_LB at tab_off (floats)."""
+    """FP32 pair tables of all specs from their FP64 host tables, into tab_LB
+    at tab_off (floats)."""
     n = len(specs)
+    if n <= 4:
+        # one copy an array and one launch a table, 0.07 ms a table;
+        # kmc_build_tables, with an allocation of its own, 0.3 for any few
+        for t, N, P, o in zip(specs, Ns, Ps, tab_off):
+            d, tc = (_dev(np.asarray(a, np.float64).reshape(t.S, t.S), torch.float64, tab_LB.device)
+                     for a in (t.distances, t.transitions_constant))
+            with torch.cuda.device(tab_LB.device):
+                check(lib().kmc_build_table(int(N), int(P), float(t.nu), float(t.I_0), float(t.R), _ptr(d), _ptr(tc),
+                                            C.c_void_p(tab_LB.data_ptr() + 4 * int(o)), _stream_handle()))
+        return
     keep = [np.ascontiguousarray(np.asarray(a, np.float64).reshape(t.S, t.S))
             for t in specs for a in (t.distances, t.transitions_constant)]
     dist = (C.c_void_p * n)(*[a.ctypes.data for a in keep[0::2]])

@@ -75,6 +75,7 @@ class _Pack:
     buffer."""
     _NP = {torch.uint8: np.uint8, torch.int32: np.int32, torch.int64: np.int64, torch.float32: np.float32,
            torch.float64: np.float64}
+    _LARGE = 1 << 20
 
     def __init__(self):
         self._items = []          # (name, offset, bytes, dtype, shape, array or None)
@@ -96,17 +97,28 @@ class _Pack:
         self._place(name, int(np.prod(shape, dtype=np.int64)), dtype, shape, None)
 
     def upload(self, dev):
-        host = np.empty(self._inputs, np.uint8)
-        for _, off, nb, _, _, a in self._items:
-            if a is not None:
-                host[off:off + nb] = a.reshape(-1).view(np.uint8)
         self.buffer = torch.empty(max(self._size, 256), dtype=torch.uint8, device=dev)
-        # the fill first: the copy from pageable memory waits for the stream,
+        # the fill first: the copies from pageable memory wait for the stream,
         # so the buffer is complete for launches on any stream
         if self._size > self._inputs:
             self.buffer[self._inputs:].zero_()
-        if self._inputs:
-            self.buffer[:self._inputs].copy_(torch.from_numpy(host))
+        # Neighbouring arrays in one copy; a large one from where it is (packing
+        # 16 MB took 4 ms, a copy more takes 0.03).
+        host, start = np.empty(self._inputs, np.uint8), 0
+        for _, off, nb, _, _, a in self._items:
+            if a is None:
+                continue
+            raw = a.reshape(-1).view(np.uint8)
+            if nb < self._LARGE:
+                host[off:off + nb] = raw
+                continue
+            if start < off:
+                self.buffer[start:off].copy_(torch.from_numpy(host[start:off]))
+            self.buffer[off:off + nb].copy_(torch.from_numpy(np.require(raw, requirements="W")))
+            start = off + ((nb + 255) & ~255)
+        if start < self._inputs:
+            self.buffer[start:self._inputs].copy_(torch.from_numpy(host[start:]))
+        self._items = [(*it[:5], None) for it in self._items]      # the host arrays are not needed any more
         return {name: self.buffer[off:off + nb].view(dt).view(shape) for name, off, nb, dt, shape, _ in self._items}
 
     def download(self, first, last):

@@ -72,6 +72,26 @@ def test_launch_covers_budgets_as_they_are(monkeypatch):
         assert segs[-1].max_hops_per_launch == -(-5000 // reanchor) * reanchor
 
 
+def test_pack_sends_large_arrays_from_where_they_are():
+    """Large arrays between small ones, first and last; read-only ones too."""
+    big = np.arange(engine._Pack._LARGE // 8 + 3, dtype=np.float64)
+    frozen = big[::-1].copy()
+    frozen.setflags(write=False)
+    for order in ("Bsb", "sBs", "BbB", "sss", "B", "bs"):
+        pk, want = engine._Pack(), {}
+        for k, c in enumerate(order):
+            a = {"B": big + k, "b": frozen, "s": np.arange(5 + k, dtype=np.int32)}[c]
+            want[f"a{k}"] = a
+            pk.add(f"a{k}", a, torch.float64 if c in "Bb" else torch.int32)
+        pk.zeros("z", 7, torch.int64)
+        t = pk.upload(torch.device("cpu"))
+        for k, a in want.items():
+            np.testing.assert_array_equal(t[k].numpy(), a)
+        assert not t["z"].any()
+        host = pk.download("a0", "z")
+        np.testing.assert_array_equal(host["a0"], want["a0"])
+
+
 @pytest.mark.gpu
 def test_budgets_raised_in_place_are_run(engine_lib):
     net = _positions_spec(24, 5, seed=1)

@@ -59,6 +59,7 @@ namespace {
 
 constexpr int kThreads = 128;
 constexpr int kWarps = kThreads / 32;
+constexpr int kDirectHops = 3;     // runs this short build no table of factors (f64_chain)
 // A site in a list: exp(+-E/kT) = m 2^k (a source's +, a target's -).
 struct __align__(16) Site {
     double m;
@@ -135,9 +136,17 @@ __device__ __forceinline__ void f64_chain(
     const double inv_kT = 1.0 / kT;
     const double IR = I0 * R;
     const double mIR = -I0 * R;
+    // A run of a few hops evaluates its pairs by the reference's expression:
+    // the table's exponentials, one a pair of acceptors, are 38 FP64
+    // instructions for N^2 pairs, the expression's 45 for at most N^2/4 + N P a
+    // hop (N = 200, one hop: 1.0 ms with the table, 0.86 without any).
+    const bool direct = hops <= kDirectHops;
     double *invd = lay.invd > 0 ? invd_s : invd_g;
     for (int j = tid; j < kExpTable; j += kThreads) exp_tab[j] = exp_table_entry(j);
-    if (tid == 0) wide_always = wide_now[0] = wide_now[1] = 0;
+    if (tid == 0) {
+        wide_always = direct;
+        wide_now[0] = wide_now[1] = 0;
+    }
     for (int k = tid; k < N * N; k += kThreads) {
         const int i = k / N, j = k - (k / N) * N;
         const double dij = d[(size_t)i * S + j];
@@ -149,7 +158,7 @@ __device__ __forceinline__ void f64_chain(
         const double cap = tc[k] * nu;
         double rest, m = 1.0;
         int e = 0;
-        if (i < N && j < N && i != j) {
+        if (i < N && j < N && i != j && !direct) {
             const double x = over_kT(IR / d[k], unit, kT, inv_kT, rest);
             if (splittable(x)) m = exp_split(x, rest, exp_tab, e);
             else wide_always = 1;

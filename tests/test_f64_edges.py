@@ -1,0 +1,47 @@
+"""The FP64 hop loop at the edges of its inputs: very short runs, uniforms on
+the ends of their interval, electrode counts beyond 32 bits, energies and
+rates at the ends of the exponent range."""
+import numpy as np
+import pytest
+
+from kmc_dn_gb300 import workloads
+from kmc_dn_gb300.rng import replay_uniforms
+
+pytestmark = pytest.mark.gpu
+
+
+def _net(N, P, seed=0, kT=1.0, nu=1.0, volts=1.0):
+    L = float(np.sqrt(N / workloads.DENSITY))
+    rng = np.random.Generator(np.random.PCG64(1000 * seed + N))
+    return workloads.make_network(rng, N, N // 10, L, L, workloads.perimeter_electrodes(L, P),
+                                  voltages=volts * rng.uniform(-1, 1, P), kT=kT, nu=nu, cells=30)
+
+
+def _args(n, **kw):
+    a = dict(N=n.N, P=n.P, nu=n.nu, kT=n.kT, I_0=n.I_0, R=n.R, occupation=n.occupation.astype(np.uint8),
+             distances=n.distances, E_constant=n.E_constant(), site_energies=n.site_energies(),
+             transitions_constant=n.transitions_constant)
+    a.update(kw)
+    return list(a.values())
+
+
+def _replay(oracle_mod, args, u, rtol, **kw):
+    """The kernel's run and the oracle's on one stream."""
+    from kmc_dn_gb300.engine import simulate_f64
+    hops = len(u) // 2
+    r = simulate_f64(*args, hops, record=True, uniforms=u, hop_log=True, **kw)
+    o = oracle_mod.numba_replay(*args, u, record=True, **kw)
+    assert r["status"] == 0
+    for k in ("hop_log", "traffic", "occupation", "electrode_occupation"):
+        np.testing.assert_array_equal(r[k], o[k], err_msg=k)
+    np.testing.assert_allclose(r["time"], o["time"], rtol=rtol)
+    np.testing.assert_allclose(r["occupations_in_time"], o["occupations_in_time"], rtol=rtol, atol=rtol * o["time"])
+    return r
+
+
+# (Tolerances of the times: test_kernel_shapes.py.)
+@pytest.mark.parametrize("hops", [1, 2, 3, 4, 5])
+@pytest.mark.parametrize("N,P,kT", [(1, 2, 1.0), (33, 8, 0.7), (100, 8, 1.0), (160, 8, 1.0), (400, 8, 2.0)])
+def test_short_runs(engine_lib, oracle_mod, N, P, kT, hops):
+    """Runs of up to three hops take every pair's own exponential."""
+    _replay(oracle_mod, _args(_net(N, P, kT=kT)), replay_uniforms(11 + hops, 2 * hops), 1e-10)

@@ -89,7 +89,7 @@ struct Layout {
 __host__ __device__ inline size_t layout_bytes(const Layout &l)
 {
     return 20 * static_cast<size_t>(l.tab) + 8 * static_cast<size_t>(l.rates + l.invd) + 16 * kExpTable +
-           (2 * sizeof(Site) + 2 * 8 + 4) * static_cast<size_t>(l.S) + 8 * (kThreads + 64 + 128) + 4 * 64 + 32;
+           (2 * sizeof(Site) + 2 * 8 + 8) * static_cast<size_t>(l.S) + 8 * (kThreads + 64 + 128) + 4 * 64 + 32;
 }
 
 // One chain run by the whole block (the body of both kernels below).
@@ -117,9 +117,9 @@ __device__ __forceinline__ void f64_chain(
     double *u_cl = u_ev + 32;                                      // [32] -log(1 - u1)
     double *sh_J = u_cl + 32;                                      // [64] expected net inflow
     double *sh_fx = sh_J + 64;                                     // [64] its time integral
-    int *tab_k = reinterpret_cast<int *>(sh_fx + 64);              // [S*S] exponents beside tab
-    int *eo_s = tab_k + lay.tab;                                   // [P]
-    uint32_t *occw = reinterpret_cast<uint32_t *>(eo_s + lay.S);   // [64] occupancy bits
+    long long *eo_s = reinterpret_cast<long long *>(sh_fx + 64);   // [P] electrode counters
+    int *tab_k = reinterpret_cast<int *>(eo_s + lay.S);            // [S*S] exponents beside tab
+    uint32_t *occw = reinterpret_cast<uint32_t *>(tab_k + lay.tab);   // [64] occupancy bits
     __shared__ int wide_always, wide_now[2];   // energies or couplings beyond the split exponential
     __shared__ int ev_from, ev_to;
     __shared__ double sh_dt;
@@ -180,7 +180,7 @@ __device__ __forceinline__ void f64_chain(
         occw[w] = bits;
     }
     for (int e = tid; e < P; e += kThreads) {
-        eo_s[e] = 0;
+        eo_s[e] = eo[e];
         if (flux_time) sh_fx[e] = flux_time[e];
     }
     // the electrodes' list entries, the same every hop
@@ -485,7 +485,7 @@ __device__ __forceinline__ void f64_chain(
     for (int i = tid; i < N; i += kThreads) occ_g[i] = (occw[i >> 5] >> (i & 31)) & 1u;
     if (record && tid < N) oit[tid] = oit0;
     for (int e = tid; e < P; e += kThreads) {
-        eo[e] += eo_s[e];
+        eo[e] = eo_s[e];
         if (flux_time) flux_time[e] = sh_fx[e];
     }
     if (tid == 32) *time_out = time;

@@ -60,3 +60,14 @@ def test_event_uniforms_at_the_ends(engine_lib, oracle_mod, N, P):
         u[81], u[101], u[121], u[131] = -0.0, 1.5, np.nan, 5e-324
         r = _replay(oracle_mod, _args(n), u, 1e-11)
         assert r["traffic"][0, 0] >= 6 and r["hop_log"][0].tolist() == [0, 0]
+
+
+def test_electrode_counts_beyond_32_bits(engine_lib, oracle_mod):
+    """The counters are the caller's 64-bit ones throughout the run."""
+    n = _net(30, 6, seed=3)
+    edge = 2**31
+    start = np.array([edge - 1, -edge, edge, -edge - 1, 2**62, 0], np.int64)
+    u = replay_uniforms(8, 2000)
+    r = _replay(oracle_mod, _args(n), u, 1e-11, electrode_occupation=start)
+    moved = r["electrode_occupation"] - start
+    assert moved[0] or moved[1] or moved[2] or moved[3]

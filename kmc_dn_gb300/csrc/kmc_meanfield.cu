@@ -228,14 +228,17 @@ __device__ void mf_pairs(const kmc_mf_batch &b)
     __shared__ double sh_f, sh_ts, sh_time;
     __shared__ int sh_stop;
 
-    // pair tables: K = nu*tc, B = I_0 R / d between acceptors (0 otherwise)
-    // (and on the diagonal, where the rate is K either way), no rate between
-    // electrodes
+    const double inv_kT = 1.0 / kT;
+    // pair tables: K = nu*tc, B = I_0 R / d between acceptors (0 otherwise),
+    // no rate between electrodes.  A site onto itself: dE = -I_0 R / d_ii, so
+    // the rate is K whatever the state unless the sites attract (I_0 < 0: 0
+    // for d_ii = 0); B = 0 there, for the energies' sums.
     for (int p = tid; p < SS; p += T) {
         const int i = p / S, j = p - (p / S) * S;
-        const double K = (i >= N && j >= N) ? 0.0 : nu * tcon[p];
-        const double B = (i < N && j < N && i != j) ? I0R / dist[p] : 0.0;
-        KB[i * SP + j] = Pair{static_cast<Real>(K), static_cast<Real>(B)};
+        double K = (i >= N && j >= N) ? 0.0 : nu * tcon[p];
+        const double c = (i < N && j < N) ? I0R / dist[p] : 0.0;
+        if (i == j && c < 0.0) K *= exp(c * inv_kT);
+        KB[i * SP + j] = Pair{static_cast<Real>(K), static_cast<Real>(i != j ? c : 0.0)};
     }
     for (int k = tid; k < S; k += T) {
         occ[k] = k < N ? occ_io[k] : F64 ? 1.0 : 0.0;
@@ -253,7 +256,6 @@ __device__ void mf_pairs(const kmc_mf_batch &b)
     __syncthreads();
 
     const Real ec_i = tid < N ? static_cast<Real>(Ec[tid]) : Real(0);
-    const double inv_kT = 1.0 / kT;
     const bool unit = kT == 1.0;
     const float c2 = static_cast<float>(1.4426950408889634 / kT);
     const int64_t hops = b.hops[c];

@@ -238,6 +238,9 @@ __device__ void mf_pairs(const kmc_mf_batch &b)
         double K = (i >= N && j >= N) ? 0.0 : nu * tcon[p];
         const double c = (i < N && j < N) ? I0R / dist[p] : 0.0;
         if (i == j && c < 0.0) K *= exp(c * inv_kT);
+        // 1/kT infinite or NaN: so are exponents of 0, and the network stops
+        // (the FP64 rates take no exponential for them)
+        if (F64 && !(fabs(inv_kT) < INFINITY)) K = NAN;
         KB[i * SP + j] = Pair{static_cast<Real>(K), static_cast<Real>(i != j ? c : 0.0)};
     }
     for (int k = tid; k < S; k += T) {

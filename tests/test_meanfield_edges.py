@@ -29,3 +29,11 @@ def test_sites_that_attract(engine_lib, oracle_mod, rates, tol, I_0):
     np.testing.assert_allclose(r["occupation"][0], o["occupation"], atol=tol, rtol=0)
     np.testing.assert_allclose(r["electrode_occupation"][0], o["electrode_occupation"],
                                atol=tol * max(1.0, np.abs(o["electrode_occupation"]).max()), rtol=0)
+
+
+@pytest.mark.parametrize("rates", ["f64", "f32"])
+@pytest.mark.parametrize("kT", [0.0, -0.0, np.nan, 5e-324])
+def test_no_temperature_no_result(engine_lib, rates, kT):
+    from kmc_dn_gb300._native import KMC_ERR_NONFINITE
+    r = _run(workloads.plain_network(2), 12, rates, kT=kT)
+    assert r["status"][0] == KMC_ERR_NONFINITE and r["iterations"][0] == 0

@@ -1,7 +1,7 @@
-// kmc_exp64.cuh -- FP64 exponentials as mantissa and exponent, and integer
-// comparisons, shared by the FP64 hop loop and the FP64 mean field.  A warp's
-// FP64 instruction holds its SM quarter's unit for 64 cycles on this part, a
-// comparison, a conversion or a negation as much as a multiplication.
+// kmc_exp64.cuh -- FP64 exponentials as mantissa and exponent, for the FP64 hop
+// loop, and comparisons on the integer pipe, for it and the FP64 mean field.  A
+// warp's FP64 instruction holds its SM quarter's unit for 64 cycles on this
+// part, a comparison, a conversion or a negation as much as a multiplication.
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -22,13 +22,13 @@ __device__ __forceinline__ bool not_less(double x, long long y_bits)
     return __double_as_longlong(x) >= y_bits;
 }
 
-// exp(x + y) = m * 2^k, 1 <= m <= 2, y a small correction of x, by table and
-// short polynomial (Tang, "Table-driven implementation of the exponential
-// function in IEEE floating-point arithmetic", ACM TOMS 15, 1989):
+// exp(x + y) = m * 2^k, 2^(-1/256) <= m < 2, y a small correction of x, by
+// table and short polynomial (Tang, "Table-driven implementation of the
+// exponential function in IEEE floating-point arithmetic", ACM TOMS 15, 1989):
 // x = (128 k + j) ln2/128 + r, |r| <= ln2/256, m = 2^(j/128) (1 + p(r)), the
-// table entries with their low parts.  |x| < 2^17.  Within 0.51 ulp (largest
-// of 4e6 arguments in (-708, 0]; exp() there 0.87) while |x| < 5000; beyond,
-// the reduction rounds by 2^-53 |x|, as the energies themselves do.
+// table entries with their low parts.  |x| < 2^17, where n ln2/128 has 58 bits
+// and the part of it that the subtraction leaves is exact: within 0.51 ulp of
+// m throughout (tests/test_exp64.py; exp() 0.87 on 4e6 arguments in (-708, 0]).
 constexpr int kExpTable = 128;
 __device__ __forceinline__ double exp_split(double x, double y, const double2 *table, int &k)
 {

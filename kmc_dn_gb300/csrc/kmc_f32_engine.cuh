@@ -503,35 +503,24 @@ struct PairRange {
     int h, z, P;         // holes, empty acceptors, electrodes
     int T1, T2, A1, A;   // targets of a hole row / an electrode row, pairs of the hole rows, all pairs
     float inv1, inv2;    // 1/T1, 1/T2
-    __device__ __forceinline__ void init(int h_, int N, int P_)
-    {
-        h = h_;
-        P = P_;
-        z = N - h_;
-        T1 = z + P;
-        T2 = z;
-        A1 = h * T1;
-        A = A1 + P * T2;
-        inv1 = T1 > 0 ? rcp_approx(static_cast<float>(T1)) : 0.0f;
-        inv2 = T2 > 0 ? rcp_approx(static_cast<float>(T2)) : 0.0f;
-    }
 };
 
-// Walks pairs [b, e) in row-major order, kPairStep pairs a step: all loads
+// Walks pairs [b, e) in row-major order, kStep pairs a step: all loads
 // and rates of a step come before its stores, because the compiler moves no
 // list or table load across a store of the running sums, and a step's latency
-// (two dependent shared loads and an ex2) is then paid once for kPairStep
+// (two dependent shared loads and an ex2) is then paid once for kStep
 // pairs instead of for every two.  A row change is a select plus a predicated
-// reload of the source record, not a branch.  kSum: the rates add up in s, in
-// order; kKeep: the sum (without kSum the rate) of every pair goes to rp,
-// rp + kStride, ...  Measured with 2, 4 and 8 pairs a
+// reload of the source record, not a branch.  The rates add up in s, in order;
+// kKeep: the sum after every pair goes to rp, rp + kStride, ...  Returns false
+// where a pair is none of the state's (checked in debug builds, before its
+// records are read).  Measured with 2, 4 and 8 pairs a
 // step: 4096 N=30 chains (staged table) 32.0 / 31.9 / 33.1 ms, a search
 // population of 384 networks (tables in L2) 95.7 / 79.3 / 77.2 ms, one N=100
 // chain 24.1 / 23.1 / 24.8 ms.  (Two phases, all rates by the whole group in
 // coalesced order and then each thread's sums, measured 37 to 39 ms on the
 // N=30 chains: fewer bank conflicts, more instructions.)
-template <bool kSum, bool kKeep, int kStride, int kStep, typename Pairs>
-__device__ __forceinline__ void walk_pairs(const Pairs &pairs, const typename Pairs::Rec *src,
+template <bool kKeep, int kStride, int kStep, typename Pairs>
+__device__ __forceinline__ bool walk_pairs(const Pairs &pairs, const typename Pairs::Rec *src,
                                            const typename Pairs::Rec *tgt, const PairRange &R, int b, int e, float cs,
                                            float *rp, float &s)
 {
@@ -539,6 +528,9 @@ __device__ __forceinline__ void walk_pairs(const Pairs &pairs, const typename Pa
     decode_pair(b, R.h, R.A1, R.T1, R.T2, R.inv1, R.inv2, row, col);
     bool sa = row < R.h;
     int Tc = sa ? R.T1 : R.T2;
+#ifdef KMC_DEBUG_CHECKS
+    if (e > R.A || row < 0 || row >= R.h + R.P || col < 0 || col >= Tc) return false;
+#endif
     typename Pairs::Rec sr = src[row];
     auto step = [&](auto whole, int left) {
         constexpr bool kWhole = decltype(whole)::value;
@@ -547,10 +539,11 @@ __device__ __forceinline__ void walk_pairs(const Pairs &pairs, const typename Pa
         for (int u = 0; u < kStep; ++u) {
             if (kWhole || u < left) {
                 r[u] = pairs.rate(sr, tgt_load<Pairs>(tgt, col), sa && col < R.z, cs);
-                // (the row after a last pair is not read)
                 const bool w = (col + 1 == Tc);
                 col = w ? 0 : col + 1;
                 row += w ? 1 : 0;
+                // (a whole step that ends the last row reads the record after
+                // it: at most src[S], and the list has room for S + 2)
                 if (w && (kWhole || u + 1 < left)) sr = src[row];
                 sa = row < R.h;
                 Tc = sa ? R.T1 : R.T2;
@@ -559,8 +552,8 @@ __device__ __forceinline__ void walk_pairs(const Pairs &pairs, const typename Pa
 #pragma unroll
         for (int u = 0; u < kStep; ++u) {
             if (kWhole || u < left) {
-                if constexpr (kSum) s += r[u];
-                if constexpr (kKeep) rp[u * kStride] = kSum ? s : r[u];
+                s += r[u];
+                if constexpr (kKeep) rp[u * kStride] = s;
             }
         }
     };
@@ -570,6 +563,7 @@ __device__ __forceinline__ void walk_pairs(const Pairs &pairs, const typename Pa
         if constexpr (kKeep) rp += kStep * kStride;
     }
     if (k < e) step(BoolC<false>{}, e - k);
+    return true;
 }
 
 // ---------------------------------------------------------------------------
@@ -1049,11 +1043,7 @@ __device__ void run_chain(const kmc_batch &B, const Grp &grp, ChainSmem<typename
     const float *Vel = B.el_energy + eoff;
     uint8_t *occ_g = B.occupation + so;
     const float cs = kLog2e / B.chain_kT[c];
-    if (Pairs::kUniformTable && !(B.chain_kT[c] == B.uniform_kT)) {
-        // the staged table was scaled for another temperature
-        if (g == 0) B.status[c] = KMC_ERR_INVALID;
-        return;
-    }
+    static_assert(!Pairs::kUniformTable, "one temperature for a launch: warp slices only");
     const int64_t hops_done0 = B.hops_done[c];
     int64_t todo = B.hops_total[c] - hops_done0;
     if (todo > B.max_hops_per_launch) todo = B.max_hops_per_launch;
@@ -1286,8 +1276,10 @@ __device__ void run_chain(const kmc_batch &B, const Grp &grp, ChainSmem<typename
             }
         };
         auto walk_balanced = [&](auto store) {
-            PairRange range{h, z, P, T1, T2, A1, A, inv1, inv2};
-            walk_pairs<true, decltype(store)::value, RS, kPairStep>(pairs, sm.src, sm.tgt, range, run_b, run_e, cs, rp, lsum);
+            const PairRange range{h, z, P, T1, T2, A1, A, inv1, inv2};
+            [[maybe_unused]] const bool in_range = walk_pairs<decltype(store)::value, RS, kPairStep>(
+                pairs, sm.src, sm.tgt, range, run_b, run_e, cs, rp, lsum);
+            KMC_DCHECK(in_range);
         };
         if (aligned) {
             if (rp) walk_aligned(BoolC<true>{});

@@ -267,10 +267,10 @@ __device__ void run_warp(const kmc_batch &B, const Slice<G> &sl, ChainSmem<typen
             const PairRange range{h, z, P, T1, T2, A1, A, inv1, inv2};
             float lsum = 0.0f;
             if (kb < ke) {
-                if (stored)
-                    walk_pairs<true, true, RS, kPairStep>(pairs, sm.src, sm.tgt, range, kb, ke, cs, sm.rates + g, lsum);
-                else
-                    walk_pairs<true, false, RS, kPairStep>(pairs, sm.src, sm.tgt, range, kb, ke, cs, nullptr, lsum);
+                [[maybe_unused]] const bool in_range =
+                    stored ? walk_pairs<true, RS, kPairStep>(pairs, sm.src, sm.tgt, range, kb, ke, cs, sm.rates + g, lsum)
+                           : walk_pairs<false, RS, kPairStep>(pairs, sm.src, sm.tgt, range, kb, ke, cs, nullptr, lsum);
+                KMC_DCHECK(in_range);
             }
             npairs += static_cast<unsigned>(A);
             KMC_SECTION(1);

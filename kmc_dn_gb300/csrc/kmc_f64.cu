@@ -707,7 +707,7 @@ extern "C" int kmc_simulate_f64_static(int32_t n_acceptors, int32_t n_electrodes
     const int rc = static_workspace(&ws);
     if (rc != KMC_OK) return rc;
     // The kernel writes every workspace entry it reads within the call
-    // (1/d, I_0 R/d and the running sums), so the contents a previous call
+    // (the pairs' factors, 1/d and the rates), so the contents a previous call
     // left behind need no clearing.
     return simulate_f64(n_acceptors, n_electrodes, nu, kT, I_0, R, occupation, distances, E_constant,
                         site_energies, transitions_constant, electrode_occupation, hops, record,

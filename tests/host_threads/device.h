@@ -124,6 +124,7 @@ inline double __hiloint2double(int h, int l)
 inline float __uint2float_rn(uint32_t x) { return static_cast<float>(x); }
 inline float __int2float_rn(int x) { return static_cast<float>(x); }
 inline int __float2int_rz(float x) { return static_cast<int>(x); }
+inline double __ull2double_rn(uint64_t x) { return static_cast<double>(x); }
 inline uint64_t __double2ull_rz(double x) { return x >= 0x1p64 ? ~0ull : static_cast<uint64_t>(x); }
 inline float __fadd_rn(float a, float b) { return a + b; }
 inline float __fsub_rn(float a, float b) { return a - b; }

@@ -21,6 +21,11 @@ double uniform()
     return static_cast<double>(rng_state >> 11) * 0x1p-53;
 }
 
+// a rate of 1 for every pair
+struct PairPlace : PositionPairs {
+    float rate(float4, float4, bool, float) const { return 1.0f; }
+};
+
 // record: the Go convention with flux, drift and log; stored: with the buffer
 // of running sums; two: two tables (read from memory, not staged).
 template <int G, typename Pairs>
@@ -123,6 +128,20 @@ int launch(int N, int P, int reanchor, int hops, int chains, bool record, bool s
     return 0;
 }
 
+#ifdef KMC_DEBUG_CHECKS
+// Runs of two holes, three empty acceptors and one electrode (11 pairs): 0
+// where those within are walked and those beyond are refused.
+int runs()
+{
+    const PairPlace place{};
+    std::vector<float4> rec(8, make_float4(0.0f, 0.0f, 0.0f, 0.0f));
+    const PairRange range{2, 3, 1, 4, 3, 8, 11, 0.25f, 1.0f / 3.0f};
+    float kept[16], sum = 0.0f;
+    auto walk = [&](int b, int e) { return walk_pairs<true, 1, 4>(place, rec.data(), rec.data(), range, b, e, 1.0f, kept, sum); };
+    return walk(0, 11) && walk(3, 9) && sum == 17.0f && !walk(0, 12) && !walk(10, 12) && !walk(11, 12) && !walk(-1, 3) ? 0 : 1;
+}
+#endif
+
 }  // namespace
 
 int main(int, char **argv)
@@ -137,6 +156,9 @@ int main(int, char **argv)
     case 4: return launch<256, PairedPositionPairs>(70, 6, 5, 10, 1, true, true, false);
     case 5: return launch<16, Far>(40, 4, 5, 40, 2, true, true, true);
     case 6: return launch<32, Far>(40, 4, 9, 40, 1, false, true, true);
+#ifdef KMC_DEBUG_CHECKS
+    case 7: return runs();
+#endif
     }
     return 2;
 }

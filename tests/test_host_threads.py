@@ -37,9 +37,17 @@ def _host_source(text):
     return text.replace('"../../include/kmc_dn_gb300.h"', '"%s/include/kmc_dn_gb300.h"' % REPO)
 
 
-def _compile(folder, source, out, *flags):
-    cmd = ["g++", "-std=c++20", "-O1", "-g", "-fsanitize=thread", "-pthread", "-w", *flags, source, "-o", out]
+def _compile(folder, source, out, *flags, sanitize="thread"):
+    cmd = ["g++", "-std=c++20", "-O1", "-g", f"-fsanitize={sanitize}", "-pthread", "-w", *flags, source, "-o", out]
     return subprocess.run(cmd, capture_output=True, text=True, cwd=folder)
+
+
+def _sources(folder):
+    for name in os.listdir(CSRC):
+        if name.endswith((".cuh", ".h")):
+            with open(os.path.join(CSRC, name)) as f:
+                (folder / name).write_text(_host_source(f.read()))
+    return ["-I", str(folder), "-I", HERE, "-I", _cuda_include()]
 
 
 @pytest.fixture(scope="module")
@@ -51,12 +59,7 @@ def engine(tmp_path_factory):
     if not shutil.which("g++") or _compile(folder, str(probe), "probe").returncode or \
             "data race" not in subprocess.run([str(folder / "probe")], capture_output=True, text=True).stderr:
         pytest.skip("no g++ with a working ThreadSanitizer")
-    for name in os.listdir(CSRC):
-        if name.endswith((".cuh", ".h")):
-            with open(os.path.join(CSRC, name)) as f:
-                (folder / name).write_text(_host_source(f.read()))
-    r = _compile(folder, os.path.join(HERE, "engine.cpp"), "engine", "-I", str(folder), "-I", HERE, "-I",
-                 _cuda_include())
+    r = _compile(folder, os.path.join(HERE, "engine.cpp"), "engine", *_sources(folder))
     assert r.returncode == 0, r.stderr[-4000:]
     return str(folder / "engine")
 
@@ -67,3 +70,17 @@ def test_shared_memory_is_ordered(engine, launch):
     races = re.findall(r"SUMMARY: ThreadSanitizer: (.*)", r.stderr)
     assert not races, "\n".join(sorted(set(races)))
     assert r.returncode == 0, r.stderr[-2000:]
+
+
+def test_debug_build_checks_the_runs(tmp_path):
+    """-DKMC_DEBUG_CHECKS: a run that leaves the state's pairs is refused before
+    its records are read, and the launches above pass their checks (with the
+    address sanitizer on their shared memory)."""
+    if not shutil.which("g++"):
+        pytest.skip("no g++")
+    r = _compile(tmp_path, os.path.join(HERE, "engine.cpp"), "checked", "-DKMC_DEBUG_CHECKS", *_sources(tmp_path),
+                 sanitize="address")
+    assert r.returncode == 0, r.stderr[-4000:]
+    for launch in range(len(LAUNCHES) + 1):
+        r = subprocess.run([str(tmp_path / "checked"), str(launch)], capture_output=True, text=True, timeout=600)
+        assert r.returncode == 0 and "error" not in r.stderr, (launch, r.stderr[-2000:])

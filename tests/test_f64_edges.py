@@ -50,13 +50,14 @@ def test_short_runs(engine_lib, oracle_mod, N, P, kT, hops):
 @pytest.mark.parametrize("N,P", [(5, 3), (33, 8), (100, 8)])
 def test_event_uniforms_at_the_ends(engine_lib, oracle_mod, N, P):
     """An event uniform of 0 takes the dense loop's first entry, pair (0, 0),
-    which fills site 0; one outside [0, 1] never passes and ends there too."""
+    which fills site 0; one outside [0, 1] never passes and ends there too.
+    (1 itself is the boundary of every pair whose successors are lost in the
+    total's rounding: which of them is first depends on the sums' order.)"""
     for fill in (False, True):
         n = _net(N, P, seed=2)
         n.occupation[0] = fill
         u = replay_uniforms(5, 160)
         u[[1, 3, 41, 159]] = 0.0
-        u[[21, 61]] = 1.0
         u[81], u[101], u[121], u[131] = -0.0, 1.5, np.nan, 5e-324
         r = _replay(oracle_mod, _args(n), u, 1e-11)
         assert r["traffic"][0, 0] >= 6 and r["hop_log"][0].tolist() == [0, 0]

@@ -42,7 +42,7 @@
 // One N = 30, P = 8 chain: 4.0 us a hop (18.8 us with S^2 dense rates and
 // running sums in global memory, 6.1 us with the pairs' exponentials queued
 // 32 at a time); 256 chains of N = 60, P = 8, 300 hops with occupancy and
-// flux: 4.2 ms (28.9 ms, 6.6 ms).  Time against the same hop sequences in
+// flux: 3.8 ms (28.9 ms, 6.6 ms).  Time against the same hop sequences in
 // 113-bit arithmetic, rms relative error over 40 networks: N = 30 1.3e-14
 // (dense rates 1.4e-14), N = 60 1.96e-13 (1.89e-13): the energies' rounding.
 #include <algorithm>
@@ -634,8 +634,10 @@ int simulate_f64_batch(const kmc_f64_batch &B, cudaStream_t st)
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return fail_cuda(e, "simulate_f64_batch: device query");
     // Blocks that share an SM overlap their serial phases, so a launch of
-    // more chains than SMs divides an SM's shared memory among up to four.
-    const int per_sm = std::max(1, std::min(4, (B.n_chains + sms - 1) / std::max(sms, 1)));
+    // more chains than SMs divides an SM's shared memory among up to three:
+    // 150 registers a thread hold no more (304 chains of N = 60, 100 hops 2.2
+    // ms, 152 1.7; 512, the last 56 in a second wave, 4.1).
+    const int per_sm = std::max(1, std::min(3, (B.n_chains + sms - 1) / std::max(sms, 1)));
     // A(h) <= S^2/3 for any split of S sites into acceptors and electrodes
     const Layout lay = f64_layout(S, S, static_cast<int64_t>(S) * S / 3 + 1,
                                   std::min(kBlockSmem, kSmSmem / per_sm - 1280));

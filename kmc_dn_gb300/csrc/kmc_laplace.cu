@@ -19,12 +19,12 @@
 // F is zero but for the nodes beside the boundary, so its transform is four
 // matrix-vector products a field (the sides' data) and four outer products.
 // The inverse transform is the work: two products with Q a field, FP64, whose
-// unit takes 64 cycles a warp instruction and SM quarter, spread over one
-// wave of blocks.  Q itself is never stored: its entries are the 2n values
+// unit takes 64 cycles a warp instruction and SM quarter, spread over
+// more blocks than the SMs hold at once.  Q itself is never stored: its entries are the 2n values
 // sin(pi q/n), q = (k+1)(j+1) mod 2n, in shared memory.  (Half the products
 // could be had from Q's mirror symmetry Q[k][m-1-j] = (-1)^k Q[k][j]; that
 // moved the result by 7e-15, where this is within 1e-15 of the plain products.)
-// Four launches; 9 fields of 99 x 99 cells: 84 us (134 us in nine launches
+// Four launches; 9 fields of 99 x 99 cells: 74 us (141 us in nine launches
 // with Q and dense products in 16 x 16 tiles).
 #include <cmath>
 #include <cstdint>
@@ -37,7 +37,14 @@ namespace {
 
 constexpr int kSides = 4;              // left, right (along y), bottom, top (along x)
 constexpr int kThreads = 128;
-constexpr int kRows = 6;               // rows of a field per block of a product: 147 blocks for 9 fields of 98 rows
+// Rows of a field per block of a product.  Few, so that even small meshes give
+// blocks to every SM several times over, but a block's copy of the sine table
+// (2n entries) is shared by its rows.  Kernels of 9 fields, us, at 3 / 4 / 6 /
+// 8 / 12 rows: 30 cells a side 30 / 30 / 35 / 34 / 39, 99: 74 / 86 / 89 / 104
+// / 137, 150: 142 / 183 / 180 / 237 / 242, 99 x 300: 252 / 296 / 329 / 382 /
+// 518, 300: 934 / 981 / 903 / 1161 / 1190, 1000: 30 / 32 / 34 / 32 / 36 ms,
+// 2000: 237 / 237 / 344 / 343 / 238 ms.
+constexpr int kRows = 3;
 
 // Per direction: sqrt(2/n) sin(pi q/n), q = 0 .. 2n-1, and the eigenvalues
 // 2 - 2 cos(pi (k+1)/n).

@@ -377,67 +377,66 @@ __device__ __forceinline__ void f64_chain(
                 if (lane == 0) ev_from = -1;      // zero, negative, infinite or NaN
             } else {
                 const double u2 = u_ev[hop & 31];
-                // u2 in (0, 1]; on any other (a replay stream may hold 0) the
-                // dense loop takes its first entry: pair (0, 0)
-                int f = 0, t = 0;
-                if (static_cast<unsigned long long>(__double_as_longlong(u2)) - 1ull < 0x3ff0000000000000ull) {
-                    // First k with cum_k/total >= u2 (the reference's test).
-                    // Where cum_k is 2^13 units in the last place or more away
-                    // from u2*total (over 1e-12 relative, far more than the
-                    // rounding of either side), the product decides it, else a
-                    // division.
-                    const long long ut = __double_as_longlong(u2 * total), lo = ut - 8192, hi = ut + 8192;
-                    // the first warp, then the first thread, whose last sum may pass
-                    int w = 0;
-                    double before = 0.0;
+                // First k with cum_k/total >= u2 (the reference's test).
+                // Where cum_k is 2^13 units in the last place or more away
+                // from u2*total (over 1e-12 relative, far more than the
+                // rounding of either side), the product decides it, else a
+                // division.
+                const long long ut = __double_as_longlong(u2 * total), lo = ut - 8192, hi = ut + 8192;
+                // the first warp, then the first thread, whose last sum may pass
+                int w = 0;
+                double before = 0.0;
 #pragma unroll
-                    for (int v = 0; v < kWarps - 1; ++v)
-                        if (!not_less(upto[v], lo)) { w = v + 1; before = upto[v]; }
-                    double sums = before + incl[w * 32 + lane];     // up to each thread's end
-                    const unsigned b = __ballot_sync(0xffffffffu, not_less(sums, lo));
-                    int g = w * 32 + (b ? __ffs(b) - 1 : 31);
-                    int ev = -1, last = 0;
-                    double run = __shfl_sync(0xffffffffu, sums, (g - 1) & 31);
-                    if (!(g & 31)) run = before;
-                    for (;;) {
-                        // 32 pairs of thread g's run at a time, a lane each
-                        const int gb = g * M, ge = min(gb + M, A);
-                        for (int k0 = gb; k0 < ge && ev < 0; k0 += 32) {
-                            const int k = k0 + lane;
-                            const double r = k < ge ? rates[k] : 0.0;
-                            double x = r;
-                            const int n = min(32, ge - k0);
-                            for (int s = 1; s < n; s <<= 1) {
-                                const double o = __shfl_up_sync(0xffffffffu, x, s);
-                                if (lane >= s) x += o;
-                            }
-                            const double cum = run + x;
-                            const bool hit = k < ge && (not_less(cum, hi) || (not_less(cum, lo) && cum / total >= u2));
-                            const unsigned hits = __ballot_sync(0xffffffffu, hit);
-                            if (hits) {
-                                ev = k0 + __ffs(hits) - 1;
-                            } else {
-                                const unsigned some = __ballot_sync(0xffffffffu, positive(r));
-                                if (some) last = k0 + 31 - __clz(some);
-                                run = __shfl_sync(0xffffffffu, cum, 31);
-                            }
+                for (int v = 0; v < kWarps - 1; ++v)
+                    if (!not_less(upto[v], lo)) { w = v + 1; before = upto[v]; }
+                double sums = before + incl[w * 32 + lane];     // up to each thread's end
+                const unsigned b = __ballot_sync(0xffffffffu, not_less(sums, lo));
+                int g = w * 32 + (b ? __ffs(b) - 1 : 31);
+                int ev = -1, last = 0;
+                double run = __shfl_sync(0xffffffffu, sums, (g - 1) & 31);
+                if (!(g & 31)) run = before;
+                for (;;) {
+                    // 32 pairs of thread g's run at a time, a lane each
+                    const int gb = g * M, ge = min(gb + M, A);
+                    for (int k0 = gb; k0 < ge && ev < 0; k0 += 32) {
+                        const int k = k0 + lane;
+                        const double r = k < ge ? rates[k] : 0.0;
+                        double x = r;
+                        const int n = min(32, ge - k0);
+                        for (int s = 1; s < n; s <<= 1) {
+                            const double o = __shfl_up_sync(0xffffffffu, x, s);
+                            if (lane >= s) x += o;
                         }
-                        if (ev >= 0 || ++g >= kThreads || g * M >= A) break;
-                        // not in that run after all: the next thread's, from the
-                        // prefix it has
-                        if ((g >> 5) != w) before += incl[w++ * 32 + 31];
-                        run = (g & 31) ? before + incl[g - 1] : before;
+                        const double cum = run + x;
+                        const bool hit = k < ge && (not_less(cum, hi) || (not_less(cum, lo) && cum / total >= u2));
+                        const unsigned hits = __ballot_sync(0xffffffffu, hit);
+                        if (hits) {
+                            ev = k0 + __ffs(hits) - 1;
+                        } else {
+                            const unsigned some = __ballot_sync(0xffffffffu, positive(r));
+                            if (some) last = k0 + 31 - __clz(some);
+                            run = __shfl_sync(0xffffffffu, cum, 31);
+                        }
                     }
-                    // u2 within the rounding of 1: the last pair that can hop
-                    if (ev < 0) ev = last;
-                    int row, col;
-                    if (ev < A1) row = div_small(ev, T1, inv1, col);
-                    else row = N + div_small(ev - A1, T2, inv2, col);
-                    if (col >= z) col += N - z;
-                    f = src[row].id;
-                    t = tgt[col].id;
+                    if (ev >= 0 || ++g >= kThreads || g * M >= A) break;
+                    // not in that run after all: the next thread's, from the
+                    // prefix it has
+                    if ((g >> 5) != w) before += incl[w++ * 32 + 31];
+                    run = (g & 31) ? before + incl[g - 1] : before;
                 }
+                // u2 within the rounding of 1: the last pair that can hop
+                if (ev < 0) ev = last;
+                int row, col;
+                if (ev < A1) row = div_small(ev, T1, inv1, col);
+                else row = N + div_small(ev - A1, T2, inv2, col);
+                if (col >= z) col += N - z;
                 if (lane == 0) {
+                    int f = src[row].id, t = tgt[col].id;
+                    // a replay's u2 outside (0, 1] (it may hold 0): the dense
+                    // loop takes its first entry, pair (0, 0)
+                    if (uniforms &&
+                        static_cast<unsigned long long>(__double_as_longlong(u2)) - 1ull >= 0x3ff0000000000000ull)
+                        f = t = 0;
                     ev_from = f;
                     ev_to = t;
                     if (f >= N) eo_s[f - N] -= 1;
@@ -470,7 +469,7 @@ __device__ __forceinline__ void f64_chain(
         to = ev_to;
         dt = sh_dt;
         h += (to < N ? 1 : 0) - (from < N ? 1 : 0);
-        if (from == to) h += 1 - static_cast<int>(occw[0] & 1u);      // (0, 0) fills site 0
+        if (uniforms && from == to) h += 1 - static_cast<int>(occw[0] & 1u);      // (0, 0) fills site 0
         if (flux_time)
             for (int e = tid; e < P; e += kThreads) sh_fx[e] += sh_J[e] * dt;
     }

@@ -89,13 +89,14 @@ struct Layout {
 __host__ __device__ inline size_t layout_bytes(const Layout &l)
 {
     return 20 * static_cast<size_t>(l.tab) + 8 * static_cast<size_t>(l.rates + l.invd) + 16 * kExpTable +
-           (2 * sizeof(Site) + 2 * 8 + 8) * static_cast<size_t>(l.S) + 8 * (kThreads + 64 + 128) + 4 * 64 + 32;
+           (2 * sizeof(Site) + 2 * 8) * static_cast<size_t>(l.S) + 8 * (kThreads + 64 + 128) + 4 * 64 + 32;
 }
 
 // One chain run by the whole block (the body of both kernels below).
 // kTab: tc and (I_0 R)/d are read from shared memory; kRate: the rates of a
-// hop sit there.
-template <bool kTab, bool kRate>
+// hop sit there; kReplay: the uniforms are the caller's (apart, because the
+// test for those that Philox does not draw costs 2 % of a run).
+template <bool kTab, bool kRate, bool kReplay>
 __device__ __forceinline__ void f64_chain(
     const Layout &lay, int N, int P, double nu, double kT, double I0, double R, uint8_t *occ_g, const double *d,
     const double *Ec, const double *se_in, const double *tc, int64_t *eo, int64_t hops,
@@ -117,8 +118,7 @@ __device__ __forceinline__ void f64_chain(
     double *u_cl = u_ev + 32;                                      // [32] -log(1 - u1)
     double *sh_J = u_cl + 32;                                      // [64] expected net inflow
     double *sh_fx = sh_J + 64;                                     // [64] its time integral
-    long long *eo_s = reinterpret_cast<long long *>(sh_fx + 64);   // [P] electrode counters
-    int *tab_k = reinterpret_cast<int *>(eo_s + lay.S);            // [S*S] exponents beside tab
+    int *tab_k = reinterpret_cast<int *>(sh_fx + 64);              // [S*S] exponents beside tab
     uint32_t *occw = reinterpret_cast<uint32_t *>(tab_k + lay.tab);   // [64] occupancy bits
     __shared__ int wide_always, wide_now[2];   // energies or couplings beyond the split exponential
     __shared__ int ev_from, ev_to;
@@ -179,10 +179,8 @@ __device__ __forceinline__ void f64_chain(
             if (occ_g[w * 32 + b]) bits |= 1u << b;
         occw[w] = bits;
     }
-    for (int e = tid; e < P; e += kThreads) {
-        eo_s[e] = eo[e];
-        if (flux_time) sh_fx[e] = flux_time[e];
-    }
+    if (flux_time)
+        for (int e = tid; e < P; e += kThreads) sh_fx[e] = flux_time[e];
     // the electrodes' list entries, the same every hop
     for (int i = N + tid; i < S; i += kThreads) {
         const double e = se_in[i];
@@ -269,7 +267,7 @@ __device__ __forceinline__ void f64_chain(
             // the uniforms of the next 32 hops, mapped
             const int64_t hh = hop + lane;
             double u1 = 0.5, u2 = 0.5;
-            if (uniforms) {
+            if constexpr (kReplay) {
                 if (hh < hops) {
                     u1 = uniforms[2 * hh];
                     u2 = uniforms[2 * hh + 1];
@@ -280,6 +278,9 @@ __device__ __forceinline__ void f64_chain(
                 u1 = u01_from64(r.x, r.y);
                 u2 = u01_from64(r.z, r.w);
             }
+            // (a replay may hold 0; what is not in (0, 1] passes at k = 0, or never)
+            if (kReplay && static_cast<unsigned long long>(__double_as_longlong(u2)) - 1ull >= 0x3ff0000000000000ull)
+                u2 = NAN;
             u_ev[lane] = u2;
             u_cl[lane] = -log(1.0 - u1);
         }
@@ -424,24 +425,27 @@ __device__ __forceinline__ void f64_chain(
                     if ((g >> 5) != w) before += incl[w++ * 32 + 31];
                     run = (g & 31) ? before + incl[g - 1] : before;
                 }
-                // u2 within the rounding of 1: the last pair that can hop
-                if (ev < 0) ev = last;
-                int row, col;
-                if (ev < A1) row = div_small(ev, T1, inv1, col);
-                else row = N + div_small(ev - A1, T2, inv2, col);
-                if (col >= z) col += N - z;
+                int f = 0, t = 0;
+                if (kReplay && ev < 0 && (__double2hiint(u2) & 0x7ff00000) == 0x7ff00000) {
+                    // NaN: the dense loop's first entry, pair (0, 0), which
+                    // fills site 0: a hole from nowhere if it was empty
+                    if (lane == 0) ev_from = (occw[0] & 1u) ? 0 : S;
+                } else {
+                    // u2 within the rounding of 1: the last pair that can hop
+                    if (ev < 0) ev = last;
+                    int row, col;
+                    if (ev < A1) row = div_small(ev, T1, inv1, col);
+                    else row = N + div_small(ev - A1, T2, inv2, col);
+                    if (col >= z) col += N - z;
+                    f = src[row].id;
+                    t = tgt[col].id;
+                    if (lane == 0) ev_from = f;
+                }
                 if (lane == 0) {
-                    int f = src[row].id, t = tgt[col].id;
-                    // a replay's u2 outside (0, 1] (it may hold 0): the dense
-                    // loop takes its first entry, pair (0, 0)
-                    if (uniforms &&
-                        static_cast<unsigned long long>(__double_as_longlong(u2)) - 1ull >= 0x3ff0000000000000ull)
-                        f = t = 0;
-                    ev_from = f;
                     ev_to = t;
-                    if (f >= N) eo_s[f - N] -= 1;
-                    if (t >= N) eo_s[t - N] += 1;
-                    // fire and forget: nothing of this launch reads it
+                    // fire and forget: nothing of this launch reads them
+                    if (f >= N) atomicAdd(reinterpret_cast<unsigned long long *>(&eo[f - N]), ~0ull);
+                    if (t >= N) atomicAdd(reinterpret_cast<unsigned long long *>(&eo[t - N]), 1ull);
                     if (record) atomicAdd(&traffic[(size_t)f * S + t], 1.0);
                     if (hop_log) { hop_log[2 * hop] = f; hop_log[2 * hop + 1] = t; }
                 }
@@ -469,7 +473,6 @@ __device__ __forceinline__ void f64_chain(
         to = ev_to;
         dt = sh_dt;
         h += (to < N ? 1 : 0) - (from < N ? 1 : 0);
-        if (uniforms && from == to) h += 1 - static_cast<int>(occw[0] & 1u);      // (0, 0) fills site 0
         if (flux_time)
             for (int e = tid; e < P; e += kThreads) sh_fx[e] += sh_J[e] * dt;
     }
@@ -483,22 +486,20 @@ __device__ __forceinline__ void f64_chain(
     __syncthreads();
     for (int i = tid; i < N; i += kThreads) occ_g[i] = (occw[i >> 5] >> (i & 31)) & 1u;
     if (record && tid < N) oit[tid] = oit0;
-    for (int e = tid; e < P; e += kThreads) {
-        eo[e] = eo_s[e];
-        if (flux_time) flux_time[e] = sh_fx[e];
-    }
+    if (flux_time)
+        for (int e = tid; e < P; e += kThreads) flux_time[e] = sh_fx[e];
     if (tid == 32) *time_out = time;
     if (tid == 0) *status_out = status;
 }
 
-template <bool kTab, bool kRate>
+template <bool kTab, bool kRate, bool kReplay>
 __global__ void __launch_bounds__(kThreads, 1) f64_chain_kernel(
     const Layout lay, int N, int P, double nu, double kT, double I0, double R, uint8_t *occ_g, const double *d,
     const double *Ec, const double *se_in, const double *tc, int64_t *eo, int64_t hops,
     int record, double *traffic, double *oit, const double *uniforms, uint64_t seed,
     int32_t *hop_log, double *time_out, int32_t *status_out, double *ws, double *flux_time)
 {
-    f64_chain<kTab, kRate>(lay, N, P, nu, kT, I0, R, occ_g, d, Ec, se_in, tc, eo, hops, record, traffic, oit,
+    f64_chain<kTab, kRate, kReplay>(lay, N, P, nu, kT, I0, R, occ_g, d, Ec, se_in, tc, eo, hops, record, traffic, oit,
                            uniforms, seed, hop_log, time_out, status_out, ws, flux_time);
 }
 
@@ -524,7 +525,7 @@ __global__ void __launch_bounds__(kThreads, 1) f64_batch_kernel(const Layout lay
     double *fx = B.flux_time ? B.flux_time + eo : nullptr;
     double *tr = B.record ? B.traffic + B.traffic_off[c] : nullptr;
     double *oit = B.record ? B.occupations_in_time + so : nullptr;
-    f64_chain<kTab, kRate>(lay, N, P, B.nu[c], B.kT[c], B.I_0[c], B.R[c], B.occupation + so, B.distances + po,
+    f64_chain<kTab, kRate, false>(lay, N, P, B.nu[c], B.kT[c], B.I_0[c], B.R[c], B.occupation + so, B.distances + po,
                            B.E_constant + so, B.site_energies + vo, B.transitions_constant + po,
                            B.electrode_occupation + eo, B.hops[c], B.record, tr, oit, nullptr, B.seeds[c], nullptr,
                            B.time_out + c, B.status_out + c, B.workspace + (size_t)c * ws_doubles, fx);
@@ -596,8 +597,12 @@ int simulate_f64(int N, int P, double nu, double kT, double I0, double R, uint8_
                                           static_cast<double *>(ws), flux_time);
         return KMC_OK;
     };
-    const int rc = lay.tab > 0 ? launch(f64_chain_kernel<true, true>)
-                   : lay.rates > 0 ? launch(f64_chain_kernel<false, true>) : launch(f64_chain_kernel<false, false>);
+    const int rc = uniforms ? (lay.tab > 0     ? launch(f64_chain_kernel<true, true, true>)
+                               : lay.rates > 0 ? launch(f64_chain_kernel<false, true, true>)
+                                               : launch(f64_chain_kernel<false, false, true>))
+                            : (lay.tab > 0     ? launch(f64_chain_kernel<true, true, false>)
+                               : lay.rates > 0 ? launch(f64_chain_kernel<false, true, false>)
+                                               : launch(f64_chain_kernel<false, false, false>));
     if (rc != KMC_OK) return rc;
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail_cuda(e, "f64 launch");
@@ -722,9 +727,12 @@ namespace kmc {
 int preload_f64()
 {
     int rc;
-    if ((rc = touch_kernel(f64_chain_kernel<true, true>)) != KMC_OK) return rc;
-    if ((rc = touch_kernel(f64_chain_kernel<false, true>)) != KMC_OK) return rc;
-    if ((rc = touch_kernel(f64_chain_kernel<false, false>)) != KMC_OK) return rc;
+    if ((rc = touch_kernel(f64_chain_kernel<true, true, false>)) != KMC_OK) return rc;
+    if ((rc = touch_kernel(f64_chain_kernel<true, true, true>)) != KMC_OK) return rc;
+    if ((rc = touch_kernel(f64_chain_kernel<false, true, false>)) != KMC_OK) return rc;
+    if ((rc = touch_kernel(f64_chain_kernel<false, true, true>)) != KMC_OK) return rc;
+    if ((rc = touch_kernel(f64_chain_kernel<false, false, false>)) != KMC_OK) return rc;
+    if ((rc = touch_kernel(f64_chain_kernel<false, false, true>)) != KMC_OK) return rc;
     if ((rc = touch_kernel(f64_batch_kernel<true, true>)) != KMC_OK) return rc;
     if ((rc = touch_kernel(f64_batch_kernel<false, true>)) != KMC_OK) return rc;
     return touch_kernel(f64_batch_kernel<false, false>);

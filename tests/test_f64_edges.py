@@ -68,7 +68,7 @@ def test_electrode_counts_beyond_32_bits(engine_lib, oracle_mod):
     n = _net(30, 6, seed=3)
     edge = 2**31
     start = np.array([edge - 1, -edge, edge, -edge - 1, 2**62, 0], np.int64)
-    u = replay_uniforms(8, 2000)
+    u = replay_uniforms(8, 2 * 2500)
     r = _replay(oracle_mod, _args(n), u, 1e-11, electrode_occupation=start)
     moved = r["electrode_occupation"] - start
     assert moved[0] or moved[1] or moved[2] or moved[3]

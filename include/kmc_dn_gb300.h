@@ -334,8 +334,9 @@ int kmc_build_table(int32_t n_acceptors, int32_t n_electrodes, double nu, double
  * kmc_build_table for n_tables geometries whose FP64 tables are HOST arrays:
  * table t (S = n_acceptors[t] + n_electrodes[t]) goes to tab_LB +
  * tab_off[t] floats.  All arguments but tab_LB are host arrays, distances
- * and transitions_constant arrays of n_tables host pointers.  One launch for
- * all of them.  Returns when the tables are built (the host arrays are free
+ * and transitions_constant arrays of n_tables host pointers.  They pass
+ * through 64 MB of device memory (or the largest table's), a launch a
+ * filling.  Returns when the tables are built (the host arrays are free
  * then).
  */
 int kmc_build_tables(int32_t n_tables, const int32_t *n_acceptors, const int32_t *n_electrodes,

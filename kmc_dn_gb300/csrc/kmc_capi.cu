@@ -95,7 +95,7 @@ struct EngineState {
 // and lifetimes -- the order of the Python Batch's work lists.
 // A launch of few chains cannot fill the GPU, and its run time is the
 // per-hop latency of one chain: each chain then gets a wider group (one
-// N=120 chain takes 2.7 us per hop at 256 lanes, 12.9 us at the size
+// N=120 chain takes 2.3 us per hop at 256 lanes, 8.6 us at the size
 // default of 32), up to twice the next power of two of its site count and
 // 512 lanes, while the launch's chains x lanes stay within a quarter of the
 // engine's resident threads (512 per SM).  The Python layer applies the

@@ -4,7 +4,8 @@
 //                 pair table of (L, B) = (log2(nu*tc), I_0 R/d) pairs
 //                 (calc_transitions_constant kmc_dopant_networks.py:824-830;
 //                 the Coulomb term of dE :72-75 / simulation.go:67-68).
-//                 (build_tables: all geometries of a batch in one launch)
+//                 (build_tables: the geometries of a batch, as many a launch
+//                 as their FP64 tables fill a bounded staging buffer)
 //  site_energies  constant site energies of many chains from the Laplace
 //                 basis fields sampled at the acceptors: the superposition
 //                 sum_e V_e phi_e + mu phi_mu plus donor compensation, which

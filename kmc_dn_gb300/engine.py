@@ -414,7 +414,7 @@ def balanced_warps_per_block(n_work, sms):
 def widen_small_launch(G, S, n_chains, sms):
     """Lanes for a chain of a launch too small to fill the GPU: its run time
     is one chain's per-hop latency, so each chain gets a wider group (one
-    N=120 chain: 2.7 us per hop at 256 lanes, 12.9 us at the size default of
+    N=120 chain: 2.3 us per hop at 256 lanes, 8.6 us at the size default of
     32), up to twice the next power of two of S and 512 lanes, while the
     launch's chains x lanes stay within a quarter of the engine's resident
     threads (512 per SM).  The C host path applies the same rule."""

@@ -228,20 +228,14 @@ __device__ void mf_pairs(const kmc_mf_batch &b)
     __shared__ double sh_f, sh_ts, sh_time;
     __shared__ int sh_stop;
 
-    const double inv_kT = 1.0 / kT;
-    // pair tables: K = nu*tc, B = I_0 R / d between acceptors (0 otherwise),
-    // no rate between electrodes.  A site onto itself: dE = -I_0 R / d_ii, so
-    // the rate is K whatever the state unless the sites attract (I_0 < 0: 0
-    // for d_ii = 0); B = 0 there, for the energies' sums.
+    // pair tables: K = nu*tc, B = I_0 R / d between acceptors (0 otherwise,
+    // and on the diagonal, where the rate is K either way unless the sites
+    // attract), no rate between electrodes
     for (int p = tid; p < SS; p += T) {
         const int i = p / S, j = p - (p / S) * S;
-        double K = (i >= N && j >= N) ? 0.0 : nu * tcon[p];
-        const double c = (i < N && j < N) ? I0R / dist[p] : 0.0;
-        if (i == j && c < 0.0) K *= exp(c * inv_kT);
-        // 1/kT infinite or NaN: so are exponents of 0, and the network stops
-        // (the FP64 rates take no exponential for them)
-        if (F64 && !(fabs(inv_kT) < INFINITY)) K = NAN;
-        KB[i * SP + j] = Pair{static_cast<Real>(K), static_cast<Real>(i != j ? c : 0.0)};
+        const double K = (i >= N && j >= N) ? 0.0 : nu * tcon[p];
+        const double B = (i < N && j < N && i != j) ? I0R / dist[p] : 0.0;
+        KB[i * SP + j] = Pair{static_cast<Real>(K), static_cast<Real>(B)};
     }
     for (int k = tid; k < S; k += T) {
         occ[k] = k < N ? occ_io[k] : F64 ? 1.0 : 0.0;
@@ -257,6 +251,20 @@ __device__ void mf_pairs(const kmc_mf_batch &b)
     }
     if (tid == 0) { sh_time = 0.0; sh_stop = 0; }
     __syncthreads();
+
+    const double inv_kT = 1.0 / kT;
+    if (I0R < 0.0) {
+        // a site onto itself: dE = -I_0 R / d_ii > 0, a rate of 0 for d_ii = 0
+        for (int k = tid; k < N; k += T)
+            KB[k * SP + k].x *= static_cast<Real>(exp(I0R / dist[k * S + k] * inv_kT));
+        __syncthreads();
+    }
+    if (F64 && !(fabs(inv_kT) < INFINITY)) {
+        // 1/kT infinite or NaN: so are exponents of 0, and the network stops
+        // (the FP64 rates take no exponential for them)
+        for (int k = tid; k < N; k += T) KB[k * SP + k].x = NAN;
+        __syncthreads();
+    }
 
     const Real ec_i = tid < N ? static_cast<Real>(Ec[tid]) : Real(0);
     const bool unit = kT == 1.0;
